@@ -123,15 +123,31 @@ __device__ __forceinline__ uint64_t hp_morton_key(float mnx, float mny, float mn
 }
 
 // ---- triangle vertices (indexed mesh, 3 vertex indices per triangle) --------
+// Three consecutive 4-byte words from any 4-byte aligned address as two loads,
+// the 8-byte aligned pair of them and the other one. A gather of triangles is
+// bound by the L1's request rate (a request costs about one cycle for every
+// line that its lanes touch, whatever a lane reads), so eight requests a
+// triangle instead of twelve shorten it.
+__device__ __forceinline__ void load3(const uint32_t* p, uint32_t& x, uint32_t& y, uint32_t& z) {
+    const bool hi = (reinterpret_cast<uintptr_t>(p) & 4u) != 0;  // the pair is (y, z)
+    const uint2 pair = __ldg(reinterpret_cast<const uint2*>(hi ? p + 1 : p));
+    const uint32_t one = __ldg(hi ? p : p + 2);
+    x = hi ? one : pair.x;
+    y = hi ? pair.x : pair.y;
+    z = hi ? pair.y : one;
+}
+
 __device__ __forceinline__ void load_vertex(const float* __restrict__ v, int64_t nv, int idx,
                                             float& x, float& y, float& z, int* err) {
     if (idx < 0 || idx >= nv) {
         hp_report(err, HP_DEV_BAD_INPUT, idx);
         idx = 0;
     }
-    x = __ldg(v + 3 * (int64_t)idx + 0);
-    y = __ldg(v + 3 * (int64_t)idx + 1);
-    z = __ldg(v + 3 * (int64_t)idx + 2);
+    uint32_t a, b, c;
+    load3(reinterpret_cast<const uint32_t*>(v + 3 * (int64_t)idx), a, b, c);
+    x = __uint_as_float(a);
+    y = __uint_as_float(b);
+    z = __uint_as_float(c);
 }
 
 struct tri_verts {
@@ -141,10 +157,11 @@ struct tri_verts {
 __device__ __forceinline__ tri_verts load_tri(const float* __restrict__ v, int64_t nv,
                                               const int32_t* __restrict__ t, int64_t tri, int* err) {
     tri_verts r;
-    int a = __ldg(t + 3 * tri + 0), b = __ldg(t + 3 * tri + 1), c = __ldg(t + 3 * tri + 2);
-    load_vertex(v, nv, a, r.x0, r.y0, r.z0, err);
-    load_vertex(v, nv, b, r.x1, r.y1, r.z1, err);
-    load_vertex(v, nv, c, r.x2, r.y2, r.z2, err);
+    uint32_t a, b, c;
+    load3(reinterpret_cast<const uint32_t*>(t + 3 * tri), a, b, c);
+    load_vertex(v, nv, (int)a, r.x0, r.y0, r.z0, err);
+    load_vertex(v, nv, (int)b, r.x1, r.y1, r.z1, err);
+    load_vertex(v, nv, (int)c, r.x2, r.y2, r.z2, err);
     return r;
 }
 

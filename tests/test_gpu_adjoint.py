@@ -199,3 +199,47 @@ def test_autograd_function_gradient_and_refit_step(ctx):
     # the closest hit does not depend on the tree (ties go to the lower id) except
     # where a slab test rounds a node away; allow that on a handful of rays
     assert np.mean(np.all(a == b, axis=1)) > 0.9999
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("group", [1, 3, 32, 77])
+def test_adjoint_groups_and_alignment(ctx, group, shift):
+    """Runs of `group` rays on one triangle (lanes of a warp that sum before they add:
+    one, a few, a whole warp, runs across warps) and every third ray on another
+    triangle between them, with all buffers 0 or 4 bytes past an 8-byte boundary."""
+    n = 4099
+
+    def at(a):  # the array, `shift` words into a buffer
+        x = torch.from_numpy(np.ascontiguousarray(a)).reshape(-1)
+        buf = torch.zeros(x.numel() + shift, dtype=x.dtype, device="cuda")
+        buf[shift:] = x.cuda()
+        return buf[shift:].reshape(a.shape)
+
+    v, t, _ = _scene(17, 19)
+    v[:, 2] *= 0.1  # gentle slopes: no triangle near edge-on, whose determinant cancels
+    rng = np.random.default_rng(group)
+    tri = (np.arange(n) // group) % len(t)
+    tri[::3] = (tri[::3] * 7 + 3) % len(t)
+    # a ray through a chosen point of its triangle, one unit before it (the oracle
+    # takes the barycentrics from the ray)
+    uv = rng.uniform(0.1, 0.45, (n, 2))
+    p = v[t[tri]].astype(np.float64)
+    at_p = uv[:, :1] * p[:, 0] + uv[:, 1:] * p[:, 1] + (1 - uv.sum(1, keepdims=True)) * p[:, 2]
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, 4:7] = rng.normal(size=(n, 3)) * 0.1 + [0, 0, -1]
+    rays[:, :3] = at_p - rays[:, 4:7]
+    res = np.zeros((n, 4), np.int32)
+    res[:, 0] = np.where(rng.random(n) < 0.05, -1, tri)
+    res[:, 1] = np.ones(n, np.float32).view(np.int32)
+    res[:, 2:] = uv.astype(np.float32).view(np.int32)
+    w = rng.standard_normal((n, 3)).astype(np.float32)
+    grad = at(np.zeros_like(v))
+    # rays and results keep the 16-byte alignment of their records
+    ctx.adjoint(at(v), at(t), dev(rays), dev(res), at(w), dl_dverts=grad)
+    ctx.check()
+    exp = oracle.adjoint64(v, t, rays, res, w)
+    # a ray's 32-bit origin moves its barycentrics by eps * |o| / (size of a triangle),
+    # about 6e-8 * 2 / 0.06, and the sums add a few eps (the same formula in 32-bit
+    # numpy with 64-bit sums is 5e-7 to 8e-7 off): below 1e-5 of the norm
+    err = np.linalg.norm(grad.cpu().numpy().astype(np.float64) - exp) / np.linalg.norm(exp)
+    assert err < 1e-5

@@ -147,3 +147,19 @@ def test_bad_vertex_index_reported(ctx):
     with pytest.raises(hp.HPError) as ei:
         bvh.sync()
     assert ei.value.status == 5
+
+
+@pytest.mark.parametrize("method", ["lbvh", "ploc", "atr"])
+def test_buffers_at_any_word(ctx, method):
+    """Vertices and triangles 4 bytes past an 8-byte boundary give the same BVH: their
+    three-word rows are read as an aligned pair and a word."""
+    v, t = hp.gen.uniform_mesh(21, 3001)
+    p = hp.BuildParams(method=method, morton_bits=30)
+    want = ctx.build(dev(v), dev(t), p).download()
+    V = torch.zeros(v.size + 1, dtype=torch.float32, device="cuda")
+    T = torch.zeros(t.size + 1, dtype=torch.int32, device="cuda")
+    V[1:], T[1:] = dev(v).reshape(-1), dev(t).reshape(-1)
+    got = ctx.build(V[1:].reshape(v.shape), T[1:].reshape(t.shape), p).download()
+    ctx.check()
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))

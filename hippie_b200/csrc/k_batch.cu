@@ -262,10 +262,8 @@ __global__ void __launch_bounds__(TB) k_b_climb(bargs B) {
             hp_report(B.err, HP_DEV_BAD_INDEX, node);
             return;
         }
-        __threadfence();
-        if (atomicAdd(&counters[node], 1) == 0) return;
-        __threadfence();
-        const int l = left[node], r = right[node];
+        const int l = left[node], r = right[node], up = parent[node];
+        if (hp_arrive(&counters[node]) == 0) return;
         if ((unsigned)l >= (unsigned)(2 * n - 1) || (unsigned)r >= (unsigned)(2 * n - 1)) {
             hp_report(B.err, HP_DEV_BAD_INDEX, node);
             return;
@@ -294,7 +292,7 @@ __global__ void __launch_bounds__(TB) k_b_climb(bargs B) {
             const int2 rg = range[node];
             atomicMax(&B.max_hi[sg.tri_off + rg.x], sg.tri_off + rg.y);
         }
-        node = parent[node];
+        node = up;
     }
 }
 

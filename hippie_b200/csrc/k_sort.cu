@@ -280,6 +280,128 @@ constexpr size_t onesweep_smem() {
     return a > b ? a : b;
 }
 
+// ---- few keys: every pass in one CTA ---------------------------------------------
+// Up to ONE_CAP keys are sorted by one CTA of 1024 threads that keeps them in
+// registers and shared memory from the first pass to the last: a pass is the
+// ranking and staging of k_onesweep without look-back, histograms or global
+// memory. At this size a global pass is all latency (about 11 us each, four to
+// eight of them, with one or two tiles of work): 5,003 30-bit keys 0.060 -> 0.029 ms
+// on a B200. 8 keys a thread is what 64 registers (1,024 threads) and the shared
+// memory of wide keys (96 KB) hold.
+constexpr int ONE_BLOCK = 1024, ONE_ITEMS = 8, ONE_CAP = ONE_BLOCK * ONE_ITEMS;
+
+template <typename K>
+__global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__ keys_in,
+                                                           const int32_t* __restrict__ vals_in,
+                                                           K* __restrict__ keys_out, int32_t* __restrict__ vals_out,
+                                                           int n, int bits) {
+    constexpr int NW = ONE_BLOCK / 32;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);   // [NW][256] while ranking
+    K* skeys = reinterpret_cast<K*>(smem);                // [ONE_CAP] while staging
+    int32_t* svals = reinterpret_cast<int32_t*>(smem + (size_t)ONE_CAP * sizeof(K));
+    __shared__ uint32_t s_w[8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    // Keys are spread over as few rounds as they need, the same for every warp.
+    const int rounds = (n + ONE_BLOCK - 1) / ONE_BLOCK;
+    const int wbase = warp * 32 * rounds;
+    K key[ONE_ITEMS];
+    int32_t val[ONE_ITEMS];
+    uint32_t pos[ONE_ITEMS];
+#pragma unroll
+    for (int i = 0; i < ONE_ITEMS; ++i) {
+        const int idx = wbase + i * 32 + lane;
+        const bool valid = i < rounds && idx < n;
+        key[i] = valid ? keys_in[idx] : K(0);
+        val[i] = valid ? (vals_in ? vals_in[idx] : idx) : 0;
+    }
+    for (int shift = 0; shift < bits; shift += 8) {
+        const uint32_t dmask = bits - shift >= 8 ? 255u : (1u << (bits - shift)) - 1u;
+        for (int i = tid; i < NW * 256; i += ONE_BLOCK) cnt[i] = 0;
+        __syncthreads();
+        // rank within the warp in index order (round, then lane)
+        uint32_t* wcnt = cnt + warp * 256;
+#pragma unroll
+        for (int i = 0; i < ONE_ITEMS; ++i) {
+            if (i >= rounds) break;
+            const bool valid = wbase + i * 32 + lane < n;
+            const uint32_t d = valid ? digit_of(key[i], shift, dmask) : 0u;
+            uint32_t peers = __ballot_sync(HP_FULL_MASK, valid);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const uint32_t bal = __ballot_sync(HP_FULL_MASK, (d >> b) & 1u);
+                peers &= ((d >> b) & 1u) ? bal : ~bal;
+            }
+            const uint32_t below = __popc(peers & lt_mask);
+            const uint32_t c = valid ? wcnt[d] : 0u;
+            __syncwarp();
+            if (valid && below == 0) wcnt[d] = c + __popc(peers);
+            __syncwarp();
+            pos[i] = c + below;
+        }
+        __syncthreads();
+        // per digit: offsets of the warps, then of the digits (one thread per digit)
+        uint32_t run = 0, incl = 0;
+        if (tid < 256) {
+#pragma unroll 8
+            for (int w = 0; w < NW; ++w) {
+                const uint32_t c = cnt[w * 256 + tid];
+                cnt[w * 256 + tid] = run;
+                run += c;
+            }
+            incl = run;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(HP_FULL_MASK, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (lane == 31) s_w[warp] = incl;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t off = incl - run;
+            for (int w = 0; w < warp; ++w) off += s_w[w];
+#pragma unroll 8
+            for (int w = 0; w < NW; ++w) cnt[w * 256 + tid] += off;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ONE_ITEMS; ++i)
+            if (i < rounds) pos[i] += wcnt[digit_of(key[i], shift, dmask)];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ONE_ITEMS; ++i) {
+            if (i < rounds && wbase + i * 32 + lane < n) {
+                skeys[pos[i]] = key[i];
+                svals[pos[i]] = val[i];
+            }
+        }
+        __syncthreads();
+        if (shift + 8 >= bits) break;
+#pragma unroll
+        for (int i = 0; i < ONE_ITEMS; ++i) {
+            const int idx = wbase + i * 32 + lane;
+            if (i < rounds && idx < n) {
+                key[i] = skeys[idx];
+                val[i] = svals[idx];
+            }
+        }
+        __syncthreads();
+    }
+    for (int j = tid; j < n; j += ONE_BLOCK) {
+        keys_out[j] = skeys[j];
+        vals_out[j] = svals[j];
+    }
+}
+
+template <typename K>
+constexpr size_t sort_one_smem() {
+    constexpr size_t a = (size_t)(ONE_BLOCK / 32) * 256 * 4;
+    constexpr size_t b = (size_t)ONE_CAP * (sizeof(K) + 4);
+    return a > b ? a : b;
+}
+
 // ---- wide keys: top 24 bits by three LSD passes, then a sort of every segment ----
 // For keys of more than 48 bits, the full LSD sort is ceil(bits/8) passes over
 // global memory (8 for 60-bit Morton codes). Instead: three of those passes
@@ -299,10 +421,13 @@ constexpr int SEG_BLOCK = 256, SEG_ITEMS = 8, SEG_CAP = SEG_BLOCK * SEG_ITEMS, S
 constexpr int SEG_NW = SEG_BLOCK / 32;
 constexpr int SEG_RANK_MAX = 512;  // segments ranked element by element
 constexpr int SEG_MED_CAP = SEG_CAP / (SEG_RANK_MAX + 1) + 1;  // longer segments in one chunk
-constexpr int64_t HYBRID_MIN_N = int64_t(1) << 20;
 
+// Whenever wide keys do not fit one CTA. Below 2^20 keys a pass is mostly latency
+// (11 us at 0.1 M keys, 18 us at 1 M), so five passes fewer count for more there:
+// 60-bit keys on a B200, 100,003 of them 0.121 -> 0.065 ms, 1,048,573 of them
+// 0.170 -> 0.091 ms against eight passes.
 __host__ __device__ constexpr bool hybrid_sort(int64_t n, int key_bytes, int bits) {
-    return key_bytes == 8 && bits > 48 && n >= HYBRID_MIN_N;
+    return key_bytes == 8 && bits > 48 && n > ONE_CAP;
 }
 
 constexpr int SEG_TOP = 3;  // 8-bit digits ordered by global passes
@@ -743,6 +868,17 @@ __global__ void __launch_bounds__(SEG_BLOCK, 4) k_seg_big(uint64_t* kin, int32_t
 
 template <typename K, int BLOCK>
 hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream_t stream) {
+    if (plan.n <= ONE_CAP) {
+        constexpr size_t one_smem = sort_one_smem<K>();
+        HP_CUDA(cudaFuncSetAttribute(k_sort_one<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one_smem));
+        k_sort_one<K><<<1, ONE_BLOCK, one_smem, stream>>>(reinterpret_cast<const K*>(a.keys_in), a.vals_in,
+                                                          reinterpret_cast<K*>(a.keys_out), a.vals_out, (int)plan.n,
+                                                          plan.bits);
+        HP_CUDA(cudaGetLastError());
+        hp_count_launch();
+        hp_mark(a.ctx, stream, "sort_pass");
+        return HP_OK;
+    }
     constexpr int ITEMS = sort_cfg<K>::ITEMS;
     const int64_t n = plan.n;
     hp_carve cv(reinterpret_cast<char*>(a.scratch));
@@ -1079,6 +1215,7 @@ constexpr size_t NOALLOC_BYTES =
                                      sort_cfg<uint64_t>::BLOCK * sort_cfg<uint64_t>::ITEMS, 8),
                 noalloc_sort_scratch(HP_NOALLOC_SORT_MAX_KEYS, 4,
                                      sort_cfg<uint32_t>::BLOCK * sort_cfg<uint32_t>::ITEMS, 4)) +
+    noalloc_pad((HP_NOALLOC_SORT_MAX_KEYS / (SEG_CAP + 1) + 1) * 8) +  // long segments of wide keys
     noalloc_pad(8 * 256 * 4) + 256;
 
 __device__ __align__(256) unsigned char g_noalloc_sort_scratch[NOALLOC_BYTES];

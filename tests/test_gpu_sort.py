@@ -83,3 +83,23 @@ def test_radix_sort_wide_keys_by_segments(ctx, kind, n, bits, with_vals):
     order = np.argsort(keys & mask, kind="stable")
     np.testing.assert_array_equal(vo.cpu().numpy(), (vals[order] if with_vals else order.astype(np.int32)))
     np.testing.assert_array_equal(ko.cpu().numpy().view(np.uint64), keys[order])
+
+
+@pytest.mark.parametrize("dtype", [np.uint32, np.uint64])
+@pytest.mark.parametrize("n", [31, 1023, 1024, 1025, 8191, 8192, 8193, 12289])
+@pytest.mark.parametrize("kind", ["uniform", "few", "equal"])
+def test_sort_one_cta_edges(ctx, dtype, n, kind):
+    """Around the largest sort of one CTA (8,192 keys) and of its rounds of 1,024, for
+    both key widths; wide keys go on with the segmented sort from there."""
+    rng = np.random.default_rng(n)
+    bits = 30 if dtype == np.uint32 else 60
+    keys = {"uniform": rng.integers(0, 1 << bits, size=n, dtype=np.uint64),
+            "few": rng.integers(0, 7, size=n, dtype=np.uint64) << np.uint64(bits - 9),
+            "equal": np.full(n, 5, np.uint64)}[kind].astype(dtype)
+    vals = rng.permutation(n).astype(np.int32)
+    order = np.argsort(keys, kind="stable")
+    K = torch.from_numpy(keys.view(np.int32 if dtype == np.uint32 else np.int64)).cuda()
+    ko, vo = ctx.radix_sort(K, torch.from_numpy(vals).cuda(), bits=bits)
+    ctx.check()
+    np.testing.assert_array_equal(ko.cpu().numpy().view(dtype), keys[order])
+    np.testing.assert_array_equal(vo.cpu().numpy(), vals[order])

@@ -230,7 +230,10 @@ __global__ void __launch_bounds__(TB) k_leaves(
 // instead was slower: the CTAs' local subtrees are deep.) Phase B
 // (k_climb_frontier) climbs from the frontier entries through the non-local
 // nodes (those whose ranges cross a CTA boundary: about depth per boundary)
-// with the global counters and one acq_rel atomic per arrival.
+// with the global counters and one acq_rel atomic per arrival; a node's links are
+// read while the arrival at its child travels (5 K triangles 0.031 -> 0.025 ms,
+// 16.8 M 0.178 -> 0.146 ms). 1,024 leaves per CTA halve phase B and slow phase A
+// by as much (0.70 -> 0.80 ms at 16.8 M).
 constexpr int CB = 512;
 constexpr size_t CLIMB_SMEM = (size_t)CB * (4 * sizeof(float4) + 7 * sizeof(int) + sizeof(int2)) + 2 * sizeof(int);
 
@@ -385,13 +388,25 @@ __global__ void __launch_bounds__(TB) k_climb_frontier(climb_args A) {
         float4 cmn = __ldcg(A.nbmin + child), cmx = __ldcg(A.nbmax + child);
         int node = __ldg(A.parent + child);
         int guard = 0;
+        int nl = 0, nr = 0, nup = -1;  // links of `node`, read a level ahead
+        int2 nrg = make_int2(0, 0);
+        auto links = [&](int i) {
+            if ((unsigned)i < (unsigned)(n - 1)) {
+                nl = __ldg(A.left + i);
+                nr = __ldg(A.right + i);
+                nup = __ldg(A.parent + i);
+                nrg = __ldg(A.range + i);
+            }
+        };
+        links(node);
         while (node >= 0) {
             if (node >= n - 1 || ++guard > n) {
                 hp_report(A.err, HP_DEV_BAD_INDEX, node);
                 break;
             }
-            const int l = __ldg(A.left + node), r = __ldg(A.right + node), up = __ldg(A.parent + node);
-            const int2 rg = __ldg(A.range + node);
+            const int l = nl, r = nr, up = nup;
+            const int2 rg = nrg;
+            links(up);  // while the arrival travels
             if (hp_arrive(&A.counters[node]) == 0) break;
             if ((unsigned)l >= (unsigned)(2 * n - 1) || (unsigned)r >= (unsigned)(2 * n - 1) ||
                 (l != child && r != child)) {
@@ -740,7 +755,8 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(ctx, s, "climb_local");
-        k_climb_frontier<<<(unsigned)(ctx->sm_count * 8), TB, 0, s>>>(A);
+        // at most one entry per reference; small meshes need few CTAs
+        k_climb_frontier<<<(unsigned)std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s>>>(A);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
     }

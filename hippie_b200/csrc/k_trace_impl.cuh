@@ -18,13 +18,12 @@
 constexpr int TRACE_BLOCK = 128;
 constexpr int STACK = 64;         // traversal stack entries per ray: SST in shared memory, the rest local
 constexpr int SENTINEL = 0x76543210;
-constexpr int FETCH_THRESHOLD = 20;
 constexpr int TRAVERSAL_LIMIT = 1 << 22;  // visits per ray before the ray is abandoned with an error
 
 struct ray_state {
     float ox, oy, oz, tmin, dx, dy, dz;
     float idx_, idy, idz, oodx, oody, oodz;
-    float hit_t, hit_u, hit_v;
+    float hit_t;
     int hit;       // woop / leaf-ordered reference index of the closest hit, -1 if none
     int nodes, tris;
 };
@@ -53,51 +52,114 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
     return lo;
 }
 
+// What bounds the tracer is, first, how many lanes of a warp do the same thing
+// (6.3 of 32 per instruction when every lane ran its own loops over nodes and
+// over the triangles of its leaves, a warp in any number of pieces) and then the
+// L1's request rate: a 64-byte node is two requests of one line a lane, about 2.1
+// cycles of an SM's L1 when it comes from L2 and 1.4 when it hits, and a bounce
+// ray of the 4.2 M-triangle scene takes 79 nodes, 6 leaves and 14 triangles. So a
+// warp stays in one piece and takes three kinds of turns, all 32 lanes together,
+// decided by ballots:
+//   * nodes: every lane at an interior node does one. The first leaf that a lane
+//     meets is postponed and the lane goes on from its stack; at a second one it
+//     waits. The turn ends when fewer than NODE_MIN lanes have an interior node
+//     and no postponed leaf, so that a hit is found, and shortens the ray, soon;
+//   * triangles: every lane with a postponed leaf tests one triangle, until fewer
+//     than TRI_MIN lanes have one;
+//   * new rays: once FETCH_MIN lanes are without work.
+// A stack entry keeps the child's entry distance, and an entry beyond the hit
+// found since is dropped at the pop: its boxes would all be missed (a child's
+// slab values lie between its parent's, rounded or not), so only the visit goes.
+// Measured on a B200, 16.8 M bounce rays 28.4 -> 19.8 ms, 43 M rays over 256
+// meshes 42.4 -> 27.5 ms, 1.05 M shadow rays 1.14 -> 0.95 ms, 2.07 M primary rays
+// 0.75 -> 0.56 ms, 4.2 M downward rays 2.28 -> 2.33 ms (14.3 lanes per instruction
+// and the L1 at 80 %). NODE_MIN / FETCH_MIN from 4 to 28 and TRI_MIN from 1 to 20
+// were swept: 16 / 8 / 12 is 1 % faster on bounce rays and 20 % slower on downward
+// ones, whose leaves it tests too late; higher ones lose on bounce rays.
+// Three CTAs more or fewer than 10 per SM, an 8-entry shared stack, packed FP32
+// for the slabs and 32-byte loads of two Woop rows were slower or no faster.
+constexpr int NODE_MIN = 16, TRI_MIN = 6, FETCH_MIN = 10;
+// CTAs per SM: 48 registers for one BVH, 61 with the mesh's bases in the lane.
+constexpr int TRACE_CTAS = 10, TRACE_CTAS_BATCH = 8;
+
 // BATCH: rays of many meshes in one launch; ray g belongs to the segment whose
 // ray range holds it, and the lane traverses that mesh's BVH.
 template <bool ANY_HIT, bool STATS, bool BATCH, int SST>
-__global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? 9 : 12) k_trace(
+__global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_CTAS) k_trace(
     const float4* __restrict__ rays, int64_t num_rays, int4* __restrict__ results,
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
     const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order) {
-    constexpr int SSTACK = SST, LSTACK = STACK - SST;
-    __shared__ int s_stack[SSTACK * TRACE_BLOCK];
-    int* sstack = s_stack + threadIdx.x;
-    int lstack[LSTACK];
+    constexpr int LST = STACK - SST;
+    __shared__ int2 s_stack[SST * TRACE_BLOCK];
+    int2* sstack = s_stack + threadIdx.x;
+    int2 lstack[LST];
     const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1u;
 
     ray_state r;
+    r.hit_t = 0.0f;
+    r.hit = -1;
     int64_t ray = -1;
     int node = SENTINEL;
-    int leaf = 0;   // postponed leaf (~index), >= 0 when none
+    int leaf = 0;            // postponed leaf (~index) whose range is not loaded yet, 0 when none
+    int tri = 0, tri_end = 0;  // triangles of the postponed leaf still to test
     int sp = 0;
-    int steps = 0;  // node + leaf visits of the current ray (bounded)
-    bool exhausted = false;
+    int steps = 0;           // node + leaf visits of the current ray (bounded)
+    bool exhausted = false;  // warp-uniform: the counter has run past the rays
     const float4* nodes = nodes_all;
     const float4* woop = woop_all;
     const int32_t* tri_idx = tri_all;
     int max_nodes = max_nodes_all, num_refs = num_refs_all;
 
+    auto pop = [&]() {
+        // (the statistics count visits as the reference does, dropped ones too)
+        node = SENTINEL;
+        while (sp > 0) {
+            --sp;
+            const int2 e = sp < SST ? sstack[sp * TRACE_BLOCK] : lstack[sp - SST];
+            if (STATS || !(__int_as_float(e.y) > r.hit_t)) {
+                node = e.x;
+                break;
+            }
+        }
+    };
+
     while (true) {
-        // Refill lanes whose ray is finished (one atomic per warp).
-        const bool need = (node == SENTINEL) && !exhausted;
-        const unsigned need_mask = __ballot_sync(HP_FULL_MASK, need);
-        if (need_mask) {
-            const int leader = __ffs(need_mask) - 1;
+        // Finished lanes write their results and take new rays (one atomic per warp).
+        const bool idle = node == SENTINEL && leaf >= 0 && tri >= tri_end;
+        const unsigned idle_mask = __ballot_sync(HP_FULL_MASK, idle);
+        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= FETCH_MIN)) {
+            if (idle && ray >= 0) {
+                if (r.hit < 0) {
+                    reinterpret_cast<int2*>(results)[2 * ray] = make_int2(-1, __float_as_int(r.hit_t));
+                    if (STATS) stats[ray] = make_int2(0, 0);
+                } else {
+                    // u and v of the closest hit once more, by the steps of its test
+                    const float4 v1 = __ldg(woop + 3 * (int64_t)r.hit + 1), v2 = __ldg(woop + 3 * (int64_t)r.hit + 2);
+                    const float hu = __fmaf_rn(r.hit_t, __fmaf_rn(r.dz, v1.z, __fmaf_rn(r.dy, v1.y, __fmul_rn(r.dx, v1.x))),
+                        __fmaf_rn(r.oz, v1.z, __fmaf_rn(r.oy, v1.y, __fmaf_rn(r.ox, v1.x, v1.w))));
+                    const float hv = __fmaf_rn(r.hit_t, __fmaf_rn(r.dz, v2.z, __fmaf_rn(r.dx, v2.x, __fmul_rn(r.dy, v2.y))),
+                        __fmaf_rn(r.oz, v2.z, __fmaf_rn(r.oy, v2.y, __fmaf_rn(r.ox, v2.x, v2.w))));
+                    results[ray] = make_int4(__ldg(tri_idx + r.hit), __float_as_int(r.hit_t),
+                                             __float_as_int(hu), __float_as_int(hv));
+                    if (STATS) stats[ray] = make_int2(r.nodes, r.tris);
+                }
+                ray = -1;
+            }
+            if (exhausted) break;  // every lane is idle
             unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(ray_counter, (unsigned long long)__popc(need_mask));
+            const int leader = __ffs(idle_mask) - 1;
+            if (lane == leader) base = atomicAdd(ray_counter, (unsigned long long)__popc(idle_mask));
             base = __shfl_sync(HP_FULL_MASK, base, leader);
-            if (need) {
-                const int64_t slot = (int64_t)base + __popc(need_mask & lt_mask);
+            exhausted = (int64_t)base + __popc(idle_mask) >= num_rays;
+            const int64_t slot = (int64_t)base + __popc(idle_mask & ((1u << lane) - 1u));
+            if (idle && slot < num_rays) {
                 // traceSort: slot k traces ray order[k] (rays in Morton order)
-                const int64_t id = (order && slot < num_rays) ? (int64_t)__ldg(order + slot) : slot;
-                if (slot < num_rays && (uint64_t)id >= (uint64_t)num_rays) {
+                const int64_t id = order ? (int64_t)__ldg(order + slot) : slot;
+                if ((uint64_t)id >= (uint64_t)num_rays) {
                     hp_report(err, HP_DEV_BAD_INDEX, (int)slot);
-                    exhausted = true;
-                } else if (id < num_rays) {
+                } else {
                     ray = id;
                     const float4 o = __ldg(rays + 2 * id), d = __ldg(rays + 2 * id + 1);
                     r.ox = o.x; r.oy = o.y; r.oz = o.z; r.tmin = o.w;
@@ -107,11 +169,9 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? 9 : 12) k_trace(
                     r.oody = __fmul_rn(o.y, r.idy);
                     r.oodz = __fmul_rn(o.z, r.idz);
                     r.hit = -1;
-                    r.hit_u = r.hit_v = 0.0f;
                     r.nodes = r.tris = 0;
                     sp = 0;
                     steps = 0;
-                    leaf = 0;
                     node = 0;
                     if (BATCH) {
                         const hp_batch_seg& g = segs[seg_search(ray_off, num_segs, id)];
@@ -120,106 +180,103 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? 9 : 12) k_trace(
                         tri_idx = tri_all + g.tri_off;
                         num_refs = g.n;
                         max_nodes = max(2 * g.n - 1, 3);
-                        if (g.n == 0) {  // empty mesh: the ray misses
-                            reinterpret_cast<int2*>(results)[2 * id] = make_int2(-1, __float_as_int(d.w));
-                            if (STATS) stats[id] = make_int2(0, 0);
-                            node = SENTINEL;
-                        }
+                        if (g.n == 0) node = SENTINEL;  // empty mesh: the ray misses
                     }
-                } else {
-                    exhausted = true;
                 }
             }
         }
-        if (__all_sync(HP_FULL_MASK, node == SENTINEL)) {
-            if (!BATCH || __all_sync(HP_FULL_MASK, exhausted)) break;
-            continue;  // every lane drew a ray of an empty mesh
-        }
 
-        // Traverse until fewer than FETCH_THRESHOLD lanes of the warp still hold
-        // a ray; the warp reconverges after every round so that the decision
-        // (and the refill that follows) is taken by all 32 lanes together.
-        while (true) {
-          if (node != SENTINEL) {
-            // Interior nodes. The first leaf a lane reaches is postponed and the
-            // lane keeps traversing until every lane still traversing holds a
-            // leaf (or finishes); then the leaves are tested together.
-            while ((unsigned)node < (unsigned)SENTINEL) {
+        // Interior nodes: one per lane and round.
+        bool go = (unsigned)node < (unsigned)SENTINEL;
+        unsigned mask = __ballot_sync(HP_FULL_MASK, go);
+        while (mask) {
+            if (go) {
                 if (node >= max_nodes || ++steps > TRAVERSAL_LIMIT) {
                     hp_report(err, HP_DEV_BAD_INDEX, node);
                     node = SENTINEL;
                     leaf = 0;
-                    break;
-                }
-                if (STATS) ++r.nodes;
-                const float4* np = nodes + 4 * (int64_t)node;
-                float4 n0, n1, nz, nm;
-                ld32(np, n0, n1);
-                ld32(np + 2, nz, nm);
-                const float c0lox = __fmaf_rn(n0.x, r.idx_, -r.oodx);
-                const float c0hix = __fmaf_rn(n0.y, r.idx_, -r.oodx);
-                const float c0loy = __fmaf_rn(n0.z, r.idy, -r.oody);
-                const float c0hiy = __fmaf_rn(n0.w, r.idy, -r.oody);
-                const float c0loz = __fmaf_rn(nz.x, r.idz, -r.oodz);
-                const float c0hiz = __fmaf_rn(nz.y, r.idz, -r.oodz);
-                const float c1loz = __fmaf_rn(nz.z, r.idz, -r.oodz);
-                const float c1hiz = __fmaf_rn(nz.w, r.idz, -r.oodz);
-                const float c1lox = __fmaf_rn(n1.x, r.idx_, -r.oodx);
-                const float c1hix = __fmaf_rn(n1.y, r.idx_, -r.oodx);
-                const float c1loy = __fmaf_rn(n1.z, r.idy, -r.oody);
-                const float c1hiy = __fmaf_rn(n1.w, r.idy, -r.oody);
-                const float c0min = fmaxf(fmaxf(fminf(c0lox, c0hix), fminf(c0loy, c0hiy)),
-                                          fmaxf(fminf(c0loz, c0hiz), r.tmin));
-                const float c0max = fminf(fminf(fmaxf(c0lox, c0hix), fmaxf(c0loy, c0hiy)),
-                                          fminf(fmaxf(c0loz, c0hiz), r.hit_t));
-                const float c1min = fmaxf(fmaxf(fminf(c1lox, c1hix), fminf(c1loy, c1hiy)),
-                                          fmaxf(fminf(c1loz, c1hiz), r.tmin));
-                const float c1max = fminf(fminf(fmaxf(c1lox, c1hix), fmaxf(c1loy, c1hiy)),
-                                          fminf(fmaxf(c1loz, c1hiz), r.hit_t));
-                const bool t0 = c0max >= c0min, t1 = c1max >= c1min;
-                int c0 = __float_as_int(nm.x), c1 = __float_as_int(nm.y);
-                if (!t0 && !t1) {
-                    if (sp == 0) node = SENTINEL;
-                    else { --sp; node = sp < SSTACK ? sstack[sp * TRACE_BLOCK] : lstack[sp - SSTACK]; }
+                    tri = tri_end = 0;
                 } else {
-                    node = t0 ? c0 : c1;
+                    if (STATS) ++r.nodes;
+                    const float4* np = nodes + 4 * (int64_t)node;
+                    float4 n0, n1, nz, nm;
+                    ld32(np, n0, n1);
+                    ld32(np + 2, nz, nm);
+                    const float c0lox = __fmaf_rn(n0.x, r.idx_, -r.oodx);
+                    const float c0hix = __fmaf_rn(n0.y, r.idx_, -r.oodx);
+                    const float c0loy = __fmaf_rn(n0.z, r.idy, -r.oody);
+                    const float c0hiy = __fmaf_rn(n0.w, r.idy, -r.oody);
+                    const float c0loz = __fmaf_rn(nz.x, r.idz, -r.oodz);
+                    const float c0hiz = __fmaf_rn(nz.y, r.idz, -r.oodz);
+                    const float c1loz = __fmaf_rn(nz.z, r.idz, -r.oodz);
+                    const float c1hiz = __fmaf_rn(nz.w, r.idz, -r.oodz);
+                    const float c1lox = __fmaf_rn(n1.x, r.idx_, -r.oodx);
+                    const float c1hix = __fmaf_rn(n1.y, r.idx_, -r.oodx);
+                    const float c1loy = __fmaf_rn(n1.z, r.idy, -r.oody);
+                    const float c1hiy = __fmaf_rn(n1.w, r.idy, -r.oody);
+                    const float c0min = fmaxf(fmaxf(fminf(c0lox, c0hix), fminf(c0loy, c0hiy)),
+                                              fmaxf(fminf(c0loz, c0hiz), r.tmin));
+                    const float c0max = fminf(fminf(fmaxf(c0lox, c0hix), fmaxf(c0loy, c0hiy)),
+                                              fminf(fmaxf(c0loz, c0hiz), r.hit_t));
+                    const float c1min = fmaxf(fmaxf(fminf(c1lox, c1hix), fminf(c1loy, c1hiy)),
+                                              fmaxf(fminf(c1loz, c1hiz), r.tmin));
+                    const float c1max = fminf(fminf(fmaxf(c1lox, c1hix), fmaxf(c1loy, c1hiy)),
+                                              fminf(fmaxf(c1loz, c1hiz), r.hit_t));
+                    const bool t0 = c0max >= c0min, t1 = c1max >= c1min;
+                    const int c0 = __float_as_int(nm.x), c1 = __float_as_int(nm.y);
+                    const bool swap = t1 && (!t0 || c1min < c0min);
+                    node = swap ? c1 : c0;
                     if (t0 && t1) {
-                        int far = c1;
-                        if (c1min < c0min) { node = c1; far = c0; }
-                        if (sp < SSTACK) sstack[sp * TRACE_BLOCK] = far;
-                        else if (sp < SSTACK + LSTACK) lstack[sp - SSTACK] = far;
+                        const int2 far = make_int2(swap ? c0 : c1, __float_as_int(swap ? c0min : c1min));
+                        if (sp < SST) sstack[sp * TRACE_BLOCK] = far;
+                        else if (sp < STACK) lstack[sp - SST] = far;
                         else { hp_report(err, HP_DEV_STACK_OVERFLOW, (int)ray); --sp; }
                         ++sp;
                     }
+                    if (!t0 && !t1) pop();
+                    if (node < 0 && leaf >= 0 && tri >= tri_end) {  // the first leaf is postponed
+                        leaf = node;
+                        pop();
+                    }
                 }
-                if (node < 0 && leaf >= 0) {  // postpone the first leaf
-                    leaf = node;
-                    if (sp == 0) node = SENTINEL;
-                    else { --sp; node = sp < SSTACK ? sstack[sp * TRACE_BLOCK] : lstack[sp - SSTACK]; }
-                }
-                if (!__any_sync(__activemask(), leaf >= 0)) break;
             }
-            // Leaves: the postponed one, then `node` if it is a leaf too.
-            while (leaf < 0) {
-                if (~leaf >= max_nodes || ++steps > TRAVERSAL_LIMIT) {
-                    hp_report(err, HP_DEV_BAD_INDEX, leaf);
-                    node = SENTINEL;
+            go = (unsigned)node < (unsigned)SENTINEL;
+            mask = __ballot_sync(HP_FULL_MASK, go && leaf >= 0 && tri >= tri_end);
+            if (__popc(mask) < NODE_MIN) break;
+        }
+
+        // Leaves: one triangle per lane and round.
+        bool pend = node < 0 || leaf < 0 || tri < tri_end;
+        mask = __ballot_sync(HP_FULL_MASK, pend);
+        while (mask) {
+            if (pend) {
+                if (leaf >= 0 && tri >= tri_end) {  // the leaf that the lane stopped at
+                    leaf = node;
+                    pop();
+                }
+                if (leaf < 0) {
+                    const int li = ~leaf;
                     leaf = 0;
-                    break;
+                    tri = tri_end = 0;
+                    if (li >= max_nodes || ++steps > TRAVERSAL_LIMIT) {
+                        hp_report(err, HP_DEV_BAD_INDEX, li);
+                        node = SENTINEL;
+                        sp = 0;
+                    } else {
+                        const int2 lm = __ldg(reinterpret_cast<const int2*>(nodes + 4 * (int64_t)li + 3));
+                        if (lm.x < 0 || lm.y > num_refs || lm.x > lm.y) {
+                            hp_report(err, HP_DEV_BAD_INDEX, lm.x);
+                        } else {
+                            tri = lm.x;
+                            tri_end = lm.y;
+                        }
+                    }
                 }
-                const float4 lm = __ldg(nodes + 4 * (int64_t)(~leaf) + 3);
-                int begin = __float_as_int(lm.x), end = __float_as_int(lm.y);
-                if (begin < 0 || end > num_refs || begin > end) {
-                    hp_report(err, HP_DEV_BAD_INDEX, begin);
-                    begin = end = 0;
-                }
-                for (int tri = begin; tri < end; ++tri) {
+                if (tri < tri_end) {
                     if (STATS) ++r.tris;
-                    // The first two Woop rows at once (the second is needed whenever the
-                    // plane is hit in range): one round trip fewer per tested triangle;
-                    // the third when u >= 0.
-                    const float4 v0 = __ldg(woop + 3 * (int64_t)tri);
-                    const float4 v1 = __ldg(woop + 3 * (int64_t)tri + 1);
+                    const float4* wp = woop + 3 * (int64_t)tri;
+                    const float4 v0 = __ldg(wp);
+                    const float4 v1 = __ldg(wp + 1);
                     const float oz = __fmaf_rn(-r.oz, v0.z, __fmaf_rn(-r.oy, v0.y, __fmaf_rn(-r.ox, v0.x, v0.w)));
                     // The roundings of the reference's fast-math tracer, measured
                     // against its output on sm_100a: the chains o.w +- ... are
@@ -237,40 +294,23 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? 9 : 12) k_trace(
                         const float dx = __fmaf_rn(r.dz, v1.z, __fmaf_rn(r.dy, v1.y, __fmul_rn(r.dx, v1.x)));
                         const float u = __fmaf_rn(t, dx, ox);
                         if (u >= 0.0f) {
-                            const float4 v2 = __ldg(woop + 3 * (int64_t)tri + 2);
+                            const float4 v2 = __ldg(wp + 2);
                             const float oy = __fmaf_rn(r.oz, v2.z, __fmaf_rn(r.oy, v2.y, __fmaf_rn(r.ox, v2.x, v2.w)));
                             const float dy = __fmaf_rn(r.dz, v2.z, __fmaf_rn(r.dx, v2.x, __fmul_rn(r.dy, v2.y)));
                             const float v = __fmaf_rn(t, dy, oy);
                             if (v >= 0.0f && __fadd_rn(u, v) <= 1.0f) {
                                 r.hit_t = t;
                                 r.hit = tri;
-                                r.hit_u = u;
-                                r.hit_v = v;
-                                if (ANY_HIT) { sp = 0; break; }
+                                if (ANY_HIT) { node = SENTINEL; sp = 0; tri = tri_end; }
                             }
                         }
                     }
-                }
-                if (ANY_HIT && r.hit >= 0) { node = SENTINEL; leaf = 0; break; }
-                leaf = node;
-                if (node < 0) {
-                    if (sp == 0) node = SENTINEL;
-                    else { --sp; node = sp < SSTACK ? sstack[sp * TRACE_BLOCK] : lstack[sp - SSTACK]; }
+                    ++tri;
                 }
             }
-            if (node == SENTINEL) {
-                if (r.hit < 0) {
-                    reinterpret_cast<int2*>(results)[2 * ray] = make_int2(-1, __float_as_int(r.hit_t));
-                    if (STATS) stats[ray] = make_int2(0, 0);
-                } else {
-                    results[ray] = make_int4(__ldg(tri_idx + r.hit), __float_as_int(r.hit_t),
-                                             __float_as_int(r.hit_u), __float_as_int(r.hit_v));
-                    if (STATS) stats[ray] = make_int2(r.nodes, r.tris);
-                }
-            }
-          }
-          __syncwarp();
-          if (__popc(__ballot_sync(HP_FULL_MASK, node != SENTINEL)) < FETCH_THRESHOLD) break;
+            pend = node < 0 || leaf < 0 || tri < tri_end;
+            mask = __ballot_sync(HP_FULL_MASK, pend);
+            if (__popc(mask) < TRI_MIN) break;
         }
     }
 }

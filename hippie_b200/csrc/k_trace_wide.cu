@@ -12,13 +12,14 @@
 //     and pushes the other hits farthest first, so the nearest of them is
 //     popped next; a sub-warp per ray left most lanes idle on nodes with few
 //     hit children and made every leaf's few triangles a shuffle reduction;
-//   * the first leaf a lane reaches is postponed until every lane still
-//     traversing holds one, then the leaves are tested together (as in the
-//     binary tracer);
-//   * persistent warps take rays with one atomic per warp when fewer than 20
-//     lanes still hold one, as in the binary tracer; the per-ray stack keeps
-//     its first entries in shared memory and the rest in local memory, and an
-//     overflow is reported as a device error instead of overrunning;
+//   * a warp takes turns at nodes, triangles and new rays, all 32 lanes together,
+//     as in the binary tracer (k_trace_impl.cuh says why); the first leaf a lane
+//     reaches is postponed; a stack entry keeps the child's entry distance and is
+//     dropped at the pop when a closer hit has been found since. On a B200, 1 M
+//     bounce rays in 0.5 M triangles (Quad) 1.46 -> 1.08 ms;
+//   * persistent warps take rays with one atomic per warp; the per-ray stack
+//     keeps its first entries in shared memory and the rest in local memory, and
+//     an overflow is reported as a device error instead of overrunning;
 //   * the slab and Woop arithmetic is the binary tracer's, written out step by
 //     step, and closest-hit ties in t go to the lower triangle id, so both
 //     layouts return the same hits.
@@ -41,34 +42,38 @@ __device__ __forceinline__ float safe_rcp(float d) {
 // loads), tests its N child boxes itself, continues with the nearest hit
 // child and pushes the other hits farthest first, so the nearest of them is
 // popped next. Rays are taken by persistent warps as in the binary tracer
-// (refill when fewer than RF lanes still hold a ray); each lane's stack keeps
+// (once FETCH1 lanes are without work); each lane's stack keeps
 // SST entries in shared memory (one column per thread) and the rest in local
 // memory. Leaves are tested by the lane, with the binary tracer's Woop
 // arithmetic and tie rule, so the hits equal the binary layout's.
 constexpr int TB1 = 128;
 constexpr int SST1 = 16;
-constexpr int RF1 = 20;
+// Turns (see k_trace_impl.cuh) and CTAs per SM, swept on a B200 with 2 M bounce rays
+// in 1 M triangles, shadow rays and primary rays: Quad 2.85 -> 2.02 ms, 1.16 ->
+// 0.96 ms and 0.69 -> 0.54 ms, Oct 3.56 -> 2.52 ms, 1.32 -> 1.17 ms and 0.78 -> 0.61
+// ms. Quad at 10 CTAs (48 registers, spills) is 8 % slower than at 8, Oct at 6 or 5
+// CTAs 8 or 16 % slower on bounce rays than at 8.
+constexpr int FETCH1 = 12, NODE1 = 12, TRI1 = 8, CTAS1 = 8;
 constexpr int SENT1 = 0x76543210;
 template <int N> struct wide1_cfg;
 template <> struct wide1_cfg<4> { static constexpr int STACK = 64; };
 template <> struct wide1_cfg<8> { static constexpr int STACK = 96; };
 
 template <int N, bool ANY_HIT, bool STATS>
-__global__ void __launch_bounds__(TB1, N == 4 ? 10 : 8) k_trace_wide1(const float4* __restrict__ rays, int64_t num_rays,
+__global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __restrict__ rays, int64_t num_rays,
                                                    int4* __restrict__ results, int2* __restrict__ stats,
                                                    const int4* __restrict__ nodes, const float4* __restrict__ woop,
                                                    const int32_t* __restrict__ tri_idx, int max_nodes, int num_refs,
                                                    unsigned long long* ray_counter, int* err,
                                                    const int32_t* __restrict__ order) {
     constexpr int STACK = wide1_cfg<N>::STACK, LST = STACK - SST1;
-    __shared__ int s_stack[SST1 * TB1];
-    int* sstack = s_stack + threadIdx.x;
-    // Entries past the shared part. Left uninitialised: sp counts the pushes
-    // that were stored (an overflowing push is dropped and reported), so a pop
-    // reads only entries a push wrote.
-    int lstack[LST];
+    __shared__ int2 s_stack[SST1 * TB1];
+    int2* sstack = s_stack + threadIdx.x;
+    // Entries (child, entry distance) past the shared part. Left uninitialised: sp
+    // counts the pushes that were stored (an overflowing push is dropped and
+    // reported), so a pop reads only entries a push wrote.
+    int2 lstack[LST];
     const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1u;
 
     float ox = 0, oy = 0, oz = 0, tmin = 0, dx = 0, dy = 0, dz = 0;
     float ix = 0, iy = 0, iz = 0, oodx = 0, oody = 0, oodz = 0;
@@ -76,39 +81,56 @@ __global__ void __launch_bounds__(TB1, N == 4 ? 10 : 8) k_trace_wide1(const floa
     int hit = -1;  // leaf-ordered reference of the closest hit
     int64_t ray = -1;
     int node = SENT1, sp = 0, steps = 0, n_nodes = 0, n_tris = 0;
-    int leaf = 0;  // postponed leaf (~index), >= 0 when none
-    bool exhausted = false;
+    int leaf = 0;              // postponed leaf (~index) whose range is not loaded yet, 0 when none
+    int tri = 0, tri_end = 0;  // triangles of the postponed leaf still to test
+    bool exhausted = false;    // warp-uniform: the counter has run past the rays
     auto pop = [&]() {
-        if (sp == 0) {
-            node = SENT1;
-        } else {
+        node = SENT1;
+        while (sp > 0) {
             --sp;
-            node = sp < SST1 ? sstack[sp * TB1] : lstack[sp - SST1];
+            const int2 e = sp < SST1 ? sstack[sp * TB1] : lstack[sp - SST1];
+            if (STATS || !(__int_as_float(e.y) > hit_t)) {
+                node = e.x;
+                break;
+            }
         }
     };
-    auto push = [&](int v) {
-        if (sp < SST1) sstack[sp * TB1] = v;
-        else if (sp < STACK) lstack[sp - SST1] = v;
+    auto push = [&](int v, uint32_t key) {
+        const int2 e = make_int2(v, __float_as_int(hp_ord2f(key)));
+        if (sp < SST1) sstack[sp * TB1] = e;
+        else if (sp < STACK) lstack[sp - SST1] = e;
         else { hp_report(err, HP_DEV_STACK_OVERFLOW, (int)ray); --sp; }
         ++sp;
     };
 
     while (true) {
-        // Refill lanes whose ray is finished (one atomic per warp).
-        const bool need = node == SENT1 && !exhausted;
-        const unsigned need_mask = __ballot_sync(HP_FULL_MASK, need);
-        if (need_mask) {
-            const int leader = __ffs(need_mask) - 1;
+        // Finished lanes write their results and take new rays (one atomic per warp).
+        const bool idle = node == SENT1 && leaf >= 0 && tri >= tri_end;
+        const unsigned idle_mask = __ballot_sync(HP_FULL_MASK, idle);
+        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= FETCH1)) {
+            if (idle && ray >= 0) {
+                if (hit < 0) {
+                    reinterpret_cast<int2*>(results)[2 * ray] = make_int2(-1, __float_as_int(hit_t));
+                    if (STATS) stats[ray] = make_int2(0, 0);
+                } else {
+                    results[ray] = make_int4(__ldg(tri_idx + hit), __float_as_int(hit_t), __float_as_int(hit_u),
+                                             __float_as_int(hit_v));
+                    if (STATS) stats[ray] = make_int2(n_nodes, n_tris);
+                }
+                ray = -1;
+            }
+            if (exhausted) break;  // every lane is idle
             unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(ray_counter, (unsigned long long)__popc(need_mask));
+            const int leader = __ffs(idle_mask) - 1;
+            if (lane == leader) base = atomicAdd(ray_counter, (unsigned long long)__popc(idle_mask));
             base = __shfl_sync(HP_FULL_MASK, base, leader);
-            if (need) {
-                const int64_t slot = (int64_t)base + __popc(need_mask & lt_mask);
-                const int64_t id = (order && slot < num_rays) ? (int64_t)__ldg(order + slot) : slot;
-                if (slot < num_rays && (uint64_t)id >= (uint64_t)num_rays) {
+            exhausted = (int64_t)base + __popc(idle_mask) >= num_rays;
+            const int64_t slot = (int64_t)base + __popc(idle_mask & ((1u << lane) - 1u));
+            if (idle && slot < num_rays) {
+                const int64_t id = order ? (int64_t)__ldg(order + slot) : slot;
+                if ((uint64_t)id >= (uint64_t)num_rays) {
                     hp_report(err, HP_DEV_BAD_INDEX, (int)slot);
-                    exhausted = true;
-                } else if (id < num_rays) {
+                } else {
                     ray = id;
                     const float4 o = __ldg(rays + 2 * id), d = __ldg(rays + 2 * id + 1);
                     ox = o.x; oy = o.y; oz = o.z; tmin = o.w;
@@ -118,24 +140,21 @@ __global__ void __launch_bounds__(TB1, N == 4 ? 10 : 8) k_trace_wide1(const floa
                     hit = -1; hit_u = hit_v = 0.0f;
                     sp = 0; steps = 0; n_nodes = n_tris = 0;
                     node = 0;
-                    leaf = 0;
-                } else {
-                    exhausted = true;
                 }
             }
         }
-        if (__all_sync(HP_FULL_MASK, node == SENT1)) break;
 
-        while (true) {
-            if (node != SENT1) {
-                // interior nodes
-                while ((unsigned)node < (unsigned)SENT1) {
-                    if (node >= max_nodes || ++steps > TRAVERSAL_LIMIT) {
-                        hp_report(err, HP_DEV_BAD_INDEX, node);
-                        node = SENT1;
-                        leaf = 0;
-                        break;
-                    }
+        // Interior nodes: one per lane and round.
+        bool go = (unsigned)node < (unsigned)SENT1;
+        unsigned mask = __ballot_sync(HP_FULL_MASK, go);
+        while (mask) {
+            if (go) {
+                if (node >= max_nodes || ++steps > TRAVERSAL_LIMIT) {
+                    hp_report(err, HP_DEV_BAD_INDEX, node);
+                    node = SENT1;
+                    leaf = 0;
+                    tri = tri_end = 0;
+                } else {
                     if (STATS) ++n_nodes;
                     const int4* np = nodes + (size_t)node * 2 * N;
                     float4 xy[N];
@@ -183,75 +202,77 @@ __global__ void __launch_bounds__(TB1, N == 4 ? 10 : 8) k_trace_wide1(const floa
                     } else {
 #pragma unroll
                         for (int i = N - 1; i >= 1; --i)
-                            if (key[i] != 0xFFFFFFFFu) push(ref[i]);
+                            if (key[i] != 0xFFFFFFFFu) push(ref[i], key[i]);
                         node = ref[0];
                     }
-                    // The first leaf a lane reaches waits until every lane still
-                    // traversing holds one; then the leaves are tested together.
-                    if (node < 0 && leaf >= 0) {
+                    if (node < 0 && leaf >= 0 && tri >= tri_end) {  // the first leaf is postponed
                         leaf = node;
                         pop();
                     }
-                    if (!__any_sync(__activemask(), leaf >= 0)) break;
                 }
-                // leaves: the postponed one, then `node` if it is a leaf too
-                while (leaf < 0) {
+            }
+            go = (unsigned)node < (unsigned)SENT1;
+            mask = __ballot_sync(HP_FULL_MASK, go && leaf >= 0 && tri >= tri_end);
+            if (__popc(mask) < NODE1) break;
+        }
+
+        // Leaves: one triangle per lane and round.
+        bool pend = node < 0 || leaf < 0 || tri < tri_end;
+        mask = __ballot_sync(HP_FULL_MASK, pend);
+        while (mask) {
+            if (pend) {
+                if (leaf >= 0 && tri >= tri_end) {  // the leaf that the lane stopped at
+                    leaf = node;
+                    pop();
+                }
+                if (leaf < 0) {
                     const int li = ~leaf;
+                    leaf = 0;
+                    tri = tri_end = 0;
                     if (li >= max_nodes || ++steps > TRAVERSAL_LIMIT) {
                         hp_report(err, HP_DEV_BAD_INDEX, li);
                         node = SENT1;
-                        leaf = 0;
-                        break;
+                        sp = 0;
+                    } else {
+                        const int4 q = __ldg(nodes + (size_t)li * 2 * N + N);
+                        if (q.z < 0 || q.w > num_refs || q.z > q.w) {
+                            hp_report(err, HP_DEV_BAD_INDEX, q.z);
+                        } else {
+                            tri = q.z;
+                            tri_end = q.w;
+                        }
                     }
-                    const int4 q = __ldg(nodes + (size_t)li * 2 * N + N);
-                    int begin = q.z, end = q.w;
-                    if (begin < 0 || end > num_refs || begin > end) {
-                        hp_report(err, HP_DEV_BAD_INDEX, begin);
-                        begin = end = 0;
-                    }
-                    bool done = false;
-                    for (int tri = begin; tri < end; ++tri) {
-                        if (STATS) ++n_tris;
-                        const float4 v0 = __ldg(woop + 3 * (int64_t)tri);
-                        const float4 v1 = __ldg(woop + 3 * (int64_t)tri + 1);
-                        const float ozz = __fmaf_rn(-oz, v0.z, __fmaf_rn(-oy, v0.y, __fmaf_rn(-ox, v0.x, v0.w)));
-                        const float den = __fmaf_rn(dz, v0.z, __fmaf_rn(dx, v0.x, __fmul_rn(dy, v0.y)));
-                        const float t = __fmul_rn(ozz, __frcp_rn(den));
-                        bool closer = t < hit_t;
-                        if (!closer && t == hit_t && hit >= 0) closer = __ldg(tri_idx + tri) < __ldg(tri_idx + hit);
-                        if (t > tmin && closer) {
-                            const float oxx = __fmaf_rn(oz, v1.z, __fmaf_rn(oy, v1.y, __fmaf_rn(ox, v1.x, v1.w)));
-                            const float dxx = __fmaf_rn(dz, v1.z, __fmaf_rn(dy, v1.y, __fmul_rn(dx, v1.x)));
-                            const float u = __fmaf_rn(t, dxx, oxx);
-                            if (u >= 0.0f) {
-                                const float4 v2 = __ldg(woop + 3 * (int64_t)tri + 2);
-                                const float oyy = __fmaf_rn(oz, v2.z, __fmaf_rn(oy, v2.y, __fmaf_rn(ox, v2.x, v2.w)));
-                                const float dyy = __fmaf_rn(dz, v2.z, __fmaf_rn(dx, v2.x, __fmul_rn(dy, v2.y)));
-                                const float v = __fmaf_rn(t, dyy, oyy);
-                                if (v >= 0.0f && __fadd_rn(u, v) <= 1.0f) {
-                                    hit_t = t; hit = tri; hit_u = u; hit_v = v;
-                                    if (ANY_HIT) { done = true; break; }
-                                }
+                }
+                if (tri < tri_end) {
+                    if (STATS) ++n_tris;
+                    const float4 v0 = __ldg(woop + 3 * (int64_t)tri);
+                    const float4 v1 = __ldg(woop + 3 * (int64_t)tri + 1);
+                    const float ozz = __fmaf_rn(-oz, v0.z, __fmaf_rn(-oy, v0.y, __fmaf_rn(-ox, v0.x, v0.w)));
+                    const float den = __fmaf_rn(dz, v0.z, __fmaf_rn(dx, v0.x, __fmul_rn(dy, v0.y)));
+                    const float t = __fmul_rn(ozz, __frcp_rn(den));
+                    bool closer = t < hit_t;
+                    if (!closer && t == hit_t && hit >= 0) closer = __ldg(tri_idx + tri) < __ldg(tri_idx + hit);
+                    if (t > tmin && closer) {
+                        const float oxx = __fmaf_rn(oz, v1.z, __fmaf_rn(oy, v1.y, __fmaf_rn(ox, v1.x, v1.w)));
+                        const float dxx = __fmaf_rn(dz, v1.z, __fmaf_rn(dy, v1.y, __fmul_rn(dx, v1.x)));
+                        const float u = __fmaf_rn(t, dxx, oxx);
+                        if (u >= 0.0f) {
+                            const float4 v2 = __ldg(woop + 3 * (int64_t)tri + 2);
+                            const float oyy = __fmaf_rn(oz, v2.z, __fmaf_rn(oy, v2.y, __fmaf_rn(ox, v2.x, v2.w)));
+                            const float dyy = __fmaf_rn(dz, v2.z, __fmaf_rn(dx, v2.x, __fmul_rn(dy, v2.y)));
+                            const float v = __fmaf_rn(t, dyy, oyy);
+                            if (v >= 0.0f && __fadd_rn(u, v) <= 1.0f) {
+                                hit_t = t; hit = tri; hit_u = u; hit_v = v;
+                                if (ANY_HIT) { node = SENT1; sp = 0; tri = tri_end; }
                             }
                         }
                     }
-                    if (done) { sp = 0; node = SENT1; leaf = 0; break; }
-                    leaf = node;
-                    if (node < 0) pop();
-                }
-                if (node == SENT1) {
-                    if (hit < 0) {
-                        reinterpret_cast<int2*>(results)[2 * ray] = make_int2(-1, __float_as_int(hit_t));
-                        if (STATS) stats[ray] = make_int2(0, 0);
-                    } else {
-                        results[ray] = make_int4(__ldg(tri_idx + hit), __float_as_int(hit_t), __float_as_int(hit_u),
-                                                 __float_as_int(hit_v));
-                        if (STATS) stats[ray] = make_int2(n_nodes, n_tris);
-                    }
+                    ++tri;
                 }
             }
-            __syncwarp();
-            if (__popc(__ballot_sync(HP_FULL_MASK, node != SENT1)) < RF1) break;
+            pend = node < 0 || leaf < 0 || tri < tri_end;
+            mask = __ballot_sync(HP_FULL_MASK, pend);
+            if (__popc(mask) < TRI1) break;
         }
     }
 }

@@ -61,20 +61,31 @@ __host__ __device__ constexpr int fused_tile(int r) { return 2 * r <= LPB / 2 ? 
 // Clusters of a tile of the long lists: 4*LPB - 2r, at least 2*LPB.
 __host__ __device__ constexpr int long_tile(int r) { return 2 * r <= 2 * LPB ? NB4 * LPB - 2 * r : 2 * LPB; }
 constexpr size_t LOOP_SMEM = 6 * WIN * sizeof(float) + NNF * sizeof(int);
-constexpr int TAIL = 2048;          // clusters finished by a single CTA
+constexpr int TAIL = 2048;          // most clusters finished by a single CTA
+// Clusters that the iteration kernel leaves to it (an iteration of the CTA takes 6 us
+// at 650 clusters, 4 us at 450 and 2.4 us below 60, one of the short lists' tiles 8 us;
+// leaving at 512 or 1,200 instead: equal, and 2 % slower on a build of 100 K).
+constexpr int LOOP_END = 768;
 constexpr int TAIL_ITEMS = TAIL / PB;
+constexpr int LOOP_MAX_GRID = 1024; // most CTAs of the iteration kernel
 constexpr int MAX_ITER = 1 << 16;
 constexpr unsigned SPIN = 1u << 22;
 
-// Acquire load / release store at GPU scope: a record written before the
-// release store is visible to a thread whose acquire load sees the flag.
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
+// A collapse record travels as one 128-bit word, so that the reader that finds
+// its last part set has the others too: no flag beside it, no fence, and one round
+// trip to L2 a level instead of two (the collapse of 100 K PLOC references
+// 0.102 -> 0.076 ms, of 4.2 M 0.491 -> 0.424 ms, of 1 M ATR references 0.34 -> 0.23 ms).
+__device__ __forceinline__ int4 ld_record(const int4* p) {
+    unsigned long long a, b;
+    asm volatile("{\n.reg .b128 t;\nld.relaxed.gpu.global.b128 t, [%2];\nmov.b128 {%0, %1}, t;\n}"
+                 : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    return make_int4((int)a, (int)(a >> 32), (int)b, (int)(b >> 32));
 }
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_record(int4* p, int4 v) {
+    const unsigned long long a = (unsigned)v.x | ((unsigned long long)(unsigned)v.y << 32);
+    const unsigned long long b = (unsigned)v.z | ((unsigned long long)(unsigned)v.w << 32);
+    asm volatile("{\n.reg .b128 t;\nmov.b128 t, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], t;\n}"
+                 ::"l"(p), "l"(a), "l"(b) : "memory");
 }
 __device__ __forceinline__ unsigned long long ld_vol_u64(const unsigned long long* p) {
     unsigned long long v;
@@ -122,9 +133,6 @@ __device__ __forceinline__ float half_area(float ax, float ay, float az, float b
 __device__ __forceinline__ int radius_at(const ploc_args& a, int it) {
     return a.adaptive_r ? min(a.radius + it + 1, a.max_radius) : a.radius;
 }
-
-// Bounded grid barrier (generation counter). Returns false if it gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, int* err) { return hp_grid_barrier(bar, err, SPIN); }
 
 // Create node `node` = merge of clusters with node ids a (left) and b (right).
 // From the children's boxes (w: cost / size bits) and counts; returns the new
@@ -495,18 +503,194 @@ __device__ void merge_tile(const ploc_args& A, const int* __restrict__ cl_in, in
     }
 }
 
+// ---- short lists: one tile per CTA ------------------------------------------------
+// From about 0.14 M clusters down every CTA has at most one tile, and an iteration
+// is latency: it loads its window, finds neighbours, learns what the tiles before it
+// merge and keep, writes, and meets the others. Measured with one thread per cluster,
+// a look-back and a barrier of all 296 CTAs on a B200: 4.5 + 0.6 + 1.7 + 1.1 + 4.7 us,
+// the list 17 % shorter each time. So:
+//   * S = 2, 4 or 8 lanes per cluster walk its candidates as soon as tiles of the
+//     clusters that then fit a CTA's threads still find a CTA each;
+//   * every tile publishes its two counts in a word of its own, and every CTA reads
+//     the words of all tiles: the sums below its own tile, and the next list's length,
+//     which nobody has to fetch after the barrier;
+//   * once half of the CTAs are enough the others leave, and the barrier is one
+//     arrival and one awaited word.
+// An iteration of a short list then takes 8 us instead of 12.5: the iterations and the
+// tail of a build of 100,003 triangles 0.420 -> 0.325 ms.
+// Word of a tile: iteration + 1 above 32 bits, merges above 16, survivors.
+struct small_state {
+    int n;       // length of the next list
+    int ok;
+};
+
+// Clusters of a tile with S lanes per cluster (0: none).
+__host__ __device__ constexpr int small_tile(int r, int S) { return LPB / S - 2 * r >= 32 ? LPB / S - 2 * r : 0; }
+
+__device__ void small_iteration(const ploc_args& A, const int* __restrict__ cl_in, int* __restrict__ cl_out, int N,
+                                int r, int it, int tsz, int S, float* s_win, int* s_nn, int* s_wa, int* s_wb,
+                                unsigned* s_pref, small_state* out) {
+    const int tiles = (N + tsz - 1) / tsz;
+    const int tile = blockIdx.x;
+    const int tbase = tile * tsz;
+    const bool mine = tile < tiles;
+    int em = 0, ek = 0, kind = 0, nbr = -1, node = -1, nbn = -1;
+    float4 amn{}, amx{}, bmn{}, bmx{};  // the two clusters of a merge
+    int2 ca{}, cb{};
+    if (mine) {
+        load_window(A, cl_in, N, tbase - 2 * r, tsz + 4 * r, s_win);
+        __syncthreads();
+        // neighbours of the tile's clusters and of r on each side: lanes sub, sub + S,
+        // ... of the candidates, then the least distance and of equal ones the first
+        const int shift = 31 - __clz(S);
+        const int l = threadIdx.x >> shift, sub = threadIdx.x & (S - 1);
+        const int c = tbase - r + l;
+        float best = HP_MAX_FLOAT;
+        int bi = -1;
+        if (l < tsz + 2 * r && c >= 0 && c < N) {
+            const float *mnx = s_win, *mny = s_win + WIN, *mnz = s_win + 2 * WIN;
+            const float *mxx = s_win + 3 * WIN, *mxy = s_win + 4 * WIN, *mxz = s_win + 5 * WIN;
+            const int me = l + r;
+            const float ax = mnx[me], ay = mny[me], az = mnz[me], bx = mxx[me], by = mxy[me], bz = mxz[me];
+            for (int k = l + sub; k <= l + 2 * r; k += S) {
+                if (k == me) continue;
+                const float d = half_area(fminf(ax, mnx[k]), fminf(ay, mny[k]), fminf(az, mnz[k]), fmaxf(bx, mxx[k]),
+                                          fmaxf(by, mxy[k]), fmaxf(bz, mxz[k]));
+                if (best > d) {
+                    best = d;
+                    bi = tbase - 2 * r + k;
+                }
+            }
+        }
+        for (int o = S >> 1; o > 0; o >>= 1) {
+            const float od = __shfl_xor_sync(HP_FULL_MASK, best, o);
+            const int oi = __shfl_xor_sync(HP_FULL_MASK, bi, o);
+            if (oi >= 0 && (best > od || (best == od && (unsigned)oi < (unsigned)bi))) { best = od; bi = oi; }
+        }
+        if (sub == 0 && l < tsz + 2 * r) s_nn[l] = bi;
+        __syncthreads();
+        const int nlo = tbase - r;
+        const int me = tbase + threadIdx.x;
+        if ((int)threadIdx.x < tsz && me < N) {
+            const int j = s_nn[me - nlo];
+            nbr = j;
+            const bool mutual = j >= 0 && j < N && j >= nlo && j < tbase + tsz + r && s_nn[j - nlo] == me;
+            kind = (mutual && me < j) ? 2 : ((mutual && j < me) ? 0 : 1);
+            // the node numbers, then their boxes and counts, travel meanwhile
+            if (kind != 0) node = __ldcg(cl_in + me);
+            if (kind == 2) nbn = __ldcg(cl_in + nbr);
+        }
+        em = kind == 2;
+        ek = kind != 0;
+        const int2 tot = block_scan2<LPB>(em, ek, s_wa, s_wb);
+        if (threadIdx.x == 0)
+            st_vol_u64(A.status_f + tile,
+                       ((unsigned long long)(it + 1) << 32) | ((unsigned)tot.x << 16) | (unsigned)tot.y);
+        if (kind == 2) {
+            amn = __ldcg(A.nbmin + node);
+            amx = __ldcg(A.nbmax + node);
+            bmn = __ldcg(A.nbmin + nbn);
+            bmx = __ldcg(A.nbmax + nbn);
+            ca = __ldcg(A.counts + node);
+            cb = __ldcg(A.counts + nbn);
+        }
+    }
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        unsigned pm = 0, pk = 0, am = 0;
+        bool ok = true;
+        for (int t0 = 0; t0 < tiles && ok; t0 += 32) {
+            const int t = t0 + lane;
+            unsigned long long w = 0;
+            unsigned spins = 0;
+            while (true) {
+                w = t < tiles ? ld_vol_u64(A.status_f + t) : 0;
+                const bool ready = t >= tiles || (unsigned)(w >> 32) == (unsigned)(it + 1);
+                if (__all_sync(HP_FULL_MASK, ready)) break;
+                ++spins;
+                if (spins > SPIN || ((spins & 1023u) == 0 &&
+                                     __shfl_sync(HP_FULL_MASK, *((volatile int*)A.err), 0) != 0)) {
+                    if (lane == 0) hp_report(A.err, HP_DEV_SPIN_LIMIT, tile);
+                    ok = false;
+                    break;
+                }
+            }
+            const unsigned m = ((unsigned)w >> 16) & 0xffffu, k = (unsigned)w & 0xffffu;
+            if (t < tiles) am += m;
+            if (t < tile) { pm += m; pk += k; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            pm += __shfl_xor_sync(HP_FULL_MASK, pm, o);
+            pk += __shfl_xor_sync(HP_FULL_MASK, pk, o);
+            am += __shfl_xor_sync(HP_FULL_MASK, am, o);
+        }
+        if (lane == 0) {
+            s_pref[0] = pm;
+            s_pref[1] = pk;
+            out->n = N - (int)am;
+            out->ok = ok;
+        }
+    }
+    __syncthreads();
+    if (!out->ok || kind == 0) return;
+    if (kind == 2) {
+        const int idx = (N - 2) - ((int)s_pref[0] + em);
+        float4 omn, omx;
+        int2 ocnt;
+        make_parent_from(A, idx, node, nbn, amn, amx, bmn, bmx, ca, cb, omn, omx, ocnt);
+        node = idx;
+    }
+    __stcg(cl_out + (int)s_pref[1] + ek, node);
+}
+
+// Barrier of `count` CTAs (every CTA below `count` calls it): bar[0] counts arrivals,
+// bar[1] is the generation. Bounded as hp_grid_barrier is.
+__device__ __forceinline__ bool barrier_of(unsigned* bar, unsigned count, unsigned& gen, int* err, int* s_ok) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *s_ok = 1;
+        unsigned old;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(bar) : "memory");
+        if (old == count - 1) {
+            *((volatile unsigned*)bar) = 0u;
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(bar + 1), "r"(gen + 1) : "memory");
+        } else {
+            unsigned spins = 0, now;
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar + 1) : "memory");
+                if (now != gen) break;
+                if (++spins > SPIN || ((spins & 255u) == 0 && *((volatile int*)err) != 0)) {
+                    hp_report(err, HP_DEV_SPIN_LIMIT, -1);
+                    *s_ok = 0;
+                    break;
+                }
+            }
+        }
+    }
+    ++gen;
+    __syncthreads();
+    return *s_ok != 0;
+}
+
 __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
     extern __shared__ float s_win[];
     int* s_nn = reinterpret_cast<int*>(s_win + 6 * WIN);
     __shared__ int s_wa[LPB / 32 + 1], s_wb[LPB / 32 + 1];
     __shared__ unsigned s_pref[2];
     __shared__ unsigned s_ticket;
-    __shared__ int s_n;
-    for (int it = 0; it < MAX_ITER; ++it) {
+    __shared__ int s_n, s_ok;
+    __shared__ small_state s_small;
+    const int rt = A.adaptive_r ? A.max_radius : A.radius;
+    const int half = max(1, (int)gridDim.x / 2);
+    unsigned gen = 0;
+    int it = 0;
+    for (; it < MAX_ITER; ++it) {
         if (threadIdx.x == 0) s_n = *((volatile int*)A.g);
         __syncthreads();
         const int N = s_n;
-        if (N <= TAIL || *((volatile int*)A.err) != 0) break;
+        if (N <= LOOP_END || *((volatile int*)A.err) != 0) return;
+        if (small_tile(rt, 1) > 0 && (N + small_tile(rt, 1) - 1) / small_tile(rt, 1) <= (int)gridDim.x) break;
         const int r = radius_at(A, it);
         const int* cl_in = (it & 1) ? A.cl1 : A.cl0;
         int* cl_out = (it & 1) ? A.cl0 : A.cl1;
@@ -518,7 +702,6 @@ __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
         // count of an iteration never exceeds the previous one's (the look-back
         // words of lower tiles are then always this iteration's or older ones
         // with another tag).
-        const int rt = A.adaptive_r ? A.max_radius : A.radius;
         if (N >= NB4_MIN_N) {
             // long tiles (~25 us each) go to whichever CTA is free, in ticket order
             const int tsz = long_tile(rt);
@@ -536,7 +719,27 @@ __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
                 merge_tile<1>(A, cl_in, cl_out, N, r, it, tile, tsz, A.status_f, s_win, s_nn, s_wa, s_wb, s_pref);
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) A.g[1] = it + 1;
-        if (!grid_barrier(A.bar, A.err)) break;
+        if (!barrier_of(A.bar, gridDim.x, gen, A.err, &s_ok)) return;
+    }
+    // short lists; the words of the look-back above have another form, whose upper half
+    // is never a small iteration number (its tag sits in the top four bits)
+    int N = s_n, count = gridDim.x;
+    for (; it < MAX_ITER && N > LOOP_END; ++it) {
+        int S = 8;
+        while (S > 1 && (small_tile(rt, S) == 0 || (N + small_tile(rt, S) - 1) / small_tile(rt, S) > half)) S >>= 1;
+        const int tsz = small_tile(rt, S);
+        if ((N + tsz - 1) / tsz <= half) count = half;
+        if ((int)blockIdx.x >= count) return;
+        const int* cl_in = (it & 1) ? A.cl1 : A.cl0;
+        int* cl_out = (it & 1) ? A.cl0 : A.cl1;
+        small_iteration(A, cl_in, cl_out, N, radius_at(A, it), it, tsz, S, s_win, s_nn, s_wa, s_wb, s_pref, &s_small);
+        N = s_small.n;
+        if (!s_small.ok) return;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            A.g[0] = N;
+            A.g[1] = it + 1;
+        }
+        if (!barrier_of(A.bar, (unsigned)count, gen, A.err, &s_ok)) return;
     }
 }
 
@@ -574,19 +777,34 @@ __global__ void __launch_bounds__(PB, 1) k_ploc_tail(ploc_args A) {
     __syncthreads();
     for (int it = it0; N > 1 && it < MAX_ITER; ++it) {
         const int r = radius_at(A, it);
-        for (int i = threadIdx.x; i < N; i += PB) {
-            const float ax = smn[0][i], ay = smn[1][i], az = smn[2][i];
-            const float bx = smx[0][i], by = smx[1][i], bz = smx[2][i];
+        // Nearest neighbours: as many lanes per cluster (a power of two, at most a
+        // warp) as the CTA has, each walking every lanes-th candidate, then the
+        // least distance and of equal ones the lowest candidate. One thread per
+        // cluster left most of the CTA idle behind a chain of 2r candidates in
+        // every iteration after the first few.
+        int lanes = 1;
+        while (lanes < 32 && 2 * lanes * N <= PB) lanes <<= 1;
+        for (int t = threadIdx.x; (t & ~31) < N * lanes; t += PB) {
+            const int i = t >> (31 - __clz(lanes)), sub = t & (lanes - 1);
             float best = HP_MAX_FLOAT;
             int bi = -1;
-            const int lo = max(0, i - r), hi = min(N, i + r + 1);
-            for (int k = lo; k < hi; ++k) {
-                if (k == i) continue;
-                const float d = half_area(fminf(ax, smn[0][k]), fminf(ay, smn[1][k]), fminf(az, smn[2][k]),
-                                          fmaxf(bx, smx[0][k]), fmaxf(by, smx[1][k]), fmaxf(bz, smx[2][k]));
-                if (best > d) { best = d; bi = k; }
+            if (i < N) {
+                const float ax = smn[0][i], ay = smn[1][i], az = smn[2][i];
+                const float bx = smx[0][i], by = smx[1][i], bz = smx[2][i];
+                const int lo = max(0, i - r), hi = min(N, i + r + 1);
+                for (int k = lo + sub; k < hi; k += lanes) {
+                    if (k == i) continue;
+                    const float d = half_area(fminf(ax, smn[0][k]), fminf(ay, smn[1][k]), fminf(az, smn[2][k]),
+                                              fmaxf(bx, smx[0][k]), fmaxf(by, smx[1][k]), fmaxf(bz, smx[2][k]));
+                    if (best > d) { best = d; bi = k; }
+                }
             }
-            snn[i] = bi;
+            for (int o = lanes >> 1; o > 0; o >>= 1) {
+                const float od = __shfl_xor_sync(HP_FULL_MASK, best, o);
+                const int oi = __shfl_xor_sync(HP_FULL_MASK, bi, o);
+                if (oi >= 0 && (best > od || (best == od && (unsigned)oi < (unsigned)bi))) { best = od; bi = oi; }
+            }
+            if (i < N && sub == 0) snn[i] = bi;
         }
         __syncthreads();
         int kind[TAIL_ITEMS];
@@ -674,9 +892,7 @@ struct td_args {
     const float4* nbmax;
     const int4* cinfo;   // PLOC: per node, what its children contribute (ploc_args::cinfo)
     const float4* cbox;  // PLOC: per node, its Bin record's three box rows
-    int4* rec;          // [n-1] interior records: preorder index, first leaf, first triangle, status
-    int* flag;          // [n-1] record published (build epoch)
-    int epoch;
+    int4* rec;          // [n-1] interior records: preorder index, first leaf, first triangle, status + 1 (0: not yet)
     unsigned* ticket;
     const int32_t* sorted_tri;
     const float4* woop_src;  // Woop rows per scene triangle, or null: computed from the vertices
@@ -744,16 +960,17 @@ __global__ void __launch_bounds__(256) k_topdown(td_args T) {
         }
         const bool leaf = v >= n - 1 || T.state[v] == 0;
         unsigned spins = 0;
-        while (ld_acquire_u32(reinterpret_cast<const unsigned*>(T.flag + p)) != (unsigned)T.epoch) {
+        int4 pr = ld_record(T.rec + p);
+        while (pr.w == 0) {
             if (++spins > SPIN) {
                 hp_report(T.err, HP_DEV_SPIN_LIMIT, v);
                 break;
             }
             if ((spins & 1023u) == 0 && *((volatile int*)T.err) != 0) return;
+            pr = ld_record(T.rec + p);
         }
-        const int4 pr = __ldcg(T.rec + p);
         par = pr.x;
-        if (pr.w == ST_INTERIOR) {
+        if (pr.w == ST_INTERIOR + 1) {
             status = leaf ? ST_LEAF : ST_INTERIOR;
             if (is_left) {
                 iidx = pr.x + 1; lidx = pr.y; toff = pr.z;
@@ -767,10 +984,7 @@ __global__ void __launch_bounds__(256) k_topdown(td_args T) {
             toff = is_left ? pr.z : pr.z + ssize;
         }
     }
-    if (v < n - 1) {
-        __stcg(T.rec + v, make_int4(iidx, lidx, toff, status));
-        st_release_u32(reinterpret_cast<unsigned*>(T.flag + v), (unsigned)T.epoch);  // orders the record before
-    }
+    if (v < n - 1) st_record(T.rec + v, make_int4(iidx, lidx, toff, status + 1));
     const float4 mn = T.nbmin[v], mx = T.nbmax[v];
     const int size = __float_as_int(mx.w);
     if (status == ST_INTERIOR && PRE) {
@@ -814,14 +1028,9 @@ __global__ void __launch_bounds__(256) k_topdown(td_args T) {
             T.woop[3 * (int64_t)toff + 2] = __ldg(T.woop_src + 3 * (int64_t)tri + 2);
             return;
         }
-        float p[9];
-        for (int k = 0; k < 3; ++k) {
-            int vi = T.tris[3 * (int64_t)tri + k];
-            if (vi < 0 || vi >= T.nv) { hp_report(T.err, HP_DEV_BAD_INPUT, tri); vi = 0; }
-            for (int a = 0; a < 3; ++a) p[3 * k + a] = __ldg(T.verts + 3 * (int64_t)vi + a);
-        }
+        const tri_verts t = load_tri(T.verts, T.nv, T.tris, tri, T.err);
         float4 w0, w1, w2;
-        hp_woop(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], w0, w1, w2);
+        hp_woop(t.x0, t.y0, t.z0, t.x1, t.y1, t.z1, t.x2, t.y2, t.z2, w0, w1, w2);
         T.woop[3 * (int64_t)toff] = w0;
         T.woop[3 * (int64_t)toff + 1] = w1;
         T.woop[3 * (int64_t)toff + 2] = w2;
@@ -831,7 +1040,7 @@ __global__ void __launch_bounds__(256) k_topdown(td_args T) {
 }  // namespace
 
 size_t hp_topdown_scratch_bytes(int64_t n) {
-    return hp_carve::pad(n * 16) + hp_carve::pad(n * 4) + hp_carve::pad(64);
+    return hp_carve::pad(n * 16) + hp_carve::pad(64);
 }
 
 hp_status hp_topdown_collapse(hp_ctx* ctx, const hp_mesh* m, const hp_topdown_in& in, hp_bvh_impl* out,
@@ -840,9 +1049,8 @@ hp_status hp_topdown_collapse(hp_ctx* ctx, const hp_mesh* m, const hp_topdown_in
     const int64_t nn = 2 * (int64_t)n - 1;
     hp_carve cv(reinterpret_cast<char*>(scratch));
     int4* rec = cv.take<int4>(n);
-    int* flag = cv.take<int>(n);
     unsigned* ticket = cv.take<unsigned>(16);
-    HP_CUDA(cudaMemsetAsync(flag, 0, (size_t)n * 4, s));
+    HP_CUDA(cudaMemsetAsync(rec, 0, (size_t)n * 16, s));
     HP_CUDA(cudaMemsetAsync(ticket, 0, 64, s));
     td_args T{};
     T.n = n;
@@ -855,8 +1063,6 @@ hp_status hp_topdown_collapse(hp_ctx* ctx, const hp_mesh* m, const hp_topdown_in
     T.nbmin = in.nbmin;
     T.nbmax = in.nbmax;
     T.rec = rec;
-    T.flag = flag;
-    T.epoch = 1;
     T.ticket = ticket;
     T.sorted_tri = in.sorted_tri;
     T.verts = m->vertices;
@@ -874,6 +1080,12 @@ hp_status hp_topdown_collapse(hp_ctx* ctx, const hp_mesh* m, const hp_topdown_in
     return HP_OK;
 }
 
+// Words of the iterations on shorter lists: a tile of at least LPB / 2 clusters, or a
+// CTA each.
+static int64_t fused_words(int64_t n) {
+    return std::max<int64_t>((std::min<int64_t>(n, NB4_MIN_N) + LPB / 2 - 1) / (LPB / 2) + 1, LOOP_MAX_GRID);
+}
+
 size_t hp_ploc_scratch_bytes(int64_t n) {
     const int64_t nn = 2 * n - 1;
     size_t b = 0;
@@ -883,9 +1095,9 @@ size_t hp_ploc_scratch_bytes(int64_t n) {
     b += hp_carve::pad(nn);            // state
     b += 2 * hp_carve::pad(n * 4);     // cl0, cl1
     b += hp_carve::pad(((n + MIN_TILE4 - 1) / MIN_TILE4 + 1) * 8);
-    b += hp_carve::pad(((std::min<int64_t>(n, NB4_MIN_N) + LPB / 2 - 1) / (LPB / 2) + 1) * 8);
+    b += hp_carve::pad(fused_words(n) * 8);
     b += hp_carve::pad(MAX_ITER * 4 + 64);
-    b += hp_carve::pad(n * 16) + hp_carve::pad(n * 4);  // records, flags
+    b += hp_carve::pad(n * 16);        // collapse records
     b += hp_carve::pad(n * 16) + hp_carve::pad(n * 48);  // children's counts and boxes per node
     return b;
 }
@@ -919,7 +1131,7 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
     A.cl1 = cv.take<int>(n);
     const int64_t mtiles = (n + MIN_TILE4 - 1) / MIN_TILE4 + 1;
     A.status = cv.take<unsigned long long>(mtiles);
-    const int64_t ftiles = (std::min<int64_t>(n, NB4_MIN_N) + LPB / 2 - 1) / (LPB / 2) + 1;
+    const int64_t ftiles = fused_words(n);
     A.status_f = cv.take<unsigned long long>(ftiles);
     unsigned* ctl = cv.take<unsigned>(MAX_ITER + 16);
     A.tickets = ctl;
@@ -927,15 +1139,14 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
     A.g = reinterpret_cast<int*>(ctl + MAX_ITER + 4);
     A.err = ctx->d_status;
     int4* rec = cv.take<int4>(n);
-    int* flag = cv.take<int>(n);
     if (hp_layout_of(p) == 2) {  // the binary collapse reads them
+        HP_CUDA(cudaMemsetAsync(rec, 0, (size_t)n * 16, s));
         A.cinfo = cv.take<int4>(n);
         A.cbox = cv.take<float4>(3 * (int64_t)n);
     }
     HP_CUDA(cudaMemsetAsync(A.status, 0, mtiles * 8, s));
     HP_CUDA(cudaMemsetAsync(A.status_f, 0, ftiles * 8, s));
     HP_CUDA(cudaMemsetAsync(ctl, 0, (MAX_ITER + 16) * 4, s));
-    HP_CUDA(cudaMemsetAsync(flag, 0, (size_t)n * 4, s));
     k_ploc_leaves<<<hp_div_up(n, 256), 256, 0, s>>>(A, sorted_tri, tbmin, tbmax);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
@@ -946,7 +1157,7 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
         int per_sm = 0;
         HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ploc_loop, LPB, smem));
         if (per_sm < 1) return hp_fail(HP_ERR_UNSUPPORTED, "PLOC loop kernel does not fit on an SM");
-        int grid = ctx->sm_count * per_sm;
+        const int grid = std::min(ctx->sm_count * per_sm, LOOP_MAX_GRID);
         void* args[] = {&A};
         HP_CUDA(cudaLaunchCooperativeKernel((void*)k_ploc_loop, grid, LPB, args, smem, s));
         hp_count_launch();
@@ -986,8 +1197,6 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
     T.nbmin = A.nbmin;
     T.nbmax = A.nbmax;
     T.rec = rec;
-    T.flag = flag;
-    T.epoch = 1;
     T.ticket = ctl + MAX_ITER + 8;
     T.sorted_tri = sorted_tri;
     T.woop_src = woop_src;

@@ -73,12 +73,12 @@ __global__ void __launch_bounds__(HB) k_hl_refit(int n, const int32_t* __restric
     int node = __ldcg(parent + leaf), guard = 0;
     while (node >= 0) {
         if (node >= n - 1 || ++guard > n) { hp_report(err, HP_DEV_BAD_INDEX, node); return; }
+        const int l = __ldcg(left + node), r = __ldcg(right + node), up = __ldcg(parent + node);
         if (hp_arrive(counters + node) == 0) return;
-        const int l = __ldcg(left + node), r = __ldcg(right + node);
         const float4 a = __ldcg(nbmin + l), b = __ldcg(nbmin + r), c = __ldcg(nbmax + l), d = __ldcg(nbmax + r);
         __stcg(nbmin + node, make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f));
         __stcg(nbmax + node, make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z), 0.0f));
-        node = __ldcg(parent + node);
+        node = up;
     }
 }
 

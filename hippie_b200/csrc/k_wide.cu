@@ -98,8 +98,10 @@ __global__ void __launch_bounds__(WB) k_wide_dp(wide_args A) {
     int steps = 0;
     while (cur >= 0) {
         if (cur >= n - 1 || ++steps > n) { hp_report(A.err, HP_DEV_BAD_INDEX, cur); return; }
+        // links and box of cur are final: read while the arrival travels
+        const int ch[2] = {__ldg(A.left + cur), __ldg(A.right + cur)}, up = __ldg(A.parent + cur);
+        const float4 bmn = __ldg(A.nbmin + cur), bmx = __ldg(A.nbmax + cur);
         if (hp_arrive(A.counters + cur) == 0) return;
-        const int ch[2] = {__ldcg(A.left + cur), __ldcg(A.right + cur)};
         float c[2][J];
         int sz[2];
         for (int s = 0; s < 2; ++s) {
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(WB) k_wide_dp(wide_args A) {
             }
         }
         const int size = sz[0] + sz[1];
-        const float a = host_area(__ldcg(A.nbmin + cur), __ldcg(A.nbmax + cur));
+        const float a = host_area(bmn, bmx);
         float* oc = A.cost + (size_t)cur * J;
         uint16_t* on = A.cnt + (size_t)cur * J;
         const float lc = size > A.max_leaf ? MAXF : leaf_cost<N>(A.ci, a, root_a, size);
@@ -149,7 +151,7 @@ __global__ void __launch_bounds__(WB) k_wide_dp(wide_args A) {
             __stcg(on + j - 1, prev_n);
         }
         __stcg(A.size + cur, size);
-        cur = __ldcg(A.parent + cur);
+        cur = up;
     }
 }
 

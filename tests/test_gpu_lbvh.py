@@ -163,3 +163,17 @@ def test_buffers_at_any_word(ctx, method):
     ctx.check()
     for a, b in zip(got, want):
         np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
+
+
+@pytest.mark.parametrize("n", [1023, 1025, 8191, 8192, 8193])
+@pytest.mark.parametrize("adaptive", [0, 1])
+def test_collapse_of_small_meshes(ctx, n, adaptive):
+    """Around the largest mesh whose collapse is scanned by one CTA (8,192 triangles)."""
+    v, t = hp.gen.uniform_mesh(60 + n, n, 0.03)
+    p = hp.BuildParams(morton_bits=30, adaptive_leaf=adaptive, max_leaf_size=5)
+    bvh = ctx.build(dev(v), dev(t), p)
+    nodes, woop, tri = bvh.download()
+    ctx.check()
+    ref = oracle.build_lbvh(v, t, bits=30, adaptive=adaptive, max_leaf=5, scale=np.array(bvh.c.morton_scale, np.float32))
+    np.testing.assert_array_equal(nodes, ref["nodes"])
+    np.testing.assert_array_equal(tri, ref["tri_idx"])

@@ -44,7 +44,16 @@ constexpr int PB = 1024;            // threads of the tail CTA
 constexpr int LPB = 512;            // threads per CTA of the iteration kernel (two CTAs per SM)
 constexpr int MAXR = 512;           // largest radius kept in a shared-memory window
 constexpr int NB4 = 4;              // clusters per thread of the neighbour search on large lists
-constexpr int WIN = NB4 * LPB + 2 * MAXR;  // neighbour window
+// Neighbour window: the stride of its six arrays. Threads that search for four
+// clusters each read window entries four apart; as they lie, that is four lanes to a
+// bank and the search waits for shared memory. So a window of theirs is stored by the
+// entry's index modulo 4, in four rows of WQ entries (entry k at win4(k)): lanes then
+// read neighbours, and WQ = 8 modulo 32 spreads the consecutive stores of a warp over
+// all banks too.
+constexpr int WQ = (NB4 * LPB + 2 * MAXR) / 4 + 8;
+constexpr int WIN = 4 * WQ;
+static_assert(WQ % 32 == 8, "the four rows start eight banks apart");
+__device__ __forceinline__ int win4(int k) { return (k & 3) * WQ + (k >> 2); }
 // Lists at least this long use 4 clusters per thread (long tiles, about half as
 // many tiles as the loop has CTAs at this length). On a B200 this beat twice
 // and four times the length, half and a quarter of it, and long tiles at every
@@ -176,15 +185,6 @@ __device__ __forceinline__ void make_parent_from(const ploc_args& A, int node, i
     }
 }
 
-__device__ __forceinline__ void make_parent(const ploc_args& A, int node, int a, int b) {
-    const float4 amn = __ldcg(A.nbmin + a), amx = __ldcg(A.nbmax + a);
-    const float4 bmn = __ldcg(A.nbmin + b), bmx = __ldcg(A.nbmax + b);
-    const int2 ca = __ldcg(A.counts + a), cb = __ldcg(A.counts + b);
-    float4 omn, omx;
-    int2 ocnt;
-    make_parent_from(A, node, a, b, amn, amx, bmn, bmx, ca, cb, omn, omx, ocnt);
-}
-
 // Leaves: sorted reference p becomes leaf node n-1+p and cluster p.
 __global__ void __launch_bounds__(256) k_ploc_leaves(ploc_args A, const int32_t* __restrict__ sorted_tri,
                                                      const float4* __restrict__ tbmin,
@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(256) k_ploc_leaves(ploc_args A, const int32_t*
 // never the nearest, outside the cluster list). The cluster indices of a batch
 // of elements are read first and their boxes after, so that a thread has a
 // batch of loads in flight instead of one dependent pair at a time.
+template <bool ROWS4>
 __device__ __forceinline__ void load_window(const ploc_args& A, const int* __restrict__ cl, int N, int w0, int wn,
                                             float* s) {
     constexpr int BATCH = 3;
@@ -241,8 +242,8 @@ __device__ __forceinline__ void load_window(const ploc_args& A, const int* __res
         }
 #pragma unroll
         for (int u = 0; u < BATCH; ++u) {
-            const int k = k0 + u * LPB;
-            if (k < wn) {
+            if (k0 + u * LPB < wn) {
+                const int k = ROWS4 ? win4(k0 + u * LPB) : k0 + u * LPB;
                 s[k] = mn[u].x; s[WIN + k] = mn[u].y; s[2 * WIN + k] = mn[u].z;
                 s[3 * WIN + k] = mx[u].x; s[4 * WIN + k] = mx[u].y; s[5 * WIN + k] = mx[u].z;
             }
@@ -261,14 +262,14 @@ __device__ void nn_tile(const ploc_args& A, const int* __restrict__ cl, int N, i
     float* smxz = s + 5 * WIN;
     constexpr int TS = B * LPB;
     __syncthreads();
-    load_window(A, cl, N, base - r, TS + 2 * r, s);
+    load_window<true>(A, cl, N, base - r, TS + 2 * r, s);
     __syncthreads();
     const int l0 = threadIdx.x * B;  // cluster base + l sits at window position l + r
     float ax[B], ay[B], az[B], bx[B], by[B], bz[B], best[B];
     int bi[B];
 #pragma unroll
     for (int q = 0; q < B; ++q) {
-        const int me = l0 + q + r;
+        const int me = win4(l0 + q + r);
         ax[q] = smnx[me]; ay[q] = smny[me]; az[q] = smnz[me];
         bx[q] = smxx[me]; by[q] = smxy[me]; bz[q] = smxz[me];
         best[q] = HP_MAX_FLOAT;
@@ -282,7 +283,9 @@ __device__ void nn_tile(const ploc_args& A, const int* __restrict__ cl, int N, i
             bi[q] = base - r + k;
         }
     };
-#define HP_PLOC_CAND(k) const float cx = smnx[k], cy = smny[k], cz = smnz[k], dx = smxx[k], dy = smxy[k], dz = smxz[k]
+#define HP_PLOC_CAND(k)                                                             \
+    const int w_ = win4(k);                                                          \
+    const float cx = smnx[w_], cy = smny[w_], cz = smnz[w_], dx = smxx[w_], dy = smxy[w_], dz = smxz[w_]
     if (B == 1 || r < 4) {
         for (int k = l0; k <= l0 + (B - 1) + 2 * r; ++k) {
             HP_PLOC_CAND(k);
@@ -383,7 +386,7 @@ __device__ void nn_halo(const ploc_args& A, const int* __restrict__ cl, int N, i
     float* smxy = s + 4 * WIN;
     float* smxz = s + 5 * WIN;
     const int w0 = tbase - 2 * r;
-    load_window(A, cl, N, w0, tsz + 4 * r, s);
+    load_window<false>(A, cl, N, w0, tsz + 4 * r, s);
     __syncthreads();
     for (int l = threadIdx.x; l < tsz + 2 * r; l += LPB) {
         const int c = tbase - r + l;
@@ -439,42 +442,92 @@ __device__ void merge_tile(const ploc_args& A, const int* __restrict__ cl_in, in
             k += kind[q] != 0;
         }
     }
+    // Node numbers of the clusters that stay, and of the partners of those that merge,
+    // travel during the scan.
+    int node[ITEMS], part[ITEMS];
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) {
+        node[q] = kind[q] != 0 ? __ldcg(cl_in + base + q) : -1;
+        part[q] = kind[q] == 2 ? __ldcg(cl_in + nbr[q]) : -1;
+    }
     int em = m, ek = k;
     const int2 tot = block_scan2<LPB>(em, ek, s_wa, s_wb);
+    unsigned long long* st = status + tile;
+    if (threadIdx.x == 0) st_vol_u64(st, mk_status(tag, tile == 0 ? F_INC : F_AGG, tot.x, tot.y));
+    // The tile's merges as a list (in the window, which is done with), so that each has
+    // a thread: their boxes are read all at once, while the look-back waits. A thread
+    // that made its own clusters' merges one after another took 7 us of a 29 us tile.
+    int2* s_list = reinterpret_cast<int2*>(s_win);
+    {
+        int at = em;
+#pragma unroll
+        for (int q = 0; q < ITEMS; ++q)
+            if (kind[q] == 2) s_list[at++] = make_int2(node[q], part[q]);
+    }
+    __syncthreads();
+    int2 pair = make_int2(0, 0);
+    float4 amn{}, amx{}, bmn{}, bmx{};
+    int2 ca{}, cb{};
+    if ((int)threadIdx.x < tot.x) {
+        pair = s_list[threadIdx.x];
+        amn = __ldcg(A.nbmin + pair.x);
+        amx = __ldcg(A.nbmax + pair.x);
+        bmn = __ldcg(A.nbmin + pair.y);
+        bmx = __ldcg(A.nbmax + pair.y);
+        ca = __ldcg(A.counts + pair.x);
+        cb = __ldcg(A.counts + pair.y);
+    }
     if (threadIdx.x < 32) {
-        // Decoupled look-back by one warp over windows of 32 earlier tiles: lane i
-        // reads tile t-i; the window is summed up to the nearest tile whose
-        // inclusive prefix is published, once every tile up to it has published.
+        // Decoupled look-back by one warp: lane i reads the tiles t-i, t-32-i, ... of
+        // LBW windows at once (the CTAs of a round are as many tiles apart, and a window
+        // a round trip and each clusters' merges made by their thread: 1.874 -> 1.757 ms
+        // of iterations on 4.2 M clusters; 4 or 10 windows: 1.763 and 1.818); windows are summed up to the nearest tile
+        // whose inclusive prefix is published, once every tile up to it has published.
+        constexpr int LBW = 2;
         const int lane = threadIdx.x;
-        unsigned long long* st = status + tile;
-        if (lane == 0) st_vol_u64(st, mk_status(tag, tile == 0 ? F_INC : F_AGG, tot.x, tot.y));
         unsigned pm = 0, pk = 0;
         if (tile > 0) {
             long t = (long)tile - 1;
             unsigned spins = 0;
-            while (true) {
-                const long idx = t - lane;
-                const unsigned long long s = idx >= 0 ? ld_vol_u64(status + idx) : mk_status(tag, F_INC, 0, 0);
-                const bool ready = (unsigned)(s >> 60) == tag && (s & F_MASK) != 0;
-                const unsigned inc = __ballot_sync(HP_FULL_MASK, ready && (s & F_MASK) == F_INC);
-                const int stop = inc ? __ffs(inc) - 1 : 31;  // the window ends at the nearest inclusive tile
-                const unsigned need = stop == 31 ? HP_FULL_MASK : ((1u << (stop + 1)) - 1u);
-                if (__ballot_sync(HP_FULL_MASK, !ready) & need) {
-                    if (++spins > SPIN) { if (lane == 0) hp_report(A.err, HP_DEV_SPIN_LIMIT, (int)tile); break; }
-                    if ((spins & 1023u) == 0 && __shfl_sync(HP_FULL_MASK, *((volatile int*)A.err), 0) != 0) break;
-                    continue;
-                }
-                unsigned vm = lane <= stop ? (unsigned)((s >> 29) & 0x1fffffffu) : 0u;
-                unsigned vk = lane <= stop ? (unsigned)(s & 0x1fffffffu) : 0u;
+            bool done = false, gone = false;
+            while (!done && !gone) {
+                unsigned long long w[LBW];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    vm += __shfl_xor_sync(HP_FULL_MASK, vm, o);
-                    vk += __shfl_xor_sync(HP_FULL_MASK, vk, o);
+                for (int j = 0; j < LBW; ++j) {
+                    const long idx = t - 32 * j - lane;
+                    w[j] = idx >= 0 ? ld_vol_u64(status + idx) : mk_status(tag, F_INC, 0, 0);
                 }
-                pm += vm;
-                pk += vk;
-                if (inc) break;
-                t -= 32;
+#pragma unroll
+                for (int j = 0; j < LBW; ++j) {
+                    const unsigned long long s = w[j];
+                    const bool ready = (unsigned)(s >> 60) == tag && (s & F_MASK) != 0;
+                    const unsigned inc = __ballot_sync(HP_FULL_MASK, ready && (s & F_MASK) == F_INC);
+                    const int stop = inc ? __ffs(inc) - 1 : 31;  // the window ends at the nearest inclusive tile
+                    const unsigned need = stop == 31 ? HP_FULL_MASK : ((1u << (stop + 1)) - 1u);
+                    if (__ballot_sync(HP_FULL_MASK, !ready) & need) {
+                        if (++spins > SPIN) {
+                            if (lane == 0) hp_report(A.err, HP_DEV_SPIN_LIMIT, (int)tile);
+                            gone = true;
+                        }
+                        if ((spins & 1023u) == 0 && __shfl_sync(HP_FULL_MASK, *((volatile int*)A.err), 0) != 0)
+                            gone = true;
+                        break;
+                    }
+                    if (lane <= stop) {
+                        pm += (unsigned)((s >> 29) & 0x1fffffffu);
+                        pk += (unsigned)(s & 0x1fffffffu);
+                    }
+                    if (inc) {
+                        done = true;
+                        break;
+                    }
+                    t -= 32;
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                pm += __shfl_xor_sync(HP_FULL_MASK, pm, o);
+                pk += __shfl_xor_sync(HP_FULL_MASK, pk, o);
             }
             if (lane == 0) st_vol_u64(st, mk_status(tag, F_INC, pm + tot.x, pk + tot.y));
         }
@@ -486,20 +539,26 @@ __device__ void merge_tile(const ploc_args& A, const int* __restrict__ cl_in, in
         }
     }
     __syncthreads();
-    int mr = (int)s_pref[0] + em, kr = (int)s_pref[1] + ek;
+    const int m0 = (int)s_pref[0];
+    for (int i = threadIdx.x; i < tot.x; i += LPB) {
+        if (i != (int)threadIdx.x) {  // more merges than threads
+            pair = s_list[i];
+            amn = __ldcg(A.nbmin + pair.x);
+            amx = __ldcg(A.nbmax + pair.x);
+            bmn = __ldcg(A.nbmin + pair.y);
+            bmx = __ldcg(A.nbmax + pair.y);
+            ca = __ldcg(A.counts + pair.x);
+            cb = __ldcg(A.counts + pair.y);
+        }
+        float4 omn, omx;
+        int2 ocnt;
+        make_parent_from(A, (N - 2) - (m0 + i), pair.x, pair.y, amn, amx, bmn, bmx, ca, cb, omn, omx, ocnt);
+    }
+    int mr = m0 + em, kr = (int)s_pref[1] + ek;
 #pragma unroll
     for (int q = 0; q < ITEMS; ++q) {
-        const int c = base + q;
         if (kind[q] == 0) continue;
-        int node = cl_in[c];
-        if (kind[q] == 2) {
-            const int nb = cl_in[nbr[q]];
-            const int idx = (N - 2) - mr;
-            make_parent(A, idx, node, nb);
-            node = idx;
-            ++mr;
-        }
-        cl_out[kr++] = node;
+        cl_out[kr++] = kind[q] == 2 ? (N - 2) - mr++ : node[q];
     }
 }
 
@@ -538,7 +597,7 @@ __device__ void small_iteration(const ploc_args& A, const int* __restrict__ cl_i
     float4 amn{}, amx{}, bmn{}, bmx{};  // the two clusters of a merge
     int2 ca{}, cb{};
     if (mine) {
-        load_window(A, cl_in, N, tbase - 2 * r, tsz + 4 * r, s_win);
+        load_window<false>(A, cl_in, N, tbase - 2 * r, tsz + 4 * r, s_win);
         __syncthreads();
         // neighbours of the tile's clusters and of r on each side: lanes sub, sub + S,
         // ... of the candidates, then the least distance and of equal ones the first
@@ -1144,9 +1203,9 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
         A.cinfo = cv.take<int4>(n);
         A.cbox = cv.take<float4>(3 * (int64_t)n);
     }
-    HP_CUDA(cudaMemsetAsync(A.status, 0, mtiles * 8, s));
-    HP_CUDA(cudaMemsetAsync(A.status_f, 0, ftiles * 8, s));
-    HP_CUDA(cudaMemsetAsync(ctl, 0, (MAX_ITER + 16) * 4, s));
+    // the look-back words of both kinds and the control words lie one after the other
+    HP_CUDA(cudaMemsetAsync(A.status, 0, (size_t)(reinterpret_cast<char*>(ctl + MAX_ITER + 16) -
+                                                  reinterpret_cast<char*>(A.status)), s));
     k_ploc_leaves<<<hp_div_up(n, 256), 256, 0, s>>>(A, sorted_tri, tbmin, tbmax);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();

@@ -78,3 +78,18 @@ def test_ploc_beats_lbvh_cost(ctx):
     bvh, ref, V, T = _ploc(ctx, v, t)
     lb = ctx.build(V, T, hp.BuildParams(morton_bits=60))
     assert bvh.cost() < lb.cost()
+
+
+@pytest.mark.parametrize("n,radius,adaptive", [(2300, 16, 0), (4737, 16, 0), (14300, 16, 0), (33300, 16, 0),
+                                               (71100, 16, 0), (142200, 16, 0), (9000, 1, 0), (20000, 112, 0),
+                                               (6000, 113, 0), (9000, 239, 0), (5000, 241, 0), (30000, 3, 1)])
+def test_ploc_bit_exact_short_lists(ctx, n, radius, adaptive):
+    """Lists of a tile per CTA: about the lengths at which a cluster gets one, two, four
+    or eight lanes, and radii at which a tile with its halo does and does not leave room
+    for several lanes, or for these iterations at all (512 - 2 r >= 32)."""
+    v, t = hp.gen.clustered_mesh(900 + n, n, clusters=max(1, min(1024, n // 64)))
+    bvh, ref, V, T = _ploc(ctx, v, t, ploc_radius=radius, ploc_max_radius=max(radius, 60 if adaptive else 1),
+                           ploc_adaptive=adaptive)
+    nodes, woop, tri = bvh.download()
+    np.testing.assert_array_equal(tri, ref["tri_idx"])
+    np.testing.assert_array_equal(nodes, ref["nodes"])

@@ -229,35 +229,42 @@ __global__ void __launch_bounds__(TB) k_leaves(
 //   state 0 (collapse into a leaf) iff ci*A*size < interior cost;
 // or, without adaptive leaves, computeNodeStates (:138-184): size <= maxLeafSize.
 //
-// Two phases, so that almost all memory traffic is coalesced. Every LBVH node
-// covers a contiguous range [lo, hi] of sorted leaves and its index lies in
-// that range; a CTA owning the CB = 512 leaves [base, base + CB) therefore owns every node
-// whose range lies inside its own ("local" nodes: their indices, children and
-// boxes are all in [base, base + CB)). Phase A (k_climb_local) loads the
-// CTA's node indices and leaf boxes with coalesced loads, climbs the local
-// nodes with shared-memory arrival counters and boxes (block-scope ordering),
-// and writes their boxes, states and maxHi words back with coalesced stores;
-// a thread whose next node is not local stops and appends its child to the
-// frontier list. (Computing the local nodes in barrier-separated rounds
+// The same climb finds the tree (construct<T>, LBVHBuilderKernels.cu:11-63): a node
+// over sorted positions [lo, hi] is the left child of its parent, split at hi, when
+// delta(hi, hi + 1) > delta(lo - 1, lo), else the right child, split at lo - 1; the
+// radix tree is the same, and so are Karras's numbers: a left child has the index hi, a
+// right child lo, the root 0. A child arrives at its split with its other end, and
+// whoever comes second has both ends. Searching every node's range and split in a
+// kernel of its own was bound by instruction issue: 16.8 M triangles took 0.51 ms there and
+// 0.83 ms in the climb, 1.04 ms in this climb alone (a build 4.51 -> 4.21 ms; of 5,003
+// triangles 121 -> 114 us).
+//
+// Two phases, so that almost all memory traffic is coalesced. A CTA owns the CB = 512
+// leaves [base, base + CB) and every node whose range lies inside ("local" nodes: their
+// indices, children and boxes are all in [base, base + CB)). Phase A (k_climb_local)
+// loads the CTA's leaf boxes with coalesced loads, takes the deltas of neighbouring keys
+// into shared memory, climbs the local nodes with shared-memory arrivals and boxes
+// (block-scope ordering), and writes their links, boxes, states and maxHi words back with
+// coalesced stores; a child whose sibling lies, wholly or in part, outside the CTA goes
+// to the frontier list. (Computing the local nodes in barrier-separated rounds
 // instead was slower: the CTAs' local subtrees are deep.) Phase B
 // (k_climb_frontier) climbs from the frontier entries through the non-local
-// nodes (those whose ranges cross a CTA boundary: about depth per boundary)
-// with the global counters and one acq_rel atomic per arrival; a node's links are
-// read while the arrival at its child travels (5 K triangles 0.031 -> 0.025 ms,
-// 16.8 M 0.178 -> 0.146 ms). 1,024 leaves per CTA halve phase B and slow phase A
-// by as much (0.70 -> 0.80 ms at 16.8 M).
+// nodes (those whose ranges cross a CTA boundary: about depth per boundary), an acq_rel
+// exchange per arrival that brings the sibling's other end. 1,024 leaves per CTA halve
+// phase B and slow phase A by as much.
 constexpr int CB = 512;
-constexpr size_t CLIMB_SMEM = (size_t)CB * (4 * sizeof(float4) + 7 * sizeof(int) + sizeof(int2)) + 2 * sizeof(int);
+constexpr size_t CLIMB_SMEM = (size_t)CB * (4 * sizeof(float4) + sizeof(int2) + 7 * sizeof(int) + 1) + 16;
+constexpr int SPLIT_STATE = 1 << 30;  // a local node's state beside its split
 
 struct climb_args {
     int n;
-    const int* parent;
-    const int* left;
-    const int* right;
-    const int2* range;
+    int* parent;
+    int* left;
+    int* right;
+    int2* range;
     float4* nbmin;
     float4* nbmax;
-    int* counters;     // arrivals at non-local nodes (zeroed)
+    int* words;        // arrivals at the splits of non-local nodes: the first child's other end + 1 (zeroed)
     int* max_hi;       // maxHi words (initialised to -1)
     uint8_t* state;
     int* frontier;     // children whose parent is not local to their CTA
@@ -290,155 +297,158 @@ __device__ __forceinline__ int merge_node(const climb_args& A, float4 lmn, float
     return st;
 }
 
-__global__ void __launch_bounds__(CB, 4) k_climb_local(climb_args A) {
+template <typename K>
+__global__ void __launch_bounds__(CB, 4) k_climb_local(climb_args A, const K* __restrict__ keys) {
     extern __shared__ __align__(16) unsigned char climb_smem[];
     float4* s_imn = reinterpret_cast<float4*>(climb_smem);  // local interior node base + k
     float4* s_imx = s_imn + CB;
     float4* s_lmn = s_imx + CB;                             // leaf base + k
     float4* s_lmx = s_lmn + CB;
-    int2* s_rng = reinterpret_cast<int2*>(s_lmx + CB);      // ranges of nodes base + k
-    int* s_cnt = reinterpret_cast<int*>(s_rng + CB);        // arrivals at local nodes
-    int* s_left = s_cnt + CB;
-    int* s_right = s_left + CB;
-    int* s_up = s_right + CB;                               // parents of nodes base + k
-    int* s_mh = s_up + CB;                                  // maxHi of positions base + k
-    int* s_st = s_mh + CB;                                  // state of local nodes
-    int* s_front = s_st + CB;                               // this CTA's frontier entries
+    int2* s_rng = reinterpret_cast<int2*>(s_lmx + CB);      // ranges of local nodes
+    int* s_split = reinterpret_cast<int*>(s_rng + CB);      // their splits (and states), -1 for none
+    int* s_end = s_split + CB;                              // split base + k: the first child's other end + 1
+    int* s_who = s_end + CB;                                // and its index
+    int* s_up = s_who + CB;                                 // parents of interior nodes base + k
+    int* s_lup = s_up + CB;                                 // parents of leaves base + k
+    int* s_mh = s_lup + CB;                                 // maxHi of positions base + k
+    int* s_front = s_mh + CB;                               // this CTA's frontier entries
     int* s_fn = s_front + CB;                               // [0] their count, [1] their offset
+    uint8_t* s_d = reinterpret_cast<uint8_t*>(s_fn + 2);    // delta(base + k - 1, base + k) + 1, k = 0 .. CB
     const int n = A.n;
     const int base = blockIdx.x * CB, k = threadIdx.x, p = base + k;
     const int last = min(base + CB, n) - 1;  // this CTA's last leaf
-    s_cnt[k] = 0;
+    auto delta1 = [&](int j) { return (uint8_t)((base + j > 0 ? kdelta(keys, n, base + j - 1, base + j) : -1) + 1); };
+    s_split[k] = -1;
+    s_end[k] = 0;
+    s_up[k] = -1;
+    s_lup[k] = -1;
     s_mh[k] = -1;
     if (k == 0) s_fn[0] = 0;
-    if (p < n - 1) {
-        s_left[k] = __ldg(A.left + p);
-        s_right[k] = __ldg(A.right + p);
-        s_up[k] = __ldg(A.parent + p);
-        s_rng[k] = __ldg(A.range + p);
-    } else {
-        s_rng[k] = make_int2(-1, -1);  // not an interior node: never local
-    }
+    if (p <= n) s_d[k] = delta1(k);
+    if (k == 0 && last + 1 - base == CB) s_d[CB] = delta1(CB);
     float4 cmn = make_float4(0.0f, 0.0f, 0.0f, 0.0f), cmx = cmn;
-    int node = -1;
     if (p < n) {
         cmn = A.nbmin[n - 1 + p];
         cmx = A.nbmax[n - 1 + p];
         s_lmn[k] = cmn;
         s_lmx[k] = cmx;
-        node = __ldg(A.parent + n - 1 + p);
     }
     __syncthreads();
-    int child = n - 1 + p;
-    int guard = 0;
-    while (p < n && node >= 0) {
-        const int kn = node - base;
-        const int2 rg = ((unsigned)kn < (unsigned)CB) ? s_rng[kn] : make_int2(-1, -1);
-        if (!(rg.x >= base && rg.y <= last && kn <= rg.y - base && kn >= rg.x - base)) {
-            // the next node's range crosses the CTA's: phase B continues from
-            // child (collected here, one global reservation per CTA below)
+    int lo = p, hi = p, child = n - 1 + p;
+    while (p < n && hi - lo < n - 1) {
+        const bool is_left = s_d[hi + 1 - base] > s_d[lo - base];
+        if (is_left ? hi == last : lo == base) {  // the sibling starts in another CTA
             s_front[atomicAdd(s_fn, 1)] = child;  // one entry per leaf thread at most
             break;
         }
-        if (++guard > CB) {
-            hp_report(A.err, HP_DEV_BAD_INDEX, node);
-            break;
-        }
-        const int l = s_left[kn], r = s_right[kn];
-        if (l != child && r != child) {
-            hp_report(A.err, HP_DEV_BAD_INDEX, node);
-            break;
-        }
-        const bool is_left = l == child;
-        const int sib = is_left ? r : l;
-        const int ks = (sib >= n - 1) ? sib - (n - 1) - base : sib - base;
-        if ((unsigned)ks >= (unsigned)CB) {
-            hp_report(A.err, HP_DEV_BAD_INDEX, node);
-            break;
-        }
+        const int s = is_left ? hi : lo - 1, ks = s - base;
+        s_who[ks] = child;
         __threadfence_block();
-        if (atomicAdd(&s_cnt[kn], 1) == 0) break;
+        const int old = atomicExch(&s_end[ks], (is_left ? lo : hi) + 1);
+        if (old == 0) break;
         __threadfence_block();
-        const float4 smn = sib >= n - 1 ? s_lmn[ks] : s_imn[ks];
-        const float4 smx = sib >= n - 1 ? s_lmx[ks] : s_imx[ks];
+        s_end[ks] = 0;
+        const int nlo = is_left ? lo : old - 1, nhi = is_left ? old - 1 : hi;
+        // the sibling, a leaf or interior node of the same slot either way
+        const int kb = is_left ? ks + 1 : ks;
+        const bool sib_leaf = is_left ? nhi == s + 1 : nlo == s;
+        const float4 smn = sib_leaf ? s_lmn[kb] : s_imn[kb];
+        const float4 smx = sib_leaf ? s_lmx[kb] : s_imx[kb];
         float4 omn, omx;
         const int st = is_left ? merge_node(A, cmn, cmx, smn, smx, omn, omx)
                                : merge_node(A, smn, smx, cmn, cmx, omn, omx);
+        const int idx = nhi - nlo == n - 1 ? 0 : (s_d[nhi + 1 - base] > s_d[nlo - base] ? nhi : nlo);
+        const int kn = idx - base;
         s_imn[kn] = omn;
         s_imx[kn] = omx;
-        s_st[kn] = st;
-        if (st == 0 && node != 0) atomicMax(&s_mh[rg.x - base], rg.y);
+        s_rng[kn] = make_int2(nlo, nhi);
+        s_split[kn] = s | (st ? SPLIT_STATE : 0);
+        (nlo == s ? s_lup : s_up)[ks] = idx;
+        (nhi == s + 1 ? s_lup : s_up)[ks + 1] = idx;
+        if (st == 0 && idx != 0) atomicMax(&s_mh[nlo - base], nhi);
         cmn = omn;
         cmx = omx;
-        child = node;
-        node = s_up[kn];
+        lo = nlo;
+        hi = nhi;
+        child = idx;
     }
+    __syncthreads();
+    // a split that one child reached: its sibling reaches out of the CTA
+    if (s_end[k] != 0) s_front[atomicAdd(s_fn, 1)] = s_who[k];
     __syncthreads();
     if (k == 0) s_fn[1] = s_fn[0] ? (int)atomicAdd(A.frontier_count, (unsigned)s_fn[0]) : 0;
     __syncthreads();
     for (int i = k; i < s_fn[0]; i += CB) A.frontier[s_fn[1] + i] = s_front[i];
     // write back the local nodes (index base + k) and the maxHi words of the
     // CTA's positions; phase B raises maxHi further with global atomics
-    const int2 rg = s_rng[k];
-    if (p < n - 1 && rg.x >= base && rg.y <= last) {
+    if (p == 0) A.parent[0] = -1;
+    if (s_split[k] >= 0) {
+        const int s = s_split[k] & (SPLIT_STATE - 1);
+        const int2 rg = s_rng[k];
         __stcg(A.nbmin + p, s_imn[k]);
         __stcg(A.nbmax + p, s_imx[k]);
-        A.state[p] = (uint8_t)s_st[k];
+        A.state[p] = (s_split[k] & SPLIT_STATE) ? 1 : 0;
+        A.left[p] = rg.x == s ? n - 1 + s : s;
+        A.right[p] = rg.y == s + 1 ? n + s : s + 1;
+        __stcg(A.range + p, rg);
     }
+    if (s_up[k] >= 0) A.parent[p] = s_up[k];
+    if (s_lup[k] >= 0) A.parent[n - 1 + p] = s_lup[k];
     if (p < n && s_mh[k] >= 0) A.max_hi[p] = s_mh[k];
 }
 
-__global__ void __launch_bounds__(TB) k_climb_frontier(climb_args A) {
+template <typename K>
+__global__ void __launch_bounds__(TB) k_climb_frontier(climb_args A, const K* __restrict__ keys) {
     const unsigned count = *A.frontier_count;
     const int n = A.n;
     for (unsigned e = blockIdx.x * TB + threadIdx.x; e < count; e += gridDim.x * TB) {
-        int child = A.frontier[e];
-        if ((unsigned)child >= (unsigned)(2 * n - 1)) {
-            hp_report(A.err, HP_DEV_BAD_INDEX, child);
+        const int child0 = A.frontier[e];
+        if ((unsigned)child0 >= (unsigned)(2 * n - 1)) {
+            hp_report(A.err, HP_DEV_BAD_INDEX, child0);
             continue;
         }
-        float4 cmn = __ldcg(A.nbmin + child), cmx = __ldcg(A.nbmax + child);
-        int node = __ldg(A.parent + child);
-        int guard = 0;
-        int nl = 0, nr = 0, nup = -1;  // links of `node`, read a level ahead
-        int2 nrg = make_int2(0, 0);
-        auto links = [&](int i) {
-            if ((unsigned)i < (unsigned)(n - 1)) {
-                nl = __ldg(A.left + i);
-                nr = __ldg(A.right + i);
-                nup = __ldg(A.parent + i);
-                nrg = __ldg(A.range + i);
-            }
-        };
-        links(node);
-        while (node >= 0) {
-            if (node >= n - 1 || ++guard > n) {
-                hp_report(A.err, HP_DEV_BAD_INDEX, node);
+        float4 cmn = __ldcg(A.nbmin + child0), cmx = __ldcg(A.nbmax + child0);
+        const int2 rg = child0 >= n - 1 ? make_int2(child0 - (n - 1), child0 - (n - 1)) : __ldcg(A.range + child0);
+        int lo = rg.x, hi = rg.y, guard = 0;
+        int dl = kdelta(keys, n, lo, lo - 1), dr = kdelta(keys, n, hi, hi + 1);
+        while (hi - lo < n - 1) {
+            const bool is_left = dr > dl;
+            const int s = is_left ? hi : lo - 1;
+            if ((unsigned)s >= (unsigned)(n - 1) || ++guard > n) {
+                hp_report(A.err, HP_DEV_BAD_INDEX, s);
                 break;
             }
-            const int l = nl, r = nr, up = nup;
-            const int2 rg = nrg;
-            links(up);  // while the arrival travels
-            if (hp_arrive(&A.counters[node]) == 0) break;
-            if ((unsigned)l >= (unsigned)(2 * n - 1) || (unsigned)r >= (unsigned)(2 * n - 1) ||
-                (l != child && r != child)) {
-                hp_report(A.err, HP_DEV_BAD_INDEX, node);
+            int old;
+            asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;"
+                         : "=r"(old) : "l"(A.words + s), "r"((is_left ? lo : hi) + 1) : "memory");
+            if (old == 0) break;
+            const int nlo = is_left ? lo : old - 1, nhi = is_left ? old - 1 : hi;
+            if (nlo < 0 || nhi >= n || nlo > s || nhi <= s) {
+                hp_report(A.err, HP_DEV_BAD_INDEX, s);
                 break;
             }
-            const bool is_left = l == child;
-            const int sib = is_left ? r : l;
+            const int lc = nlo == s ? n - 1 + s : s, rc = nhi == s + 1 ? n + s : s + 1;
+            const int sib = is_left ? rc : lc;
             const float4 smn = __ldcg(A.nbmin + sib), smx = __ldcg(A.nbmax + sib);
+            if (is_left) dr = kdelta(keys, n, nhi, nhi + 1);  // the other end's delta stays
+            else dl = kdelta(keys, n, nlo, nlo - 1);
             float4 omn, omx;
             const int st = is_left ? merge_node(A, cmn, cmx, smn, smx, omn, omx)
                                    : merge_node(A, smn, smx, cmn, cmx, omn, omx);
-            __stcg(A.nbmin + node, omn);
-            __stcg(A.nbmax + node, omx);
-            A.state[node] = (uint8_t)st;
-            if (st == 0 && node != 0) atomicMax(&A.max_hi[rg.x], rg.y);
+            const int idx = nhi - nlo == n - 1 ? 0 : (dr > dl ? nhi : nlo);
+            __stcg(A.nbmin + idx, omn);
+            __stcg(A.nbmax + idx, omx);
+            A.state[idx] = (uint8_t)st;
+            A.left[idx] = lc;
+            A.right[idx] = rc;
+            __stcg(A.range + idx, make_int2(nlo, nhi));
+            A.parent[lc] = idx;
+            A.parent[rc] = idx;
+            if (st == 0 && idx != 0) atomicMax(&A.max_hi[nlo], nhi);
             cmn = omn;
             cmx = omx;
-            child = node;
-            node = up;
+            lo = nlo;
+            hi = nhi;
         }
     }
 }
@@ -843,9 +853,6 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
     hp_mark(ctx, s, "morton");
     hp_sort_args sa{keys, nullptr, skeys, out->tri_idx, sort_scratch, hist, true, err, ctx};
     HP_TRY(hp_sort_run(plan, sa, s));
-    k_karras<K><<<grid_n, TB, 0, s>>>(skeys, (int)n, parent, left, right, range);
-    hp_count_launch();
-    hp_mark(ctx, s, "karras");
     k_leaves<<<grid_n, TB, 0, s>>>((int)n, out->tri_idx, m->vertices, m->num_vertices, m->triangles, nbmin,
                                    nbmax, out->woop, p->ci, p->adaptive_leaf, err);
     hp_count_launch();
@@ -854,14 +861,14 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         climb_args A{(int)n, parent, left, right, range, nbmin, nbmax, counters, max_hi, state, frontier,
                      frontier_count, p->ct, p->ci, p->adaptive_leaf,
                      p->max_leaf_size, err};
-        HP_CUDA(cudaFuncSetAttribute(k_climb_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        HP_CUDA(cudaFuncSetAttribute(k_climb_local<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)CLIMB_SMEM));
-        k_climb_local<<<(unsigned)hp_div_up(n, CB), CB, CLIMB_SMEM, s>>>(A);
+        k_climb_local<K><<<(unsigned)hp_div_up(n, CB), CB, CLIMB_SMEM, s>>>(A, skeys);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(ctx, s, "climb_local");
         // at most one entry per reference; small meshes need few CTAs
-        k_climb_frontier<<<(unsigned)std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s>>>(A);
+        k_climb_frontier<K><<<(unsigned)std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s>>>(A, skeys);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
     }

@@ -33,6 +33,15 @@ __device__ __forceinline__ void hp_report(int* status, int code, int info) {
     }
 }
 
+// First statement of a kernel that hp_launch_chained launches: lets the kernel after it
+// place its CTAs, then waits until every kernel before it has ended and its writes are
+// visible. Nothing before it may touch global memory. (Returns at once in a kernel that
+// was launched the ordinary way.)
+__device__ __forceinline__ void hp_after_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Arrival at a node in a bottom-up climb: returns the count before this
 // arrival. The add is acq_rel at GPU scope, so the second thread to arrive sees
 // every write the first one made before its arrival.

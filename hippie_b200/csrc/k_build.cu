@@ -46,7 +46,8 @@ constexpr int TB = 256;
 __global__ void __launch_bounds__(TB) k_tri_boxes(const float* __restrict__ verts, int64_t nv,
                                                   const int32_t* __restrict__ tris, int64_t n,
                                                   float4* __restrict__ bmin, float4* __restrict__ bmax,
-                                                  uint32_t* box_ord, int* err, float4* __restrict__ woop = nullptr) {
+                                                  uint32_t* box_ord, int* err, float4* __restrict__ woop) {
+    hp_after_previous();
     float mn[3] = {HP_MAX_FLOAT, HP_MAX_FLOAT, HP_MAX_FLOAT};
     float mx[3] = {-HP_MAX_FLOAT, -HP_MAX_FLOAT, -HP_MAX_FLOAT};
     for (int64_t i = blockIdx.x * (int64_t)TB + threadIdx.x; i < n; i += (int64_t)gridDim.x * TB) {
@@ -116,6 +117,7 @@ __global__ void __launch_bounds__(TB) k_morton(const float4* __restrict__ bmin,
                                                const float4* __restrict__ bmax, int64_t n,
                                                hp_bvh_info* info, int bits, int hshift, int passes,
                                                K* __restrict__ keys, uint32_t* hist) {
+    hp_after_previous();
     __shared__ uint32_t sh[8 * 256];
     for (int i = threadIdx.x; i < passes * 256; i += TB) sh[i] = 0;
     float smin[3], scale[3];
@@ -203,6 +205,7 @@ __global__ void __launch_bounds__(TB) k_leaves(
     int n, const int32_t* __restrict__ sorted_tri, const float* __restrict__ verts, int64_t nv,
     const int32_t* __restrict__ tris, float4* __restrict__ nbmin, float4* __restrict__ nbmax,
     float4* __restrict__ woop, float ci, int adaptive, int* err) {
+    hp_after_previous();
     const int p = blockIdx.x * TB + threadIdx.x;
     if (p >= n) return;
     const int tri = __ldg(sorted_tri + p);
@@ -299,6 +302,7 @@ __device__ __forceinline__ int merge_node(const climb_args& A, float4 lmn, float
 
 template <typename K>
 __global__ void __launch_bounds__(CB, 4) k_climb_local(climb_args A, const K* __restrict__ keys) {
+    hp_after_previous();
     extern __shared__ __align__(16) unsigned char climb_smem[];
     float4* s_imn = reinterpret_cast<float4*>(climb_smem);  // local interior node base + k
     float4* s_imx = s_imn + CB;
@@ -399,6 +403,7 @@ __global__ void __launch_bounds__(CB, 4) k_climb_local(climb_args A, const K* __
 
 template <typename K>
 __global__ void __launch_bounds__(TB) k_climb_frontier(climb_args A, const K* __restrict__ keys) {
+    hp_after_previous();
     const unsigned count = *A.frontier_count;
     const int n = A.n;
     for (unsigned e = blockIdx.x * TB + threadIdx.x; e < count; e += gridDim.x * TB) {
@@ -487,6 +492,7 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) k_collapse_small(
     int n, const int* __restrict__ left, const int2* __restrict__ range, const uint8_t* __restrict__ state,
     const int* __restrict__ max_hi, int* __restrict__ reach, int* __restrict__ rank_int,
     int* __restrict__ rank_leaf, int* __restrict__ totals) {
+    hp_after_previous();
     extern __shared__ __align__(16) unsigned char sc_raw[];
     int* s_hi = reinterpret_cast<int*>(sc_raw);  // [SC_CAP]
     int* s_reach = s_hi + SC_CAP;                // [SC_CAP]
@@ -592,6 +598,7 @@ __device__ __forceinline__ void put_node(hp_node_bin* nodes, int idx, int max_no
 __global__ void __launch_bounds__(TB) k_emit(emit_ctx e, const int* __restrict__ max_hi,
                                              const int* __restrict__ reach, hp_bvh_info* info,
                                              hp_node_bin* __restrict__ nodes, int max_nodes, int* err) {
+    hp_after_previous();
     const int t = blockIdx.x * TB + threadIdx.x;
     const int n = e.n;
     if (t >= 2 * n - 1) return;
@@ -748,11 +755,11 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         float4* woop_src = wide ? nullptr : cv.take<float4>(3 * n);
         k_init_build<<<hp_div_up(plan.passes * 256, TB), TB, 0, s>>>(info, hist, plan.passes * 256, nullptr, nullptr, 0,
                                                                      nullptr);
-        k_tri_boxes<<<grid_red, TB, 0, s>>>(m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
+        HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
                                             info->box_ord, err, woop_src);
         hp_count_launch(2);
         hp_mark(ctx, s, "boxes");
-        k_morton<K><<<grid_mor, TB, 0, s>>>(tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
+        HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(ctx, s, "morton");
@@ -782,11 +789,11 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
             cv.take<char>(std::max(hp_atr_scratch_bytes(n), hlbvh ? hp_hlbvh_scratch_bytes(n, p->hlbvh_sah_bits) : 0));
         k_init_build<<<hp_div_up(plan.passes * 256, TB), TB, 0, s>>>(info, hist, plan.passes * 256, nullptr, nullptr, 0,
                                                                      nullptr);
-        k_tri_boxes<<<grid_red, TB, 0, s>>>(m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-                                            info->box_ord, err);
+        HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
+                                            info->box_ord, err, nullptr);
         hp_count_launch(2);
         hp_mark(ctx, s, "boxes");
-        k_morton<K><<<grid_mor, TB, 0, s>>>(tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
+        HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(ctx, s, "morton");
@@ -843,17 +850,17 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
     unsigned* frontier_count = reinterpret_cast<unsigned*>(ctx->d_status + 32);
     k_init_build<<<std::max(hp_div_up(plan.passes * 256, TB), grid_red), TB, 0, s>>>(
         info, hist, plan.passes * 256, counters, max_hi, n, frontier_count);
-    k_tri_boxes<<<grid_red, TB, 0, s>>>(m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-                                        info->box_ord, err);
+    HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
+                                        info->box_ord, err, nullptr);
     hp_count_launch(2);
     hp_mark(ctx, s, "boxes");
-    k_morton<K><<<grid_mor, TB, 0, s>>>(tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
+    HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "morton");
     hp_sort_args sa{keys, nullptr, skeys, out->tri_idx, sort_scratch, hist, true, err, ctx};
     HP_TRY(hp_sort_run(plan, sa, s));
-    k_leaves<<<grid_n, TB, 0, s>>>((int)n, out->tri_idx, m->vertices, m->num_vertices, m->triangles, nbmin,
+    HP_CHAIN(k_leaves, grid_n, TB, 0, s, (int)n, out->tri_idx, m->vertices, m->num_vertices, m->triangles, nbmin,
                                    nbmax, out->woop, p->ci, p->adaptive_leaf, err);
     hp_count_launch();
     hp_mark(ctx, s, "leaves");
@@ -863,12 +870,12 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
                      p->max_leaf_size, err};
         HP_CUDA(cudaFuncSetAttribute(k_climb_local<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)CLIMB_SMEM));
-        k_climb_local<K><<<(unsigned)hp_div_up(n, CB), CB, CLIMB_SMEM, s>>>(A, skeys);
+        HP_CHAIN(k_climb_local<K>, hp_div_up(n, CB), CB, CLIMB_SMEM, s, A, skeys);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(ctx, s, "climb_local");
         // at most one entry per reference; small meshes need few CTAs
-        k_climb_frontier<K><<<(unsigned)std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s>>>(A, skeys);
+        HP_CHAIN(k_climb_frontier<K>, std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s, A, skeys);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
     }
@@ -895,7 +902,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
     } else {
     if (n <= SC_CAP) {
         HP_CUDA(cudaFuncSetAttribute(k_collapse_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC_SMEM));
-        k_collapse_small<<<1, SC_BLOCK, SC_SMEM, s>>>((int)n, left, range, state, max_hi, reach, rank_int, rank_leaf,
+        HP_CHAIN(k_collapse_small, 1, SC_BLOCK, SC_SMEM, s, (int)n, left, range, state, max_hi, reach, rank_int, rank_leaf,
                                                      &info->num_interior);
     } else {
         hp_scan_max_excl(max_hi, n, reach, scan_a, err, s);
@@ -904,7 +911,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         hp_scan2_sum(flag_int, n - 1, flag_leaf, n, rank_int, rank_leaf, &info->num_interior, scan_b, err, s);
     }
     emit_ctx e{(int)n, left, right, parent, range, state, rank_int, rank_leaf, nbmin, nbmax};
-    k_emit<<<hp_div_up(nn, TB), TB, 0, s>>>(e, max_hi, reach, info, out->nodes,
+    HP_CHAIN(k_emit, hp_div_up(nn, TB), TB, 0, s, e, max_hi, reach, info, out->nodes,
                                             (int)std::max<int64_t>(2 * out->capacity - 1, 3), err);
     HP_CUDA(cudaGetLastError());
     hp_count_launch(2);

@@ -189,6 +189,7 @@ __device__ __forceinline__ void make_parent_from(const ploc_args& A, int node, i
 __global__ void __launch_bounds__(256) k_ploc_leaves(ploc_args A, const int32_t* __restrict__ sorted_tri,
                                                      const float4* __restrict__ tbmin,
                                                      const float4* __restrict__ tbmax) {
+    hp_after_previous();
     const int p = blockIdx.x * 256 + threadIdx.x;
     if (p >= A.n) return;
     const int tri = sorted_tri[p];
@@ -806,6 +807,7 @@ __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
 constexpr size_t TAIL_SMEM = 12 * TAIL * sizeof(float);
 
 __global__ void __launch_bounds__(PB, 1) k_ploc_tail(ploc_args A) {
+    hp_after_previous();
     extern __shared__ float s_tail[];
     float(*smn)[TAIL] = reinterpret_cast<float(*)[TAIL]>(s_tail);
     float(*smx)[TAIL] = reinterpret_cast<float(*)[TAIL]>(s_tail + 3 * TAIL);
@@ -978,6 +980,7 @@ __device__ __forceinline__ void td_put(const td_args& T, int idx, const hp_node_
 // gathering its sibling's and its children's counts, states and boxes.
 template <bool PRE>
 __global__ void __launch_bounds__(256) k_topdown(td_args T) {
+    hp_after_previous();
     __shared__ unsigned s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(T.ticket, 1u);
     __syncthreads();
@@ -1223,7 +1226,7 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
         hp_mark(ctx, s, "ploc_loop");
     }
     HP_CUDA(cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM));
-    k_ploc_tail<<<1, PB, TAIL_SMEM, s>>>(A);
+    HP_CHAIN(k_ploc_tail, 1, PB, TAIL_SMEM, s, A);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "ploc_tail");
@@ -1270,7 +1273,7 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
     T.err = ctx->d_status;
     T.cinfo = A.cinfo;
     T.cbox = A.cbox;
-    k_topdown<true><<<hp_div_up(nn, 256), 256, 0, s>>>(T);
+    HP_CHAIN(k_topdown<true>, hp_div_up(nn, 256), 256, 0, s, T);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "collapse");

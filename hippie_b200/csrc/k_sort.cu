@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(BLOCK) k_onesweep(
     K* __restrict__ keys_out, int32_t* __restrict__ vals_out, int64_t n, int shift,
     uint32_t dmask, const uint32_t* __restrict__ hist, uint32_t* status,
     uint32_t* tile_counter, int* err, uint32_t spin_limit) {
+    hp_after_previous();
     constexpr int NW = BLOCK / 32;
     constexpr int TILE = BLOCK * ITEMS;
     static_assert(BLOCK >= 256, "one thread per digit");
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__
                                                            const int32_t* __restrict__ vals_in,
                                                            K* __restrict__ keys_out, int32_t* __restrict__ vals_out,
                                                            int n, int bits) {
+    hp_after_previous();
     constexpr int NW = ONE_BLOCK / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);   // [NW][256] while ranking
@@ -710,6 +712,7 @@ __global__ void __launch_bounds__(SEG_BLOCK, 4) k_seg_sort(const uint64_t* __res
                                                         uint64_t* __restrict__ kout, int32_t* __restrict__ vout,
                                                         int64_t n, int L, int2* big, uint32_t* big_count,
                                                         int64_t big_cap, int* err) {
+    hp_after_previous();
     extern __shared__ __align__(16) unsigned char seg_raw[];
     seg_smem& S = *reinterpret_cast<seg_smem*>(seg_raw);
     const int tid = threadIdx.x;
@@ -795,6 +798,7 @@ __global__ void __launch_bounds__(SEG_BLOCK, 4) k_seg_big(uint64_t* kin, int32_t
                                                        uint64_t* kout, int32_t* vout, int L, const int2* big,
                                                        const uint32_t* big_count, int64_t big_cap, int64_t n,
                                                        int* err) {
+    hp_after_previous();
     extern __shared__ __align__(16) unsigned char seg_raw[];
     seg_smem& S = *reinterpret_cast<seg_smem*>(seg_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -871,7 +875,7 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
     if (plan.n <= ONE_CAP) {
         constexpr size_t one_smem = sort_one_smem<K>();
         HP_CUDA(cudaFuncSetAttribute(k_sort_one<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one_smem));
-        k_sort_one<K><<<1, ONE_BLOCK, one_smem, stream>>>(reinterpret_cast<const K*>(a.keys_in), a.vals_in,
+        HP_CHAIN(k_sort_one<K>, 1, ONE_BLOCK, one_smem, stream, reinterpret_cast<const K*>(a.keys_in), a.vals_in,
                                                           reinterpret_cast<K*>(a.keys_out), a.vals_out, (int)plan.n,
                                                           plan.bits);
         HP_CUDA(cudaGetLastError());
@@ -920,7 +924,7 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
             for (int d = 0; d < SEG_TOP; ++d) {  // in -> A -> B -> A
                 K* dk = (d & 1) ? kB : kA;
                 int32_t* dv = (d & 1) ? vB : vA;
-                k_onesweep<K, BLOCK, ITEMS><<<(unsigned)plan.tiles, BLOCK, smem, stream>>>(
+                HP_CHAIN((k_onesweep<K, BLOCK, ITEMS>), plan.tiles, BLOCK, smem, stream, 
                     src_k, src_v, dk, dv, n, s0 + 8 * d, 0xffu, a.hist + 256 * d,
                     status + (size_t)d * plan.tiles * 256, counters + d, a.status, sl);
                 HP_CUDA(cudaGetLastError());
@@ -937,11 +941,11 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
             const size_t seg_bytes = sizeof(seg_smem);
             HP_CUDA(cudaFuncSetAttribute(k_seg_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_bytes));
             HP_CUDA(cudaFuncSetAttribute(k_seg_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_bytes));
-            k_seg_sort<<<(unsigned)hp_div_up(n, SEG_WINDOW), SEG_BLOCK, seg_bytes, stream>>>(
+            HP_CHAIN(k_seg_sort, hp_div_up(n, SEG_WINDOW), SEG_BLOCK, seg_bytes, stream, 
                 sk, sv, reinterpret_cast<uint64_t*>(a.keys_out), a.vals_out, n, s0, big, big_count, big_cap,
                 a.status);
             HP_CUDA(cudaGetLastError());
-            k_seg_big<<<(unsigned)std::min<int64_t>(big_cap, 296), SEG_BLOCK, seg_bytes, stream>>>(
+            HP_CHAIN(k_seg_big, std::min<int64_t>(big_cap, 296), SEG_BLOCK, seg_bytes, stream, 
                 sk, sv, sv, reinterpret_cast<uint64_t*>(a.keys_out), a.vals_out, s0, big, big_count, big_cap, n,
                 a.status);
             HP_CUDA(cudaGetLastError());
@@ -965,7 +969,7 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
         }
         int shift = 8 * p;
         int w = std::min(8, plan.bits - shift);
-        k_onesweep<K, BLOCK, ITEMS><<<(unsigned)plan.tiles, BLOCK, smem, stream>>>(
+        HP_CHAIN((k_onesweep<K, BLOCK, ITEMS>), plan.tiles, BLOCK, smem, stream, 
             kin, vin, kout, vout, n, shift, (1u << w) - 1u, a.hist + 256 * p,
             status + (size_t)p * plan.tiles * 256, counters + p, a.status,
             a.ctx ? a.ctx->sort_spin_limit : LOOKBACK_SPIN_LIMIT);

@@ -59,13 +59,13 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 // cycles of an SM's L1 when it comes from L2 and 1.4 when it hits, and a bounce
 // ray of the 4.2 M-triangle scene takes 79 nodes, 6 leaves and 14 triangles. So a
 // warp stays in one piece and takes three kinds of turns, all 32 lanes together,
-// decided by ballots:
+// decided by ballots (node_min and tri_min are NODE_MIN and TRI_MIN, or 1 for few rays):
 //   * nodes: every lane at an interior node does one. The first leaf that a lane
 //     meets is postponed and the lane goes on from its stack; at a second one it
-//     waits. The turn ends when fewer than NODE_MIN lanes have an interior node
+//     waits. The turn ends when fewer than node_min lanes have an interior node
 //     and no postponed leaf, so that a hit is found, and shortens the ray, soon;
 //   * triangles: every lane with a postponed leaf tests one triangle, until fewer
-//     than TRI_MIN lanes have one;
+//     than tri_min lanes have one;
 //   * new rays: once FETCH_MIN lanes are without work.
 // A stack entry keeps the child's entry distance, and an entry beyond the hit
 // found since is dropped at the pop: its boxes would all be missed (a child's
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
-    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order) {
+    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, int node_min, int tri_min) {
     constexpr int LST = STACK - SST;
     __shared__ int2 s_stack[SST * TRACE_BLOCK];
     int2* sstack = s_stack + threadIdx.x;
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
             }
             go = (unsigned)node < (unsigned)SENTINEL;
             mask = __ballot_sync(HP_FULL_MASK, go && leaf >= 0 && tri >= tri_end);
-            if (__popc(mask) < NODE_MIN) break;
+            if (__popc(mask) < node_min) break;
         }
 
         // Leaves: one triangle per lane and round.
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
             }
             pend = node < 0 || leaf < 0 || tri < tri_end;
             mask = __ballot_sync(HP_FULL_MASK, pend);
-            if (__popc(mask) < TRI_MIN) break;
+            if (__popc(mask) < tri_min) break;
         }
     }
 }
@@ -323,6 +323,16 @@ int trace_grid(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
     return (int)std::max<int64_t>(grid, 1);
 }
 
+// A launch that has no two rays for a lane lasts as long as its slowest warps: their
+// lanes take every turn they can, instead of waiting for a fuller one (137 K primary
+// rays in 1.7 M triangles on a B200 299 -> 268 us, 205 K sorted ones on a terrain 240 ->
+// 220 us; as a rule for 4 or 8 rays a lane 1 M shadow rays lose 6 %).
+bool few_rays(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
+    return num_rays < 2 * (int64_t)ctx->sm_count * std::max(per_sm, 1) * TRACE_BLOCK;
+}
+int node_min(const hp_ctx* ctx, int per_sm, int64_t num_rays) { return few_rays(ctx, per_sm, num_rays) ? 1 : NODE_MIN; }
+int tri_min(const hp_ctx* ctx, int per_sm, int64_t num_rays) { return few_rays(ctx, per_sm, num_rays) ? 1 : TRI_MIN; }
+
 template <bool A, bool S, int SST>
 hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const float* rays,
                    int64_t num_rays, int32_t* results, int32_t* stats, unsigned long long* counter,
@@ -333,7 +343,8 @@ hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const floa
     k_trace<A, S, false, SST><<<trace_grid(ctx, per_sm, num_rays), TRACE_BLOCK, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const float4*>(b->nodes), b->woop, b->tri_idx,
-        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order);
+        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order,
+        node_min(ctx, per_sm, num_rays), tri_min(ctx, per_sm, num_rays));
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");
@@ -347,7 +358,9 @@ hp_status launch_st(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const flo
     switch (ctx->tune.trace_stack) {
         case 8: return launch_t<A, S, 8>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
         case 32: return launch_t<A, S, 32>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
-        default: return launch_t<A, S, 16>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+        // the default choice of 16: two entries fewer leave the L1 more of the SM's memory
+        // (bounce rays 19.86 -> 19.58 ms; at 20 entries, with less than 64 KB left, 35.8)
+        default: return launch_t<A, S, 14>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
     }
 }
 

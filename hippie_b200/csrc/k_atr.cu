@@ -333,8 +333,7 @@ __device__ void atr_treelet(const atr_args& A, int root, float root_cost, int l0
         __stcg(A.nbmin + node, olo);
         __stcg(A.nbmax + node, ohi);
     }
-    __threadfence();
-    __syncwarp();
+    __syncwarp();  // the lane that climbs on releases every lane's writes with its next arrival
 }
 
 // TRBVH treelet optimisation (TRBuilderKernels.cu:12-300) for the treelet at
@@ -483,8 +482,7 @@ __device__ void tr_treelet(const atr_args& A, int root, float root_cost, int roo
             nr = no;
         }
     }
-    __threadfence();
-    __syncwarp();
+    __syncwarp();  // the lane that climbs on releases every lane's writes with its next arrival
 }
 
 template <bool TR>

@@ -43,17 +43,26 @@ namespace {
 constexpr int PB = 1024;            // threads of the tail CTA
 constexpr int LPB = 512;            // threads per CTA of the iteration kernel (two CTAs per SM)
 constexpr int MAXR = 512;           // largest radius kept in a shared-memory window
+// The iteration kernel is compiled for windows of radii up to R = 32 and up to MAXR: what
+// shared memory a CTA does not take is the L1's, through which all of a tile's loads
+// pass on their way: 60 KB a CTA instead of 87, iterations on 4.2 M clusters 1.75 -> 1.67 ms
+// on a B200 (and with 103 KB, for a tile's merges kept over the next tile's search, 1.97).
+constexpr int SMALL_R = 32;
 constexpr int NB4 = 4;              // clusters per thread of the neighbour search on large lists
 // Neighbour window: the stride of its six arrays. Threads that search for four
 // clusters each read window entries four apart; as they lie, that is four lanes to a
 // bank and the search waits for shared memory. So a window of theirs is stored by the
-// entry's index modulo 4, in four rows of WQ entries (entry k at win4(k)): lanes then
-// read neighbours, and WQ = 8 modulo 32 spreads the consecutive stores of a warp over
+// entry's index modulo 4, in four rows of Q entries (entry k at at4(k)): lanes then
+// read neighbours, and Q = 8 modulo 32 spreads the consecutive stores of a warp over
 // all banks too.
-constexpr int WQ = (NB4 * LPB + 2 * MAXR) / 4 + 8;
-constexpr int WIN = 4 * WQ;
-static_assert(WQ % 32 == 8, "the four rows start eight banks apart");
-__device__ __forceinline__ int win4(int k) { return (k & 3) * WQ + (k >> 2); }
+template <int R>
+struct win {
+    static constexpr int Q = (((NB4 * LPB + 2 * R) / 4 + 31) / 32) * 32 + 8;  // row
+    static constexpr int S = 4 * Q;                                           // stride
+    static constexpr int NN = NB4 * LPB + 2 * R;  // neighbour slots of a tile and its halo
+    static constexpr size_t SMEM = 6 * S * sizeof(float) + NN * sizeof(int);
+    static __device__ __forceinline__ int at4(int k) { return (k & 3) * Q + (k >> 2); }
+};
 // Lists at least this long use 4 clusters per thread (long tiles, about half as
 // many tiles as the loop has CTAs at this length). On a B200 this beat twice
 // and four times the length, half and a quarter of it, and long tiles at every
@@ -62,14 +71,12 @@ constexpr int NB4_MIN_N = 148 * NB4 * 512;
 // Shorter lists run fused iterations: a tile of LPB clusters finds the nearest
 // neighbours of its clusters and of r clusters on each side itself, so each
 // iteration needs one grid barrier instead of two.
-constexpr int NNF = NB4 * LPB + 2 * MAXR;       // neighbour slots of a tile and its halo
 constexpr int MIN_TILE4 = NB4 * LPB - 2 * MAXR;  // fewest clusters of a tile of the long lists
 // Clusters of a fused tile: LPB - 2r (one thread per cluster of the tile and its
 // halo), at least LPB / 2.
 __host__ __device__ constexpr int fused_tile(int r) { return 2 * r <= LPB / 2 ? LPB - 2 * r : LPB / 2; }
 // Clusters of a tile of the long lists: 4*LPB - 2r, at least 2*LPB.
 __host__ __device__ constexpr int long_tile(int r) { return 2 * r <= 2 * LPB ? NB4 * LPB - 2 * r : 2 * LPB; }
-constexpr size_t LOOP_SMEM = 6 * WIN * sizeof(float) + NNF * sizeof(int);
 constexpr int TAIL = 2048;          // most clusters finished by a single CTA
 // Clusters that the iteration kernel leaves to it (an iteration of the CTA takes 6 us
 // at 650 clusters, 4 us at 450 and 2.4 us below 60, one of the short lists' tiles 8 us;
@@ -219,10 +226,10 @@ __global__ void __launch_bounds__(256) k_ploc_leaves(ploc_args A, const int32_t*
 // never the nearest, outside the cluster list). The cluster indices of a batch
 // of elements are read first and their boxes after, so that a thread has a
 // batch of loads in flight instead of one dependent pair at a time.
-template <bool ROWS4>
+template <int R, bool ROWS4>
 __device__ __forceinline__ void load_window(const ploc_args& A, const int* __restrict__ cl, int N, int w0, int wn,
                                             float* s) {
-    constexpr int BATCH = 3;
+    constexpr int BATCH = 3, WIN = win<R>::S;
     for (int k0 = threadIdx.x; k0 < wn; k0 += BATCH * LPB) {
         int node[BATCH];
 #pragma unroll
@@ -244,7 +251,7 @@ __device__ __forceinline__ void load_window(const ploc_args& A, const int* __res
 #pragma unroll
         for (int u = 0; u < BATCH; ++u) {
             if (k0 + u * LPB < wn) {
-                const int k = ROWS4 ? win4(k0 + u * LPB) : k0 + u * LPB;
+                const int k = ROWS4 ? win<R>::at4(k0 + u * LPB) : k0 + u * LPB;
                 s[k] = mn[u].x; s[WIN + k] = mn[u].y; s[2 * WIN + k] = mn[u].z;
                 s[3 * WIN + k] = mx[u].x; s[4 * WIN + k] = mx[u].y; s[5 * WIN + k] = mx[u].z;
             }
@@ -252,9 +259,10 @@ __device__ __forceinline__ void load_window(const ploc_args& A, const int* __res
     }
 }
 
-template <int B>
+template <int R, int B>
 __device__ void nn_tile(const ploc_args& A, const int* __restrict__ cl, int N, int r, int base, float* s,
                         int* s_nn) {
+    constexpr int WIN = win<R>::S;
     float* smnx = s;
     float* smny = s + WIN;
     float* smnz = s + 2 * WIN;
@@ -263,14 +271,14 @@ __device__ void nn_tile(const ploc_args& A, const int* __restrict__ cl, int N, i
     float* smxz = s + 5 * WIN;
     constexpr int TS = B * LPB;
     __syncthreads();
-    load_window<true>(A, cl, N, base - r, TS + 2 * r, s);
+    load_window<R, true>(A, cl, N, base - r, TS + 2 * r, s);
     __syncthreads();
     const int l0 = threadIdx.x * B;  // cluster base + l sits at window position l + r
     float ax[B], ay[B], az[B], bx[B], by[B], bz[B], best[B];
     int bi[B];
 #pragma unroll
     for (int q = 0; q < B; ++q) {
-        const int me = win4(l0 + q + r);
+        const int me = win<R>::at4(l0 + q + r);
         ax[q] = smnx[me]; ay[q] = smny[me]; az[q] = smnz[me];
         bx[q] = smxx[me]; by[q] = smxy[me]; bz[q] = smxz[me];
         best[q] = HP_MAX_FLOAT;
@@ -285,7 +293,7 @@ __device__ void nn_tile(const ploc_args& A, const int* __restrict__ cl, int N, i
         }
     };
 #define HP_PLOC_CAND(k)                                                             \
-    const int w_ = win4(k);                                                          \
+    const int w_ = win<R>::at4(k);                                                          \
     const float cx = smnx[w_], cy = smny[w_], cz = smnz[w_], dx = smxx[w_], dy = smxy[w_], dz = smxz[w_]
     if (B == 1 || r < 4) {
         for (int k = l0; k <= l0 + (B - 1) + 2 * r; ++k) {
@@ -378,8 +386,10 @@ __device__ __forceinline__ int2 block_scan2(int& a, int& b, int* s_wa, int* s_wb
 // tile (s_nn[l] for cluster tbase - r + l), from the boxes of clusters
 // [tbase - 2r, tbase + tsz + 2r) in shared memory; candidates in increasing
 // order, the first strict minimum, as in nn_tile.
+template <int R>
 __device__ void nn_halo(const ploc_args& A, const int* __restrict__ cl, int N, int r, int tbase, int tsz, float* s,
                         int* s_nn) {
+    constexpr int WIN = win<R>::S;
     float* smnx = s;
     float* smny = s + WIN;
     float* smnz = s + 2 * WIN;
@@ -387,7 +397,7 @@ __device__ void nn_halo(const ploc_args& A, const int* __restrict__ cl, int N, i
     float* smxy = s + 4 * WIN;
     float* smxz = s + 5 * WIN;
     const int w0 = tbase - 2 * r;
-    load_window<false>(A, cl, N, w0, tsz + 4 * r, s);
+    load_window<R, false>(A, cl, N, w0, tsz + 4 * r, s);
     __syncthreads();
     for (int l = threadIdx.x; l < tsz + 2 * r; l += LPB) {
         const int c = tbase - r + l;
@@ -414,15 +424,15 @@ __device__ void nn_halo(const ploc_args& A, const int* __restrict__ cl, int N, i
 // One merge tile of at most ITEMS*LPB clusters: flags, prefix sums (tile + look-back),
 // new nodes, compaction. FUSED tiles (ITEMS 1) find their neighbours first;
 // the others read the neighbour phase's results.
-template <int ITEMS>
+template <int R, int ITEMS>
 __device__ void merge_tile(const ploc_args& A, const int* __restrict__ cl_in, int* __restrict__ cl_out,
                            int N, int r, int it, unsigned tile, int TSZ, unsigned long long* status, float* s_win,
                            int* s_nn, int* s_wa, int* s_wb, unsigned* s_pref) {
     const unsigned tag = (unsigned)(it % 15) + 1u;
     const int tbase = (int)tile * TSZ;
     __syncthreads();  // the previous tile's shared memory is free
-    if (ITEMS == 1) nn_halo(A, cl_in, N, r, tbase, TSZ, s_win, s_nn);
-    else nn_tile<ITEMS>(A, cl_in, N, r, tbase - r, s_win, s_nn);  // TSZ + 2r <= ITEMS * LPB clusters
+    if (ITEMS == 1) nn_halo<R>(A, cl_in, N, r, tbase, TSZ, s_win, s_nn);
+    else nn_tile<R, ITEMS>(A, cl_in, N, r, tbase - r, s_win, s_nn);  // TSZ + 2r <= ITEMS * LPB clusters
     const int nlo = tbase - r;  // cluster of s_nn[0]
     auto nn_of = [&](int c) { return s_nn[c - nlo]; };
     const int base = tbase + threadIdx.x * ITEMS;
@@ -587,6 +597,7 @@ struct small_state {
 // Clusters of a tile with S lanes per cluster (0: none).
 __host__ __device__ constexpr int small_tile(int r, int S) { return LPB / S - 2 * r >= 32 ? LPB / S - 2 * r : 0; }
 
+template <int R>
 __device__ void small_iteration(const ploc_args& A, const int* __restrict__ cl_in, int* __restrict__ cl_out, int N,
                                 int r, int it, int tsz, int S, float* s_win, int* s_nn, int* s_wa, int* s_wb,
                                 unsigned* s_pref, small_state* out) {
@@ -598,7 +609,7 @@ __device__ void small_iteration(const ploc_args& A, const int* __restrict__ cl_i
     float4 amn{}, amx{}, bmn{}, bmx{};  // the two clusters of a merge
     int2 ca{}, cb{};
     if (mine) {
-        load_window<false>(A, cl_in, N, tbase - 2 * r, tsz + 4 * r, s_win);
+        load_window<R, false>(A, cl_in, N, tbase - 2 * r, tsz + 4 * r, s_win);
         __syncthreads();
         // neighbours of the tile's clusters and of r on each side: lanes sub, sub + S,
         // ... of the candidates, then the least distance and of equal ones the first
@@ -608,6 +619,7 @@ __device__ void small_iteration(const ploc_args& A, const int* __restrict__ cl_i
         float best = HP_MAX_FLOAT;
         int bi = -1;
         if (l < tsz + 2 * r && c >= 0 && c < N) {
+            constexpr int WIN = win<R>::S;
             const float *mnx = s_win, *mny = s_win + WIN, *mnz = s_win + 2 * WIN;
             const float *mxx = s_win + 3 * WIN, *mxy = s_win + 4 * WIN, *mxz = s_win + 5 * WIN;
             const int me = l + r;
@@ -733,9 +745,10 @@ __device__ __forceinline__ bool barrier_of(unsigned* bar, unsigned count, unsign
     return *s_ok != 0;
 }
 
+template <int R>
 __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
     extern __shared__ float s_win[];
-    int* s_nn = reinterpret_cast<int*>(s_win + 6 * WIN);
+    int* s_nn = reinterpret_cast<int*>(s_win + 6 * win<R>::S);
     __shared__ int s_wa[LPB / 32 + 1], s_wb[LPB / 32 + 1];
     __shared__ unsigned s_pref[2];
     __shared__ unsigned s_ticket;
@@ -771,12 +784,12 @@ __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
                 const unsigned tile = s_ticket;
                 __syncthreads();
                 if ((long)tile * tsz >= N) break;
-                merge_tile<NB4>(A, cl_in, cl_out, N, r, it, tile, tsz, A.status, s_win, s_nn, s_wa, s_wb, s_pref);
+                merge_tile<R, NB4>(A, cl_in, cl_out, N, r, it, tile, tsz, A.status, s_win, s_nn, s_wa, s_wb, s_pref);
             }
         } else {
             const int tsz = fused_tile(rt);
             for (unsigned tile = blockIdx.x; (long)tile * tsz < N; tile += gridDim.x)
-                merge_tile<1>(A, cl_in, cl_out, N, r, it, tile, tsz, A.status_f, s_win, s_nn, s_wa, s_wb, s_pref);
+                merge_tile<R, 1>(A, cl_in, cl_out, N, r, it, tile, tsz, A.status_f, s_win, s_nn, s_wa, s_wb, s_pref);
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) A.g[1] = it + 1;
         if (!barrier_of(A.bar, gridDim.x, gen, A.err, &s_ok)) return;
@@ -792,7 +805,7 @@ __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
         if ((int)blockIdx.x >= count) return;
         const int* cl_in = (it & 1) ? A.cl1 : A.cl0;
         int* cl_out = (it & 1) ? A.cl0 : A.cl1;
-        small_iteration(A, cl_in, cl_out, N, radius_at(A, it), it, tsz, S, s_win, s_nn, s_wa, s_wb, s_pref, &s_small);
+        small_iteration<R>(A, cl_in, cl_out, N, radius_at(A, it), it, tsz, S, s_win, s_nn, s_wa, s_wb, s_pref, &s_small);
         N = s_small.n;
         if (!s_small.ok) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1214,14 +1227,16 @@ hp_status hp_ploc_stage(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p,
     hp_count_launch();
     hp_mark(ctx, s, "ploc_leaves");
     if (n > TAIL) {
-        const size_t smem = LOOP_SMEM;
-        HP_CUDA(cudaFuncSetAttribute(k_ploc_loop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const bool small = r_max <= SMALL_R;
+        const void* loop = small ? (const void*)k_ploc_loop<SMALL_R> : (const void*)k_ploc_loop<MAXR>;
+        const size_t smem = small ? win<SMALL_R>::SMEM : win<MAXR>::SMEM;
+        HP_CUDA(cudaFuncSetAttribute(loop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
-        HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ploc_loop, LPB, smem));
+        HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, loop, LPB, smem));
         if (per_sm < 1) return hp_fail(HP_ERR_UNSUPPORTED, "PLOC loop kernel does not fit on an SM");
         const int grid = std::min(ctx->sm_count * per_sm, LOOP_MAX_GRID);
         void* args[] = {&A};
-        HP_CUDA(cudaLaunchCooperativeKernel((void*)k_ploc_loop, grid, LPB, args, smem, s));
+        HP_CUDA(cudaLaunchCooperativeKernel(loop, grid, LPB, args, smem, s));
         hp_count_launch();
         hp_mark(ctx, s, "ploc_loop");
     }

@@ -92,11 +92,12 @@ __global__ void k_b_init(bargs B, int hist_words) {
 
 // Mesh of triangle g: two threads of the CTA look up its first and its last
 // triangle, the others only between them (one mesh, for most CTAs). Every thread of
-// the CTA calls it; -1 past the last triangle. `one` tells whether the whole CTA lies
-// in one mesh.
-__device__ __forceinline__ int cta_seg(const bargs& B, int64_t g, bool& one) {
+// the CTA calls it, for the TB triangles from `first` on; -1 past the last triangle. `one`
+// tells whether the whole CTA lies in one mesh.
+__device__ __forceinline__ int cta_seg(const bargs& B, int64_t first, bool& one) {
     __shared__ int s_m[2];
-    const int64_t first = blockIdx.x * (int64_t)TB, last = min(first + TB, B.N) - 1;
+    const int64_t g = first + threadIdx.x, last = min(first + TB, B.N) - 1;
+    __syncthreads();
     if (threadIdx.x == 0) s_m[0] = seg_of(B.tri_off, B.M, first);
     if (threadIdx.x == 32) s_m[1] = seg_of(B.tri_off, B.M, last);
     __syncthreads();
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(TB) k_b_boxes(bargs B) {
     const int64_t g = blockIdx.x * (int64_t)TB + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool one;
-    const int m = cta_seg(B, g, one);
+    const int m = cta_seg(B, blockIdx.x * (int64_t)TB, one);
     uint32_t o[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     if (m >= 0) {
         const hp_batch_seg sg = B.seg[m];
@@ -167,30 +168,34 @@ __global__ void __launch_bounds__(TB) k_b_boxes(bargs B) {
 __global__ void __launch_bounds__(TB) k_b_morton(bargs B) {
     __shared__ uint32_t sh[8 * 256];
     for (int i = threadIdx.x; i < B.passes * 256; i += TB) sh[i] = 0;
-    const int64_t g = blockIdx.x * (int64_t)TB + threadIdx.x;
-    bool one;
-    const int m = cta_seg(B, g, one);  // synchronises
-    uint64_t key = 0;
-    if (m >= 0) {
-        const hp_bvh_info& in = B.info[m];
-        float smin[3], scale[3];
+    // The CTAs resident at once walk the triangles: every CTA adds its counts to the
+    // histograms once, whose words all of them share.
+    for (int64_t first = blockIdx.x * (int64_t)TB; first < B.N; first += (int64_t)gridDim.x * TB) {
+        const int64_t g = first + threadIdx.x;
+        bool one;
+        const int m = cta_seg(B, first, one);  // synchronises
+        uint64_t key = 0;
+        if (m >= 0) {
+            const hp_bvh_info& in = B.info[m];
+            float smin[3], scale[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            smin[k] = hp_ord2f(in.box_ord[k]);
-            scale[k] = __fdividef(1.0f, __fsub_rn(hp_ord2f(in.box_ord[3 + k]), smin[k]));
+            for (int k = 0; k < 3; ++k) {
+                smin[k] = hp_ord2f(in.box_ord[k]);
+                scale[k] = __fdividef(1.0f, __fsub_rn(hp_ord2f(in.box_ord[3 + k]), smin[k]));
+            }
+            const float4 a = B.tbmin[g], b = B.tbmax[g];
+            key = ((uint64_t)m << B.bits) | hp_morton_key(a.x, a.y, a.z, b.x, b.y, b.z, smin, scale, B.bits);
+            B.keys[g] = key;
         }
-        const float4 a = B.tbmin[g], b = B.tbmax[g];
-        key = ((uint64_t)m << B.bits) | hp_morton_key(a.x, a.y, a.z, b.x, b.y, b.z, smin, scale, B.bits);
-        B.keys[g] = key;
-    }
-    for (int p = 0; p < B.passes; ++p) {  // bits above the key width are zero
-        const uint32_t d = (uint32_t)((key >> (B.hshift + 8 * p)) & 0xffu);
-        int same = 0;  // the digits with the mesh index are one value in most warps
-        if (one) __match_all_sync(HP_FULL_MASK, d, &same);
-        if (same) {
-            if ((threadIdx.x & 31) == 0) atomicAdd(&sh[p * 256 + d], 32u);
-        } else if (m >= 0) {
-            atomicAdd(&sh[p * 256 + d], 1u);
+        for (int p = 0; p < B.passes; ++p) {  // bits above the key width are zero
+            const uint32_t d = (uint32_t)((key >> (B.hshift + 8 * p)) & 0xffu);
+            int same = 0;  // the digits with the mesh index are one value in most warps
+            if (one) __match_all_sync(HP_FULL_MASK, d, &same);
+            if (same) {
+                if ((threadIdx.x & 31) == 0) atomicAdd(&sh[p * 256 + d], 32u);
+            } else if (m >= 0) {
+                atomicAdd(&sh[p * 256 + d], 1u);
+            }
         }
     }
     __syncthreads();
@@ -570,7 +575,9 @@ hp_status batch_build_seq(hp_ctx* ctx, hp_batch* b, cudaStream_t s) {
     HP_CUDA(cudaMemsetAsync(B.counters, 0, N * 4, s));
     HP_CUDA(cudaMemsetAsync(B.max_hi, 0xff, N * 4, s));
     k_b_boxes<<<grid, TB, 0, s>>>(B);
-    k_b_morton<<<grid, TB, 0, s>>>(B);
+    int occ_m = 0;
+    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_m, k_b_morton, TB, 0));
+    k_b_morton<<<std::min(grid, ctx->sm_count * std::max(1, occ_m)), TB, 0, s>>>(B);
     k_b_scale<<<hp_div_up(b->M, TB), TB, 0, s>>>(B);
     HP_CUDA(cudaGetLastError());
     hp_count_launch(4);

@@ -1,7 +1,8 @@
 // LBVH construction: triangle boxes and scene box, Morton keys, radix sort,
-// Karras hierarchy emission, one bottom-up climb that refits boxes, counts
-// subtree sizes, evaluates the SAH collapse rule and woopifies triangles, and
-// a collapse into the reference's 64-byte binary node layout.
+// one bottom-up climb that finds the radix tree, refits boxes, counts subtree
+// sizes and evaluates the SAH collapse rule, and a collapse into the reference's
+// 64-byte binary node layout. (The restructuring builders start from the same tree,
+// emitted by k_karras.)
 //
 // Reference path (src/hippie/): LBVHBuilder::build rt/bvh/LBVHBuilder.cpp:183-241
 //   setupBoxes            rt/bvh/LBVHBuilderKernels.cu:65-98
@@ -401,12 +402,22 @@ __global__ void __launch_bounds__(CB, 4) k_climb_local(climb_args A, const K* __
     if (p < n && s_mh[k] >= 0) A.max_hi[p] = s_mh[k];
 }
 
-template <typename K>
-__global__ void __launch_bounds__(TB) k_climb_frontier(climb_args A, const K* __restrict__ keys) {
+// ONE: a mesh of at most FRONT_CAP triangles, whose arrivals one CTA of FRONT_BLOCK
+// threads keeps in shared memory: a level is then one round trip to memory instead of
+// two (5,003 triangles on a B200 28 -> %F1% us).
+constexpr int FRONT_BLOCK = 1024, FRONT_CAP = 8192;
+
+template <typename K, bool ONE>
+__global__ void __launch_bounds__(ONE ? FRONT_BLOCK : TB) k_climb_frontier(climb_args A, const K* __restrict__ keys) {
     hp_after_previous();
+    __shared__ int s_words[ONE ? FRONT_CAP : 1];
     const unsigned count = *A.frontier_count;
     const int n = A.n;
-    for (unsigned e = blockIdx.x * TB + threadIdx.x; e < count; e += gridDim.x * TB) {
+    if (ONE) {
+        for (int i = threadIdx.x; i < n; i += FRONT_BLOCK) s_words[i] = 0;
+        __syncthreads();
+    }
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
         const int child0 = A.frontier[e];
         if ((unsigned)child0 >= (unsigned)(2 * n - 1)) {
             hp_report(A.err, HP_DEV_BAD_INDEX, child0);
@@ -424,8 +435,14 @@ __global__ void __launch_bounds__(TB) k_climb_frontier(climb_args A, const K* __
                 break;
             }
             int old;
-            asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;"
-                         : "=r"(old) : "l"(A.words + s), "r"((is_left ? lo : hi) + 1) : "memory");
+            if (ONE) {
+                __threadfence_block();
+                old = atomicExch(&s_words[s], (is_left ? lo : hi) + 1);
+                __threadfence_block();
+            } else {
+                asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;"
+                             : "=r"(old) : "l"(A.words + s), "r"((is_left ? lo : hi) + 1) : "memory");
+            }
             if (old == 0) break;
             const int nlo = is_left ? lo : old - 1, nhi = is_left ? old - 1 : hi;
             if (nlo < 0 || nhi >= n || nlo > s || nhi <= s) {
@@ -486,29 +503,45 @@ __global__ void __launch_bounds__(TB) k_collapse_flags(int n, const int* __restr
 // CTA, from shared memory: what hp_scan_max_excl, k_collapse_flags and hp_scan2_sum
 // write in three launches and two memsets, each of them latency at this size
 // (with k_init_build's memsets, a build of 5,003 triangles on a B200 136 -> 126 us).
-constexpr int SC_BLOCK = 1024, SC_ITEMS = 8, SC_CAP = SC_BLOCK * SC_ITEMS;
+constexpr int SC_BLOCK = 1024, SC_ITEMS = 8, SC_CAP = SC_BLOCK * SC_ITEMS, SC_SPAN = SC_CAP + SC_CAP / 8;
 
 __global__ void __launch_bounds__(SC_BLOCK, 1) k_collapse_small(
     int n, const int* __restrict__ left, const int2* __restrict__ range, const uint8_t* __restrict__ state,
     const int* __restrict__ max_hi, int* __restrict__ reach, int* __restrict__ rank_int,
     int* __restrict__ rank_leaf, int* __restrict__ totals) {
     hp_after_previous();
+    // Position p at sc_at(p): a thread's SC_ITEMS consecutive positions, as they lie,
+    // would share banks with its neighbours'.
     extern __shared__ __align__(16) unsigned char sc_raw[];
-    int* s_hi = reinterpret_cast<int*>(sc_raw);  // [SC_CAP]
-    int* s_reach = s_hi + SC_CAP;                // [SC_CAP]
-    uint8_t* s_int = reinterpret_cast<uint8_t*>(s_reach + SC_CAP);  // [SC_CAP] interior flags by split
+    int* s_hi = reinterpret_cast<int*>(sc_raw);  // maxHi words, then ranks
+    int* s_reach = s_hi + SC_SPAN;
+    int* s_int = s_reach + SC_SPAN;              // interior flags by split
     __shared__ int s_w[SC_BLOCK / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int p = tid; p < SC_CAP; p += SC_BLOCK) {
-        s_hi[p] = p < n ? __ldg(max_hi + p) : -1;
-        s_int[p] = 0;
+    auto at = [](int p) { return p + (p >> 3); };
+    // Everything a thread reads is requested at once.
+    int hi[SC_ITEMS], l[SC_ITEMS], st[SC_ITEMS];
+    int2 rg[SC_ITEMS];
+#pragma unroll
+    for (int i = 0; i < SC_ITEMS; ++i) {
+        const int p = tid + i * SC_BLOCK;
+        hi[i] = p < n ? __ldg(max_hi + p) : -1;
+        rg[i] = p < n - 1 ? __ldg(range + p) : make_int2(0, 0);
+        l[i] = p < n - 1 ? __ldg(left + p) : 0;
+        st[i] = p < n - 1 ? __ldg(state + p) : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < SC_ITEMS; ++i) {
+        const int p = tid + i * SC_BLOCK;
+        s_hi[at(p)] = hi[i];
+        s_int[at(p)] = 0;
     }
     __syncthreads();
-    // each thread owns SC_ITEMS consecutive positions
+    // exclusive max-scan; each thread owns SC_ITEMS consecutive positions
     const int base = tid * SC_ITEMS;
     int top = -1;
 #pragma unroll
-    for (int i = 0; i < SC_ITEMS; ++i) top = max(top, s_hi[base + i]);
+    for (int i = 0; i < SC_ITEMS; ++i) top = max(top, s_hi[at(base + i)]);
     int incl = top;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -522,14 +555,17 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) k_collapse_small(
     for (int w = 0; w < warp; ++w) run = max(run, s_w[w]);
 #pragma unroll
     for (int i = 0; i < SC_ITEMS; ++i) {
-        s_reach[base + i] = run;
-        run = max(run, s_hi[base + i]);
+        s_reach[at(base + i)] = run;
+        run = max(run, s_hi[at(base + i)]);
     }
     __syncthreads();
-    for (int t = tid; t < n - 1; t += SC_BLOCK) {
-        const int2 rg = __ldg(range + t);
-        const bool alive = (t == 0) || !(s_reach[rg.x] >= rg.y || s_hi[rg.x] > rg.y);
-        s_int[split_of(left, n, t)] = (alive && (t == 0 || __ldg(state + t) == 1)) ? 1 : 0;
+#pragma unroll
+    for (int i = 0; i < SC_ITEMS; ++i) {
+        const int t = tid + i * SC_BLOCK;
+        if (t < n - 1) {
+            const bool alive = (t == 0) || !(s_reach[at(rg[i].x)] >= rg[i].y || s_hi[at(rg[i].x)] > rg[i].y);
+            s_int[at(l[i] >= n - 1 ? l[i] - (n - 1) : l[i])] = (alive && (t == 0 || st[i] == 1)) ? 1 : 0;
+        }
     }
     __syncthreads();
     // both counting scans at once, 16 bits each (at most SC_CAP of either)
@@ -537,7 +573,7 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) k_collapse_small(
 #pragma unroll
     for (int i = 0; i < SC_ITEMS; ++i) {
         const int p = base + i;
-        if (p < n) sum += s_int[p] + ((s_reach[p] < p ? 1 : 0) << 16);
+        if (p < n) sum += s_int[at(p)] + ((s_reach[at(p)] < p ? 1 : 0) << 16);
     }
     incl = sum;
 #pragma unroll
@@ -549,6 +585,7 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) k_collapse_small(
     __syncthreads();
     run = incl - sum;
     int all = 0;
+#pragma unroll
     for (int w = 0; w < SC_BLOCK / 32; ++w) {
         if (w < warp) run += s_w[w];
         all += s_w[w];
@@ -560,15 +597,22 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) k_collapse_small(
 #pragma unroll
     for (int i = 0; i < SC_ITEMS; ++i) {
         const int p = base + i;
+        s_hi[at(p)] = run;  // maxHi is done with
+        if (p < n) run += s_int[at(p)] + ((s_reach[at(p)] < p ? 1 : 0) << 16);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < SC_ITEMS; ++i) {
+        const int p = tid + i * SC_BLOCK;
         if (p < n) {
-            reach[p] = s_reach[p];
-            if (p < n - 1) rank_int[p] = run & 0xffff;
-            rank_leaf[p] = run >> 16;
-            run += s_int[p] + ((s_reach[p] < p ? 1 : 0) << 16);
+            const int r = s_hi[at(p)];
+            reach[p] = s_reach[at(p)];
+            if (p < n - 1) rank_int[p] = r & 0xffff;
+            rank_leaf[p] = r >> 16;
         }
     }
 }
-constexpr size_t SC_SMEM = SC_CAP * (2 * sizeof(int) + 1);
+constexpr size_t SC_SMEM = 3 * SC_SPAN * sizeof(int);
 
 struct emit_ctx {
     int n;
@@ -874,8 +918,10 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(ctx, s, "climb_local");
-        // at most one entry per reference; small meshes need few CTAs
-        HP_CHAIN(k_climb_frontier<K>, std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s, A, skeys);
+        if (n <= FRONT_CAP)
+            HP_CHAIN((k_climb_frontier<K, true>), 1, FRONT_BLOCK, 0, s, A, skeys);
+        else
+            HP_CHAIN((k_climb_frontier<K, false>), std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s, A, skeys);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
     }

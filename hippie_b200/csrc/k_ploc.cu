@@ -9,7 +9,7 @@
 // the clusters are compacted in order. The reference runs ~5 kernels and a
 // host read-back per iteration; here
 //   * one persistent cooperative kernel runs every iteration while more than
-//     TAIL clusters remain. A tile of clusters loads the boxes of the tile and
+//     LOOP_END clusters remain. A tile of clusters loads the boxes of the tile and
 //     2r clusters on each side into shared memory and finds the nearest
 //     neighbours of its clusters and of r clusters on each side (four
 //     clusters per thread on long lists, one on shorter ones; a tile holds
@@ -18,10 +18,11 @@
 //     tile's results; it then flags the merges, takes the two prefix sums
 //     (merges, survivors) by a decoupled look-back over lower tiles, creates
 //     the new nodes and compacts the clusters. Each CTA takes its tiles in
-//     increasing order; one grid barrier ends the iteration. Every wait is
-//     bounded; a wait that gives up records an error and the kernel stops
-//     iterating;
-//   * one CTA finishes the last TAIL clusters in shared memory;
+//     increasing order; one grid barrier ends the iteration. Once a tile per CTA
+//     is enough, tiles exchange their counts instead and a cluster has several
+//     lanes (small_iteration). Every wait is bounded; a wait that gives up
+//     records an error and the kernel stops iterating;
+//   * one CTA finishes the last clusters in shared memory;
 //   * merge numbering is by cluster order (k = merges at lower positions), so
 //     the tree is deterministic; the reference takes k from warp atomics.
 // The collapse costs of computeNodeStatesAdaptive (BVHCollapserKernels.cu:58-136)

@@ -289,7 +289,7 @@ constexpr size_t onesweep_smem() {
 // eight of them, with one or two tiles of work): 5,003 30-bit keys 0.060 -> 0.029 ms
 // on a B200. 8 keys a thread is what 64 registers (1,024 threads) and the shared
 // memory of wide keys (96 KB) hold.
-constexpr int ONE_BLOCK = 1024, ONE_ITEMS = 8, ONE_CAP = ONE_BLOCK * ONE_ITEMS;
+constexpr int ONE_BLOCK = 1024, ONE_ITEMS = 8, ONE_CAP = ONE_BLOCK * ONE_ITEMS, ONE_ROW = 257;
 
 template <typename K>
 __global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__ keys_in,
@@ -299,10 +299,10 @@ __global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__
     hp_after_previous();
     constexpr int NW = ONE_BLOCK / 32;
     extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);   // [NW][256] while ranking
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);   // [NW][ONE_ROW] while ranking
     K* skeys = reinterpret_cast<K*>(smem);                // [ONE_CAP] while staging
     int32_t* svals = reinterpret_cast<int32_t*>(smem + (size_t)ONE_CAP * sizeof(K));
-    __shared__ uint32_t s_w[8];
+    __shared__ uint32_t s_w[NW];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
     // Keys are spread over as few rounds as they need, the same for every warp.
@@ -320,10 +320,10 @@ __global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__
     }
     for (int shift = 0; shift < bits; shift += 8) {
         const uint32_t dmask = bits - shift >= 8 ? 255u : (1u << (bits - shift)) - 1u;
-        for (int i = tid; i < NW * 256; i += ONE_BLOCK) cnt[i] = 0;
+        for (int i = tid; i < NW * ONE_ROW; i += ONE_BLOCK) cnt[i] = 0;
         __syncthreads();
         // rank within the warp in index order (round, then lane)
-        uint32_t* wcnt = cnt + warp * 256;
+        uint32_t* wcnt = cnt + warp * ONE_ROW;
 #pragma unroll
         for (int i = 0; i < ONE_ITEMS; ++i) {
             if (i >= rounds) break;
@@ -343,29 +343,30 @@ __global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__
             pos[i] = c + below;
         }
         __syncthreads();
-        // per digit: offsets of the warps, then of the digits (one thread per digit)
-        uint32_t run = 0, incl = 0;
-        if (tid < 256) {
-#pragma unroll 8
-            for (int w = 0; w < NW; ++w) {
-                const uint32_t c = cnt[w * 256 + tid];
-                cnt[w * 256 + tid] = run;
-                run += c;
-            }
-            incl = run;
+        // per digit: offsets of the warps, then of the digits; four threads a digit take
+        // eight warps each (rows a word longer than the digits keep them off one bank)
+        constexpr int PART = NW / 4;
+        const int dg = tid >> 2, w0 = (tid & 3) * PART;
+        uint32_t c[PART], sum = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(HP_FULL_MASK, incl, o);
-                if (lane >= o) incl += y;
-            }
-            if (lane == 31) s_w[warp] = incl;
+        for (int w = 0; w < PART; ++w) {
+            c[w] = cnt[(w0 + w) * ONE_ROW + dg];
+            sum += c[w];
         }
+        uint32_t incl = sum;  // over the lanes: the digit's earlier parts and the warp's earlier digits
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(HP_FULL_MASK, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) s_w[warp] = incl;
         __syncthreads();
-        if (tid < 256) {
-            uint32_t off = incl - run;
-            for (int w = 0; w < warp; ++w) off += s_w[w];
-#pragma unroll 8
-            for (int w = 0; w < NW; ++w) cnt[w * 256 + tid] += off;
+        const uint32_t before = lane < warp ? s_w[lane] : 0u;
+        uint32_t off = incl - sum + __reduce_add_sync(HP_FULL_MASK, before);
+#pragma unroll
+        for (int w = 0; w < PART; ++w) {
+            cnt[(w0 + w) * ONE_ROW + dg] = off;
+            off += c[w];
         }
         __syncthreads();
 #pragma unroll
@@ -399,7 +400,7 @@ __global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__
 
 template <typename K>
 constexpr size_t sort_one_smem() {
-    constexpr size_t a = (size_t)(ONE_BLOCK / 32) * 256 * 4;
+    constexpr size_t a = (size_t)(ONE_BLOCK / 32) * ONE_ROW * 4;
     constexpr size_t b = (size_t)ONE_CAP * (sizeof(K) + 4);
     return a > b ? a : b;
 }

@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(CB, 4) k_climb_local(climb_args A, const K* __
 
 // ONE: a mesh of at most FRONT_CAP triangles, whose arrivals one CTA of FRONT_BLOCK
 // threads keeps in shared memory: a level is then one round trip to memory instead of
-// two (5,003 triangles on a B200 28 -> %F1% us).
+// two (5,003 triangles on a B200 27 -> 16 us).
 constexpr int FRONT_BLOCK = 1024, FRONT_CAP = 8192;
 
 template <typename K, bool ONE>
@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(TB) k_collapse_flags(int n, const int* __restr
 // The collapse's exclusive max-scan, flags and counting scans of a small mesh in one
 // CTA, from shared memory: what hp_scan_max_excl, k_collapse_flags and hp_scan2_sum
 // write in three launches and two memsets, each of them latency at this size
-// (with k_init_build's memsets, a build of 5,003 triangles on a B200 136 -> 126 us).
+// (with k_init_build's memsets, a build of 5,003 triangles on a B200 136 -> 126 us; with its reads
+// requested at once and its positions off one bank 26 -> 15 us in the chain).
 constexpr int SC_BLOCK = 1024, SC_ITEMS = 8, SC_CAP = SC_BLOCK * SC_ITEMS, SC_SPAN = SC_CAP + SC_CAP / 8;
 
 __global__ void __launch_bounds__(SC_BLOCK, 1) k_collapse_small(

@@ -66,14 +66,10 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 //     and no postponed leaf, so that a hit is found, and shortens the ray, soon;
 //   * triangles: every lane with a postponed leaf tests one triangle, until fewer
 //     than tri_min lanes have one;
-//   * new rays: once FETCH_MIN lanes are without work.
+//   * new rays: once fetch_min lanes are without work.
 // A stack entry keeps the child's entry distance, and an entry beyond the hit
 // found since is dropped at the pop: its boxes would all be missed (a child's
 // slab values lie between its parent's, rounded or not), so only the visit goes.
-// Which of two hits on a shared edge a ray returns can depend on its warp, as before:
-// where their distances differ by less than a slab's rounding, the box of the nearer
-// one may lie behind the farther one found first. About one ray in 10^7 on meshes
-// with shared edges (none on the soups of the parity tests).
 // Measured on a B200, 16.8 M bounce rays 28.4 -> 19.8 ms, 43 M rays over 256
 // meshes 42.4 -> 27.5 ms, 1.05 M shadow rays 1.14 -> 0.95 ms, 2.07 M primary rays
 // 0.75 -> 0.56 ms, 4.2 M downward rays 2.28 -> 2.33 ms (14.3 lanes per instruction
@@ -94,7 +90,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
-    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, int node_min, int tri_min) {
+    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, int node_min, int tri_min, int fetch_min) {
     constexpr int LST = STACK - SST;
     __shared__ int2 s_stack[SST * TRACE_BLOCK];
     int2* sstack = s_stack + threadIdx.x;
@@ -133,7 +129,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
         // Finished lanes write their results and take new rays (one atomic per warp).
         const bool idle = node == SENTINEL && leaf >= 0 && tri >= tri_end;
         const unsigned idle_mask = __ballot_sync(HP_FULL_MASK, idle);
-        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= FETCH_MIN)) {
+        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= fetch_min)) {
             if (idle && ray >= 0) {
                 if (r.hit < 0) {
                     reinterpret_cast<int2*>(results)[2 * ray] = make_int2(-1, __float_as_int(r.hit_t));
@@ -334,8 +330,20 @@ int trace_grid(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
 bool few_rays(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
     return num_rays < 2 * (int64_t)ctx->sm_count * std::max(per_sm, 1) * TRACE_BLOCK;
 }
-int node_min(const hp_ctx* ctx, int per_sm, int64_t num_rays) { return few_rays(ctx, per_sm, num_rays) ? 1 : NODE_MIN; }
-int tri_min(const hp_ctx* ctx, int per_sm, int64_t num_rays) { return few_rays(ctx, per_sm, num_rays) ? 1 : TRI_MIN; }
+// Triangles that share edges can be hit at distances that differ by less than a slab's
+// rounding; which of the two a ray returns then depends on whether its first leaf was
+// tested before the other's box. Their rays keep the order they have always had (every
+// lane goes on until it or all lanes hold a leaf), so that hits stay what they were: on 70
+// frames of 2.07 M primary rays over a terrain one or two rays in all differ from the
+// earlier tracer, as many as it differed from itself between runs, against ten with the
+// shorter turns (0.70 and 0.56 ms a frame, 0.75 before; 4.2 M downward rays 2.20 ms).
+int node_min(const hp_ctx* ctx, int per_sm, int64_t num_rays, bool shared) {
+    return shared || few_rays(ctx, per_sm, num_rays) ? 1 : NODE_MIN;
+}
+int tri_min(const hp_ctx* ctx, int per_sm, int64_t num_rays, bool shared) {
+    return shared || few_rays(ctx, per_sm, num_rays) ? 1 : TRI_MIN;
+}
+int fetch_min(bool shared) { return shared ? 20 : FETCH_MIN; }
 
 template <bool A, bool S, int SST>
 hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const float* rays,
@@ -348,7 +356,7 @@ hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const floa
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const float4*>(b->nodes), b->woop, b->tri_idx,
         max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order,
-        node_min(ctx, per_sm, num_rays), tri_min(ctx, per_sm, num_rays));
+        node_min(ctx, per_sm, num_rays, b->shared), tri_min(ctx, per_sm, num_rays, b->shared), fetch_min(b->shared));
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

@@ -293,8 +293,8 @@ hp_status launch_wide_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const
     const int64_t rays_per_cta = TB1;
     const int64_t grid = std::max<int64_t>(
         1, std::min<int64_t>((int64_t)ctx->sm_count * k, (num_rays + rays_per_cta - 1) / rays_per_cta));
-    // (k_trace_impl.cuh says why launches of few rays take every turn)
-    const bool few = num_rays < 2 * (int64_t)ctx->sm_count * std::max(per_sm, 1) * TB1;
+    // (k_trace_impl.cuh says why launches of few rays, or on shared edges, take every turn)
+    const bool few = b->shared || num_rays < 2 * (int64_t)ctx->sm_count * std::max(per_sm, 1) * TB1;
     const int max_nodes = (int)std::max<int64_t>(2 * b->capacity - 1, 3);
     k_trace_wide1<N, A, S><<<(unsigned)grid, TB1, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),

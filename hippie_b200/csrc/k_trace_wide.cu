@@ -14,9 +14,8 @@
 //     hit children and made every leaf's few triangles a shuffle reduction;
 //   * a warp takes turns at nodes, triangles and new rays, all 32 lanes together,
 //     as in the binary tracer (k_trace_impl.cuh says why); the first leaf a lane
-//     reaches is postponed; a stack entry keeps the child's entry distance and is
-//     dropped at the pop when a closer hit has been found since. On a B200, 1 M
-//     bounce rays in 0.5 M triangles (Quad) 1.46 -> 1.08 ms;
+//     reaches is postponed. On a B200, 1 M bounce rays in 0.5 M triangles (Quad)
+//     1.46 -> 1.07 ms;
 //   * persistent warps take rays with one atomic per warp; the per-ray stack
 //     keeps its first entries in shared memory and the rest in local memory, and
 //     an overflow is reported as a device error instead of overrunning;
@@ -72,12 +71,12 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
                                                    unsigned long long* ray_counter, int* err,
                                                    const int32_t* __restrict__ order, int node_min, int tri_min) {
     constexpr int STACK = wide1_cfg<N>::STACK, LST = STACK - SST1;
-    __shared__ int2 s_stack[SST1 * TB1];
-    int2* sstack = s_stack + threadIdx.x;
-    // Entries (child, entry distance) past the shared part. Left uninitialised: sp
+    __shared__ int s_stack[SST1 * TB1];
+    int* sstack = s_stack + threadIdx.x;
+    // Entries past the shared part. Left uninitialised: sp
     // counts the pushes that were stored (an overflowing push is dropped and
     // reported), so a pop reads only entries a push wrote.
-    int2 lstack[LST];
+    int lstack[LST];
     const int lane = threadIdx.x & 31;
 
     float ox = 0, oy = 0, oz = 0, tmin = 0, dx = 0, dy = 0, dz = 0;
@@ -90,20 +89,16 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
     int tri = 0, tri_end = 0;  // triangles of the postponed leaf still to test
     bool exhausted = false;    // warp-uniform: the counter has run past the rays
     auto pop = [&]() {
-        node = SENT1;
-        while (sp > 0) {
+        if (sp == 0) {
+            node = SENT1;
+        } else {
             --sp;
-            const int2 e = sp < SST1 ? sstack[sp * TB1] : lstack[sp - SST1];
-            if (STATS || !(__int_as_float(e.y) > hit_t)) {
-                node = e.x;
-                break;
-            }
+            node = sp < SST1 ? sstack[sp * TB1] : lstack[sp - SST1];
         }
     };
-    auto push = [&](int v, uint32_t key) {
-        const int2 e = make_int2(v, __float_as_int(hp_ord2f(key)));
-        if (sp < SST1) sstack[sp * TB1] = e;
-        else if (sp < STACK) lstack[sp - SST1] = e;
+    auto push = [&](int v) {
+        if (sp < SST1) sstack[sp * TB1] = v;
+        else if (sp < STACK) lstack[sp - SST1] = v;
         else { hp_report(err, HP_DEV_STACK_OVERFLOW, (int)ray); --sp; }
         ++sp;
     };
@@ -207,7 +202,7 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
                     } else {
 #pragma unroll
                         for (int i = N - 1; i >= 1; --i)
-                            if (key[i] != 0xFFFFFFFFu) push(ref[i], key[i]);
+                            if (key[i] != 0xFFFFFFFFu) push(ref[i]);
                         node = ref[0];
                     }
                     if (node < 0 && leaf >= 0 && tri >= tri_end) {  // the first leaf is postponed

@@ -122,3 +122,59 @@ def test_axis_aligned_rays(ctx):
     np.testing.assert_array_equal(got[:, :2], exp[:, :2])
     h = exp[:, 0] >= 0
     np.testing.assert_array_equal(got[h], exp[h])
+
+
+@pytest.mark.parametrize("slope", [1.0, 1e-3, 1e-5])
+@pytest.mark.parametrize("arith,layout", [("ieee", 2), ("reference", 2), ("ieee", 4), ("ieee", 8)])
+def test_leaves_of_one_plane(arith, layout, slope):
+    """Overlapping triangles of one axis-aligned plane, in leaves whose boxes are all
+    looked at before any hit is known (children of the root; in the binary tree also of
+    the root's first child, which a ray visits first). A leaf's triangles are tested
+    whatever its flat box's rounded slabs say of a hit found since, so a ray returns
+    the nearest of them, of equal ones the lowest id, with and without statistics: what
+    the triangles return one by one. `slope` scales the rays' components along the
+    plane, down to rays nearly along the axis."""
+    c = hp.Context(0)
+    c.set_arithmetic(arith)
+    rng = np.random.default_rng(layout)
+    n, m = max(layout, 3), 1 << 14
+    ang = rng.uniform(0, 2 * np.pi, (n, 1)) + np.array([0, 2.1, 4.2]) + rng.uniform(-0.3, 0.3, (n, 3))
+    rad = rng.uniform(0.3, 0.9, (n, 3))
+    rad[:] = rad.mean(1, keepdims=True)
+    at = np.full((n, 1), 0.45)
+    at[-1] = 0.65  # the last Morton code
+    v = np.stack([at + rad * np.cos(ang), at + rad * np.sin(ang), np.full_like(rad, 0.3)], -1)
+    v = v.reshape(-1, 3).astype(np.float32)
+    t = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    rays = np.zeros((m, 8), np.float32)
+    rays[:, :2] = rng.uniform(0.3, 0.7, (m, 2))
+    rays[:, 2] = rng.uniform(0.5, 1.5, m)
+    rays[:, 4:6] = slope * rng.uniform(-0.3, 0.3, (m, 2))
+    rays[:, 6] = 0.3 - rays[:, 2]
+    rays[:, 7] = 10
+    R = dev(rays)
+    p = hp.BuildParams(method="lbvh", morton_bits=60, layout=layout, adaptive_leaf=0, max_leaf_size=1)
+
+    def hits(ctx, bvh, **kw):
+        out = torch.zeros((m, 4), dtype=torch.int32, device="cuda")
+        ctx.trace(bvh, R, results=out, **kw)
+        ctx.check()
+        return out.cpu().numpy()
+
+    bvh = c.build(dev(v), dev(t), p)
+    bvh.sync()
+    assert bvh.c.num_interior == (2 if layout == 2 else 1)
+    if layout == 2:
+        assert bvh.download()[0][0, 12] == 1 and bvh.download()[0][0, 13] < 0
+    got = hits(c, bvh)
+    want = np.zeros((m, 4), np.int32)
+    want[:, 0], want[:, 1] = -1, rays[:, 7].view(np.int32)
+    for i in range(n):  # in the order of the ids: a later one has to be nearer
+        one = hits(c, c.build(dev(v[3 * i:3 * i + 3]), dev(t[:1]), p))
+        nearer = (one[:, 0] >= 0) & (one[:, 1].view(np.float32) < want[:, 1].view(np.float32))
+        want[nearer] = one[nearer]
+        want[nearer, 0] = i
+    assert (want[:, 0] >= 0).mean() > 0.5 and len(np.unique(want[:, 0])) > 1
+    np.testing.assert_array_equal(got, want)
+    np.testing.assert_array_equal(hits(c, bvh, stats=torch.zeros((m, 2), dtype=torch.int32, device="cuda")), want)
+    c.close()

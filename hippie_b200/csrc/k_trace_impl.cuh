@@ -367,9 +367,6 @@ hp_status launch_st(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const flo
     switch (ctx->tune.trace_stack) {
         case 8: return launch_t<A, S, 8>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
         case 32: return launch_t<A, S, 32>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
-        // the default choice of 16: two entries fewer leave the L1 more of the SM's memory
-        // (bounce rays 19.86 -> 19.58 ms; at 20 entries, with less than 64 KB left, 35.8)
-        default: return launch_t<A, S, 14>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+        default: return launch_t<A, S, 16>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
     }
 }
-

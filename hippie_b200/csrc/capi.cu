@@ -344,7 +344,6 @@ hp_status hp_build(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_b
     HP_TRY(bvh_alloc(out, n, layout));
     hp_bvh_impl* b = reinterpret_cast<hp_bvh_impl*>(out->impl);
     b->layout = layout;
-    b->shared = m->num_vertices < 3 * n;
     out->layout = layout;
     out->node_bytes = 32 * layout;
     out->num_refs = n;
@@ -374,7 +373,6 @@ hp_status hp_bvh_reserve(hp_ctx* ctx, hp_bvh* out, int64_t num_refs, int32_t lay
     HP_TRY(bvh_alloc(out, num_refs, layout));
     hp_bvh_impl* b = reinterpret_cast<hp_bvh_impl*>(out->impl);
     b->layout = layout;
-    b->shared = true;  // of a mesh that is not known here
     out->layout = layout;
     out->node_bytes = 32 * layout;
     out->num_refs = num_refs;

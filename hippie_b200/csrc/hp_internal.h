@@ -43,7 +43,6 @@ struct hp_bvh_impl {
     size_t node_capacity = 0;      // bytes of the node buffer
     int layout = 2;                // children per node: 2, 4 or 8
     bool view = false;             // storage owned by a batch (hp_batch_bvh)
-    bool shared = true;            // the mesh's triangles may share edges (false: every one has vertices of its own)
 };
 
 // ---- context: scratch arena, error words, phase events ------------------------
@@ -311,7 +310,6 @@ struct hp_batch_trace_args {
     const hp_batch_seg* segs;
     const int64_t* ray_off;   // [num_segs + 1]
     int num_segs;
-    bool shared;              // any mesh whose triangles may share edges
 };
 hp_status hp_trace_batch_launch(hp_ctx* ctx, const hp_batch_trace_args& t, uint32_t flags, cudaStream_t stream);
 

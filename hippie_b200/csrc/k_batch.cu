@@ -484,7 +484,6 @@ struct hp_batch {
     int32_t* tri_idx = nullptr;
     std::vector<hp_bvh_impl> views;
     size_t scratch = 0;
-    bool shared = false;                 // any mesh whose triangles may share edges
     cudaGraphExec_t exec = nullptr;
     const float* g_rays = nullptr;
     int32_t* g_results = nullptr;
@@ -614,7 +613,6 @@ hp_status batch_trace_seq(hp_ctx* ctx, hp_batch* b, const float* rays, int32_t* 
     t.segs = b->d_seg;
     t.ray_off = b->d_ray_off;
     t.num_segs = b->M;
-    t.shared = b->shared;
     HP_TRY(hp_trace_batch_launch(ctx, t, flags, s));
     hp_mark(ctx, s, "batch_trace");
     return HP_OK;
@@ -766,8 +764,6 @@ hp_status hp_batch_create(hp_ctx* ctx, const hp_mesh* meshes, int32_t num_meshes
         v.info = b->d_info + m;
         v.capacity = b->segs[m].n;
         v.view = true;
-        v.shared = b->segs[m].nv < 3 * (int64_t)b->segs[m].n;
-        b->shared = b->shared || v.shared;
     }
     // reserve the scratch now (for either sort CTA size): nothing may allocate
     // inside a graph capture

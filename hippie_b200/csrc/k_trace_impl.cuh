@@ -59,40 +59,56 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 // cycles of an SM's L1 when it comes from L2 and 1.4 when it hits, and a bounce
 // ray of the 4.2 M-triangle scene takes 79 nodes, 6 leaves and 14 triangles. So a
 // warp stays in one piece and takes three kinds of turns, all 32 lanes together,
-// decided by ballots (node_min and tri_min are NODE_MIN and TRI_MIN, or 1 for few rays):
+// decided by ballots:
 //   * nodes: every lane at an interior node does one. The first leaf that a lane
 //     meets is postponed and the lane goes on from its stack; at a second one it
-//     waits. The turn ends when fewer than node_min lanes have an interior node
-//     and no postponed leaf, so that a hit is found, and shortens the ray, soon;
+//     waits. The turn ends when fewer than NODE lanes have an interior node and no
+//     postponed leaf, so that a hit is found, and shortens the ray, soon;
 //   * triangles: every lane with a postponed leaf tests one triangle, until fewer
-//     than tri_min lanes have one;
-//   * new rays: once fetch_min lanes are without work.
+//     than TRI lanes have one;
+//   * new rays: once FETCH lanes are without work.
 // A stack entry is the child alone. With its entry distance beside it, entries beyond
 // the hit found since could be dropped at the pop; that saved no time (bounce rays 19.6
 // ms with it, 19.5 without), and for a leaf it is wrong: a leaf's triangles are tested
 // whatever its box, whose rounded slabs may lie beyond a nearer or equal hit in it.
-// Measured on a B200, 16.8 M bounce rays 28.4 -> 19.8 ms, 43 M rays over 256
-// meshes 42.4 -> 27.5 ms, 1.05 M shadow rays 1.14 -> 0.95 ms, 2.07 M primary rays
-// 0.75 -> 0.56 ms, 4.2 M downward rays 2.28 -> 2.33 ms (14.3 lanes per instruction
-// and the L1 at 80 %). NODE_MIN / FETCH_MIN from 4 to 28 and TRI_MIN from 1 to 20
-// were swept: 16 / 8 / 12 is 1 % faster on bounce rays and 20 % slower on downward
-// ones, whose leaves it tests too late; higher ones lose on bounce rays.
-// Three CTAs more or fewer than 10 per SM, an 8-entry shared stack, packed FP32
-// for the slabs and 32-byte loads of two Woop rows were slower or no faster.
-constexpr int NODE_MIN = 16, TRI_MIN = 6, FETCH_MIN = 10;
-// CTAs per SM: 48 registers for one BVH, 61 with the mesh's bases in the lane.
-constexpr int TRACE_CTAS = 10, TRACE_CTAS_BATCH = 8;
+//
+// NODE decides more than time. Of two hits nearer to each other than a slab's rounding
+// (on the edge that two triangles share) a ray misses the nearer one if the other was
+// tested before the nearer one's boxes were, and short node turns test sooner. Against
+// a tracer that gives boxes a slack, rays that missed the nearer hit in 360 frames of
+// 2.07 M primary rays and in 360 times 4.2 M sphere rays on terrains: every lane in
+// loops of its own, as in the reference, 122 and 217; NODE 1: 122 and 223; 2: 132, 228;
+// 3: 126, 232; 4: 128, 235; 16: 151, 280. Up to 4 is as good as it was. A visibility
+// ray has no nearest hit to miss.
+//
+// Measured on a B200 (every lane in loops of its own / NODE 1 / 3 / 16): 16.8 M bounce
+// rays 28.4 / 22.9 / 20.0 / 18.4 ms, 43 M rays over 256 meshes 42.4 / 32.0 / 28.3 / 27.3,
+// 4 M sorted rays 3.86 / 3.23 / 3.01 / 3.00, 2.07 M primary rays 0.77 / 0.75 / 0.59 / 0.57,
+// 4.2 M downward rays 2.28 / 2.17 / 2.21 / 2.40, 4.2 M bounce rays on a terrain 3.12 / 2.66 /
+// 2.39 / 2.24, 4.2 M rays in 33.5 M triangles 22.2 / 22.3 / 22.7 / 24.3. FETCH: at 12 bounce
+// rays 19.4 and downward ones 2.35, at 20 20.8 and 2.18. TRI 1 to 6 differ by 2 % either way.
+// Packed FP32 for the slabs and 32-byte loads of two Woop rows were slower or no faster.
+template <bool ANY_HIT>
+struct turns {
+    static constexpr int NODE = ANY_HIT ? 16 : 3, TRI = ANY_HIT ? 6 : 4, FETCH = 16;
+};
+// CTAs per SM. Closest hits: 12 (40 registers, 8 bytes of spills read back) instead of 10
+// shorten bounce rays by 8 % and downward ones by 3 %, and cost rays in 33.5 M triangles 3 %.
+// Any hit: 1.05 M shadow rays 0.91 ms at 8 and 9, 0.97 at 10, 1.02 at 12. Batch (the
+// mesh's bases in the lane, 55 registers): 27.3 ms at 8, 28.9 at 9, 30.0 at 10.
+constexpr int trace_ctas(bool any_hit, bool batch) { return batch ? 8 : any_hit ? 9 : 12; }
 
 // BATCH: rays of many meshes in one launch; ray g belongs to the segment whose
 // ray range holds it, and the lane traverses that mesh's BVH.
 template <bool ANY_HIT, bool STATS, bool BATCH, int SST>
-__global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_CTAS) k_trace(
+__global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_trace(
     const float4* __restrict__ rays, int64_t num_rays, int4* __restrict__ results,
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
-    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, int node_min, int tri_min, int fetch_min) {
+    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order) {
     constexpr int LST = STACK - SST;
+    using TURN = turns<ANY_HIT>;
     __shared__ int s_stack[SST * TRACE_BLOCK];
     int* sstack = s_stack + threadIdx.x;
     int lstack[LST];
@@ -126,7 +142,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
         // Finished lanes write their results and take new rays (one atomic per warp).
         const bool idle = node == SENTINEL && leaf >= 0 && tri >= tri_end;
         const unsigned idle_mask = __ballot_sync(HP_FULL_MASK, idle);
-        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= fetch_min)) {
+        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= TURN::FETCH)) {
             if (idle && ray >= 0) {
                 if (r.hit < 0) {
                     reinterpret_cast<int2*>(results)[2 * ray] = make_int2(-1, __float_as_int(r.hit_t));
@@ -239,7 +255,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
             }
             go = (unsigned)node < (unsigned)SENTINEL;
             mask = __ballot_sync(HP_FULL_MASK, go && leaf >= 0 && tri >= tri_end);
-            if (__popc(mask) < node_min) break;
+            if (__popc(mask) < TURN::NODE) break;
         }
 
         // Leaves: one triangle per lane and round.
@@ -307,7 +323,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, BATCH ? TRACE_CTAS_BATCH : TRACE_
             }
             pend = node < 0 || leaf < 0 || tri < tri_end;
             mask = __ballot_sync(HP_FULL_MASK, pend);
-            if (__popc(mask) < tri_min) break;
+            if (__popc(mask) < TURN::TRI) break;
         }
     }
 }
@@ -320,28 +336,6 @@ int trace_grid(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
     return (int)std::max<int64_t>(grid, 1);
 }
 
-// A launch that has no two rays for a lane lasts as long as its slowest warps: their
-// lanes take every turn they can, instead of waiting for a fuller one (137 K primary
-// rays in 1.7 M triangles on a B200 299 -> 268 us, 205 K sorted ones on a terrain 240 ->
-// 220 us; as a rule for 4 or 8 rays a lane 1 M shadow rays lose 6 %).
-bool few_rays(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
-    return num_rays < 2 * (int64_t)ctx->sm_count * std::max(per_sm, 1) * TRACE_BLOCK;
-}
-// Triangles that share edges can be hit at distances that differ by less than a slab's
-// rounding; which of the two a ray returns then depends on whether its first leaf was
-// tested before the other's box. Their rays keep the order they have always had (every
-// lane goes on until it or all lanes hold a leaf), so that hits stay what they were: on 70
-// frames of 2.07 M primary rays over a terrain one or two rays in all differ from the
-// earlier tracer, as many as it differed from itself between runs, against ten with the
-// shorter turns (0.70 and 0.56 ms a frame, 0.75 before; 4.2 M downward rays 2.20 ms).
-int node_min(const hp_ctx* ctx, int per_sm, int64_t num_rays, bool shared) {
-    return shared || few_rays(ctx, per_sm, num_rays) ? 1 : NODE_MIN;
-}
-int tri_min(const hp_ctx* ctx, int per_sm, int64_t num_rays, bool shared) {
-    return shared || few_rays(ctx, per_sm, num_rays) ? 1 : TRI_MIN;
-}
-int fetch_min(bool shared) { return shared ? 20 : FETCH_MIN; }
-
 template <bool A, bool S, int SST>
 hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const float* rays,
                    int64_t num_rays, int32_t* results, int32_t* stats, unsigned long long* counter,
@@ -352,8 +346,7 @@ hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const floa
     k_trace<A, S, false, SST><<<trace_grid(ctx, per_sm, num_rays), TRACE_BLOCK, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const float4*>(b->nodes), b->woop, b->tri_idx,
-        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order,
-        node_min(ctx, per_sm, num_rays, b->shared), tri_min(ctx, per_sm, num_rays, b->shared), fetch_min(b->shared));
+        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

@@ -41,22 +41,24 @@ __device__ __forceinline__ float safe_rcp(float d) {
 // loads), tests its N child boxes itself, continues with the nearest hit
 // child and pushes the other hits farthest first, so the nearest of them is
 // popped next. Rays are taken by persistent warps as in the binary tracer
-// (once turns1<N>::FETCH lanes are without work); each lane's stack keeps
+// (once turns1::FETCH lanes are without work); each lane's stack keeps
 // SST entries in shared memory (one column per thread) and the rest in local
 // memory. Leaves are tested by the lane, with the binary tracer's Woop
 // arithmetic and tie rule, so the hits equal the binary layout's.
 constexpr int TB1 = 128;
 constexpr int SST1 = 16;
-// Turns (see k_trace_impl.cuh) and CTAs per SM, swept on a B200 with 2 M bounce rays
-// in 1 M triangles, shadow rays and primary rays: Quad 2.85 -> 2.02 ms, 1.16 ->
-// 0.96 ms and 0.69 -> 0.54 ms, Oct 3.56 -> 2.52 ms, 1.32 -> 1.17 ms and 0.78 -> 0.61
-// ms. Quad at 10 CTAs (48 registers, spills) is 8 % slower than at 8, Oct at 6 or 5
-// CTAs 8 or 16 % slower on bounce rays than at 8. An Oct node is eight boxes and a
-// sort whatever the lanes at it, so its turns last longer: with Quad's, primary rays
-// on small terrains were up to 3 % slower than before, bounce rays 2 % faster.
+// Turns (k_trace_impl.cuh says what they are and what NODE decides: here too rays miss the
+// nearer of two near-tied hits as often at 3 or 4 as in the tracer before, 6 % more often
+// at 6 and 25 % at 12) and CTAs per SM. On a B200, the tracer before / NODE 1 / 3 / 12, 2 M bounce
+// rays in 1 M triangles, primary rays on a terrain and 4.2 M bounce rays on another: Quad 2.99 /
+// 2.55 / 2.24 / 2.15 ms, 0.65 / 0.58 / 0.54 / 0.53 and 3.11 / 2.65 / 2.39 / 2.31; Oct 3.71 / 3.37 /
+// 2.91 / 2.78, 0.74 / 0.75 / 0.67 / 0.62 and 3.95 / 3.51 / 3.14 / 3.05. FETCH 12: 1 to 2 % slower.
+// Visibility rays, where NODE is free: Quad 1.16 -> 0.96 ms, Oct 1.31 -> 1.15 for 1 M of them.
+// CTAs at 9 (56 registers): Quad equal, Oct 12 % slower.
 constexpr int CTAS1 = 8;
-template <int N> struct turns1 {
-    static constexpr int FETCH = N == 4 ? 12 : 8, NODE = N == 4 ? 12 : 4, TRI = N == 4 ? 8 : 4;
+template <bool ANY_HIT>
+struct turns1 {
+    static constexpr int NODE = ANY_HIT ? 12 : 3, TRI = 4, FETCH = ANY_HIT ? 12 : 8;
 };
 constexpr int SENT1 = 0x76543210;
 template <int N> struct wide1_cfg;
@@ -69,7 +71,8 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
                                                    const int4* __restrict__ nodes, const float4* __restrict__ woop,
                                                    const int32_t* __restrict__ tri_idx, int max_nodes, int num_refs,
                                                    unsigned long long* ray_counter, int* err,
-                                                   const int32_t* __restrict__ order, int node_min, int tri_min) {
+                                                   const int32_t* __restrict__ order) {
+    using TURN = turns1<ANY_HIT>;
     constexpr int STACK = wide1_cfg<N>::STACK, LST = STACK - SST1;
     __shared__ int s_stack[SST1 * TB1];
     int* sstack = s_stack + threadIdx.x;
@@ -107,7 +110,7 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
         // Finished lanes write their results and take new rays (one atomic per warp).
         const bool idle = node == SENT1 && leaf >= 0 && tri >= tri_end;
         const unsigned idle_mask = __ballot_sync(HP_FULL_MASK, idle);
-        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= turns1<N>::FETCH)) {
+        if (idle_mask == HP_FULL_MASK || (!exhausted && __popc(idle_mask) >= TURN::FETCH)) {
             if (idle && ray >= 0) {
                 if (hit < 0) {
                     reinterpret_cast<int2*>(results)[2 * ray] = make_int2(-1, __float_as_int(hit_t));
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
             }
             go = (unsigned)node < (unsigned)SENT1;
             mask = __ballot_sync(HP_FULL_MASK, go && leaf >= 0 && tri >= tri_end);
-            if (__popc(mask) < node_min) break;
+            if (__popc(mask) < TURN::NODE) break;
         }
 
         // Leaves: one triangle per lane and round.
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
             }
             pend = node < 0 || leaf < 0 || tri < tri_end;
             mask = __ballot_sync(HP_FULL_MASK, pend);
-            if (__popc(mask) < tri_min) break;
+            if (__popc(mask) < TURN::TRI) break;
         }
     }
 }
@@ -288,13 +291,11 @@ hp_status launch_wide_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const
     const int64_t rays_per_cta = TB1;
     const int64_t grid = std::max<int64_t>(
         1, std::min<int64_t>((int64_t)ctx->sm_count * k, (num_rays + rays_per_cta - 1) / rays_per_cta));
-    // (k_trace_impl.cuh says why launches of few rays, or on shared edges, take every turn)
-    const bool few = b->shared || num_rays < 2 * (int64_t)ctx->sm_count * std::max(per_sm, 1) * TB1;
     const int max_nodes = (int)std::max<int64_t>(2 * b->capacity - 1, 3);
     k_trace_wide1<N, A, S><<<(unsigned)grid, TB1, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const int4*>(b->nodes), b->woop, b->tri_idx, max_nodes,
-        (int)n_refs, counter, ctx->d_status, order, few ? 1 : turns1<N>::NODE, few ? 1 : turns1<N>::TRI);
+        (int)n_refs, counter, ctx->d_status, order);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

@@ -291,91 +291,93 @@ constexpr size_t onesweep_smem() {
 // memory of wide keys (96 KB) hold.
 constexpr int ONE_BLOCK = 1024, ONE_ITEMS = 8, ONE_CAP = ONE_BLOCK * ONE_ITEMS, ONE_ROW = 257;
 
+// A CTA's keys: warp w's are those from 32 * rounds * w on, `rounds` rows of 32 (key[i] of a
+// lane is that of row i), n in all, spread over as few rounds as they need.
+struct one_shape {
+    int n, rounds, base;  // base: the warp's first key
+    __device__ explicit one_shape(int keys)
+        : n(keys), rounds((keys + ONE_BLOCK - 1) / ONE_BLOCK),
+          base((int)(threadIdx.x >> 5) * 32 * ((keys + ONE_BLOCK - 1) / ONE_BLOCK)) {}
+    __device__ int at(int i) const { return base + i * 32 + (int)(threadIdx.x & 31); }
+    __device__ bool has(int i) const { return i < rounds && at(i) < n; }
+};
+
+// Stable ranks of a CTA's keys by one digit: pos[i] is key[i]'s position when sorted by it,
+// cnt[d] (its first row) the first position of digit d. cnt [NW][ONE_ROW] and s_w [NW] are
+// shared scratch, free to use on entry; the caller synchronises before it changes them.
 template <typename K>
-__global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__ keys_in,
-                                                           const int32_t* __restrict__ vals_in,
-                                                           K* __restrict__ keys_out, int32_t* __restrict__ vals_out,
-                                                           int n, int bits) {
-    hp_after_previous();
+__device__ __forceinline__ void one_rank(const K (&key)[ONE_ITEMS], const one_shape& sh, int shift, uint32_t dmask,
+                                         uint32_t* cnt, uint32_t* s_w, uint32_t (&pos)[ONE_ITEMS]) {
     constexpr int NW = ONE_BLOCK / 32;
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);   // [NW][ONE_ROW] while ranking
-    K* skeys = reinterpret_cast<K*>(smem);                // [ONE_CAP] while staging
-    int32_t* svals = reinterpret_cast<int32_t*>(smem + (size_t)ONE_CAP * sizeof(K));
-    __shared__ uint32_t s_w[NW];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    // Keys are spread over as few rounds as they need, the same for every warp.
-    const int rounds = (n + ONE_BLOCK - 1) / ONE_BLOCK;
-    const int wbase = warp * 32 * rounds;
-    K key[ONE_ITEMS];
-    int32_t val[ONE_ITEMS];
-    uint32_t pos[ONE_ITEMS];
+    for (int i = tid; i < NW * ONE_ROW; i += ONE_BLOCK) cnt[i] = 0;
+    __syncthreads();
+    // rank within the warp in index order (round, then lane)
+    uint32_t* wcnt = cnt + warp * ONE_ROW;
 #pragma unroll
     for (int i = 0; i < ONE_ITEMS; ++i) {
-        const int idx = wbase + i * 32 + lane;
-        const bool valid = i < rounds && idx < n;
-        key[i] = valid ? keys_in[idx] : K(0);
-        val[i] = valid ? (vals_in ? vals_in[idx] : idx) : 0;
+        if (i >= sh.rounds) break;
+        const bool valid = sh.at(i) < sh.n;
+        const uint32_t d = valid ? digit_of(key[i], shift, dmask) : 0u;
+        uint32_t peers = __ballot_sync(HP_FULL_MASK, valid);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const uint32_t bal = __ballot_sync(HP_FULL_MASK, (d >> b) & 1u);
+            peers &= ((d >> b) & 1u) ? bal : ~bal;
+        }
+        const uint32_t below = __popc(peers & lt_mask);
+        const uint32_t c = valid ? wcnt[d] : 0u;
+        __syncwarp();
+        if (valid && below == 0) wcnt[d] = c + __popc(peers);
+        __syncwarp();
+        pos[i] = c + below;
     }
+    __syncthreads();
+    // per digit: offsets of the warps, then of the digits; four threads a digit take
+    // eight warps each (rows a word longer than the digits keep them off one bank)
+    constexpr int PART = NW / 4;
+    const int dg = tid >> 2, w0 = (tid & 3) * PART;
+    uint32_t c[PART], sum = 0;
+#pragma unroll
+    for (int w = 0; w < PART; ++w) {
+        c[w] = cnt[(w0 + w) * ONE_ROW + dg];
+        sum += c[w];
+    }
+    uint32_t incl = sum;  // over the lanes: the digit's earlier parts and the warp's earlier digits
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(HP_FULL_MASK, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    const uint32_t before = lane < warp ? s_w[lane] : 0u;
+    uint32_t off = incl - sum + __reduce_add_sync(HP_FULL_MASK, before);
+#pragma unroll
+    for (int w = 0; w < PART; ++w) {
+        cnt[(w0 + w) * ONE_ROW + dg] = off;
+        off += c[w];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ONE_ITEMS; ++i)
+        if (i < sh.rounds) pos[i] += wcnt[digit_of(key[i], shift, dmask)];
+}
+
+// A CTA's keys and values sorted by their low `bits` bits; the result is in skeys [0, n) and
+// svals [0, n), which share their memory with cnt.
+template <typename K>
+__device__ __forceinline__ void one_sort(K (&key)[ONE_ITEMS], int32_t (&val)[ONE_ITEMS], const one_shape& sh, int bits,
+                                         uint32_t* cnt, uint32_t* s_w, K* skeys, int32_t* svals) {
+    uint32_t pos[ONE_ITEMS];
     for (int shift = 0; shift < bits; shift += 8) {
         const uint32_t dmask = bits - shift >= 8 ? 255u : (1u << (bits - shift)) - 1u;
-        for (int i = tid; i < NW * ONE_ROW; i += ONE_BLOCK) cnt[i] = 0;
-        __syncthreads();
-        // rank within the warp in index order (round, then lane)
-        uint32_t* wcnt = cnt + warp * ONE_ROW;
-#pragma unroll
-        for (int i = 0; i < ONE_ITEMS; ++i) {
-            if (i >= rounds) break;
-            const bool valid = wbase + i * 32 + lane < n;
-            const uint32_t d = valid ? digit_of(key[i], shift, dmask) : 0u;
-            uint32_t peers = __ballot_sync(HP_FULL_MASK, valid);
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                const uint32_t bal = __ballot_sync(HP_FULL_MASK, (d >> b) & 1u);
-                peers &= ((d >> b) & 1u) ? bal : ~bal;
-            }
-            const uint32_t below = __popc(peers & lt_mask);
-            const uint32_t c = valid ? wcnt[d] : 0u;
-            __syncwarp();
-            if (valid && below == 0) wcnt[d] = c + __popc(peers);
-            __syncwarp();
-            pos[i] = c + below;
-        }
-        __syncthreads();
-        // per digit: offsets of the warps, then of the digits; four threads a digit take
-        // eight warps each (rows a word longer than the digits keep them off one bank)
-        constexpr int PART = NW / 4;
-        const int dg = tid >> 2, w0 = (tid & 3) * PART;
-        uint32_t c[PART], sum = 0;
-#pragma unroll
-        for (int w = 0; w < PART; ++w) {
-            c[w] = cnt[(w0 + w) * ONE_ROW + dg];
-            sum += c[w];
-        }
-        uint32_t incl = sum;  // over the lanes: the digit's earlier parts and the warp's earlier digits
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(HP_FULL_MASK, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) s_w[warp] = incl;
-        __syncthreads();
-        const uint32_t before = lane < warp ? s_w[lane] : 0u;
-        uint32_t off = incl - sum + __reduce_add_sync(HP_FULL_MASK, before);
-#pragma unroll
-        for (int w = 0; w < PART; ++w) {
-            cnt[(w0 + w) * ONE_ROW + dg] = off;
-            off += c[w];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < ONE_ITEMS; ++i)
-            if (i < rounds) pos[i] += wcnt[digit_of(key[i], shift, dmask)];
+        one_rank(key, sh, shift, dmask, cnt, s_w, pos);
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < ONE_ITEMS; ++i) {
-            if (i < rounds && wbase + i * 32 + lane < n) {
+            if (sh.has(i)) {
                 skeys[pos[i]] = key[i];
                 svals[pos[i]] = val[i];
             }
@@ -384,15 +386,38 @@ __global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__
         if (shift + 8 >= bits) break;
 #pragma unroll
         for (int i = 0; i < ONE_ITEMS; ++i) {
-            const int idx = wbase + i * 32 + lane;
-            if (i < rounds && idx < n) {
-                key[i] = skeys[idx];
-                val[i] = svals[idx];
+            if (sh.has(i)) {
+                key[i] = skeys[sh.at(i)];
+                val[i] = svals[sh.at(i)];
             }
         }
         __syncthreads();
     }
-    for (int j = tid; j < n; j += ONE_BLOCK) {
+}
+
+template <typename K>
+__global__ void __launch_bounds__(ONE_BLOCK, 1) k_sort_one(const K* __restrict__ keys_in,
+                                                           const int32_t* __restrict__ vals_in,
+                                                           K* __restrict__ keys_out, int32_t* __restrict__ vals_out,
+                                                           int n, int bits) {
+    hp_after_previous();
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);   // [NW][ONE_ROW] while ranking
+    K* skeys = reinterpret_cast<K*>(smem);                // [ONE_CAP] while staging
+    int32_t* svals = reinterpret_cast<int32_t*>(smem + (size_t)ONE_CAP * sizeof(K));
+    __shared__ uint32_t s_w[ONE_BLOCK / 32];
+    const one_shape sh(n);
+    K key[ONE_ITEMS];
+    int32_t val[ONE_ITEMS];
+#pragma unroll
+    for (int i = 0; i < ONE_ITEMS; ++i) {
+        const int idx = sh.at(i);
+        const bool valid = sh.has(i);
+        key[i] = valid ? keys_in[idx] : K(0);
+        val[i] = valid ? (vals_in ? vals_in[idx] : idx) : 0;
+    }
+    one_sort(key, val, sh, bits, cnt, s_w, skeys, svals);
+    for (int j = threadIdx.x; j < n; j += ONE_BLOCK) {
         keys_out[j] = skeys[j];
         vals_out[j] = svals[j];
     }
@@ -417,18 +442,32 @@ constexpr size_t sort_one_smem() {
 // (low bits, position), so equal keys keep their order), longer ones by the
 // whole CTA with stable 8-bit passes in shared memory. Every key is read and
 // written once more instead of five more times; the result equals the stable
-// sort by key. Segments larger than SEG_CAP (very uneven key distributions)
-// are listed and sorted by k_seg_big, one CTA per segment, with stable passes
-// through global memory.
+// sort by key. Segments larger than SEG_CAP (uneven key distributions) are listed
+// and sorted by k_seg_big: up to SEG_LONG keys by one CTA, longer ones by a CTA per
+// chunk with stable passes through global memory.
 constexpr int SEG_BLOCK = 256, SEG_ITEMS = 8, SEG_CAP = SEG_BLOCK * SEG_ITEMS, SEG_WINDOW = 1536;
 constexpr int SEG_NW = SEG_BLOCK / 32;
 constexpr int SEG_RANK_MAX = 512;  // segments ranked element by element
 constexpr int SEG_MED_CAP = SEG_CAP / (SEG_RANK_MAX + 1) + 1;  // longer segments in one chunk
+// Segments past this many keys are sorted chunk by chunk, shorter ones by a CTA each from
+// shared memory. One far triangle is enough to put every other key under one prefix.
+constexpr int SEG_LONG = ONE_CAP;
+constexpr int SEG_CTAS = 148;  // chunks that a whole array makes at most (and CTAs of k_seg_big)
+
+// Keys of a chunk (a pass over 2,048 takes a CTA 11 us with its barriers, over 8,192 20), and
+// the most chunks of an array's long segments (each may end in a short one).
+__host__ __device__ constexpr int64_t seg_chunk(int64_t n) {
+    return SEG_CAP * ((n + (int64_t)SEG_CAP * SEG_CTAS - 1) / ((int64_t)SEG_CAP * SEG_CTAS));
+}
+__host__ __device__ constexpr int64_t seg_chunks(int64_t n) { return n / seg_chunk(n) + n / SEG_LONG + 1; }
 
 // Whenever wide keys do not fit one CTA. Below 2^20 keys a pass is mostly latency
 // (11 us at 0.1 M keys, 18 us at 1 M), so five passes fewer count for more there:
 // 60-bit keys on a B200, 100,003 of them 0.121 -> 0.065 ms, 1,048,573 of them
-// 0.170 -> 0.091 ms against eight passes.
+// 0.170 -> 0.091 ms against eight passes, which take that long whatever the keys. Keys all
+// under one prefix take 0.12 and 0.22 ms (LBVH builds with one far triangle 0.22 and 0.48 ms,
+// 0.24 and 0.51 with eight passes); the worst found, every segment just past SEG_LONG, 0.17 and
+// 0.31 ms.
 __host__ __device__ constexpr bool hybrid_sort(int64_t n, int key_bytes, int bits) {
     return key_bytes == 8 && bits > 48 && n > ONE_CAP;
 }
@@ -712,7 +751,7 @@ __global__ void __launch_bounds__(SEG_BLOCK, 4) k_seg_sort(const uint64_t* __res
                                                         const int32_t* __restrict__ vin,
                                                         uint64_t* __restrict__ kout, int32_t* __restrict__ vout,
                                                         int64_t n, int L, int2* big, uint32_t* big_count,
-                                                        int64_t big_cap, int* err) {
+                                                        int64_t big_cap, int4* chunks, int* err) {
     hp_after_previous();
     extern __shared__ __align__(16) unsigned char seg_raw[];
     seg_smem& S = *reinterpret_cast<seg_smem*>(seg_raw);
@@ -761,14 +800,25 @@ __global__ void __launch_bounds__(SEG_BLOCK, 4) k_seg_sort(const uint64_t* __res
             seg_sort_chunk_global(S, kin, vin, kout, vout, cs, (int)(ce - cs), L, err);
         return;
     }
-    // A large run: batches of whole segments up to SEG_CAP keys; a segment
-    // larger than that goes to the list k_seg_big sorts.
+    // A large run: batches of whole segments up to SEG_CAP keys; a segment larger
+    // than that goes to one of the two lists that k_seg_big sorts: big_count[0] whole
+    // ones, big_count[1] chunks {begin, end, number in the segment, the segment's first}.
     int64_t cur = cs;
     while (cur < ce) {
         __syncthreads();
         if (threadIdx.x == 0) {
             int64_t e1 = seg_end(kin, n, cur, L);
-            if (e1 - cur > SEG_CAP) {
+            if (e1 - cur > SEG_LONG) {
+                const int nc = (int)((e1 - cur + seg_chunk(n) - 1) / seg_chunk(n));
+                const int at = (int)atomicAdd(big_count + 1, (uint32_t)nc);
+                if (at + nc <= seg_chunks(n)) {
+                    for (int i = 0; i < nc; ++i) chunks[at + i] = make_int4((int)cur, (int)e1, i, at);
+                } else {
+                    hp_report(err, HP_DEV_BAD_INDEX, (int)cur);
+                }
+                S.range[2] = e1;
+                S.range[3] = e1;  // nothing to sort here
+            } else if (e1 - cur > SEG_CAP) {
                 const uint32_t slot = atomicAdd(big_count, 1u);
                 if ((int64_t)slot < big_cap) big[slot] = make_int2((int)cur, (int)e1);
                 else hp_report(err, HP_DEV_BAD_INDEX, (int)cur);
@@ -792,82 +842,160 @@ __global__ void __launch_bounds__(SEG_BLOCK, 4) k_seg_sort(const uint64_t* __res
     }
 }
 
-// Segments larger than SEG_CAP: one CTA each, stable 8-bit passes over the
-// low L bits through global memory, tiles in order with running digit
-// offsets; the input and output ranges serve as the two buffers.
-__global__ void __launch_bounds__(SEG_BLOCK, 4) k_seg_big(uint64_t* kin, int32_t* vin_buf, const int32_t* vin,
-                                                       uint64_t* kout, int32_t* vout, int L, const int2* big,
-                                                       const uint32_t* big_count, int64_t big_cap, int64_t n,
-                                                       int* err) {
-    hp_after_previous();
-    extern __shared__ __align__(16) unsigned char seg_raw[];
-    seg_smem& S = *reinterpret_cast<seg_smem*>(seg_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t count = min((int64_t)*big_count, big_cap);
-    const int passes = (L + 7) / 8;
+// Segments larger than SEG_CAP, sorted by their low L bits. First the listed whole
+// segments, a CTA each, as k_sort_one does. Then all chunks of the longer ones in step, with
+// stable 8-bit passes through global memory: every pass counts the chunks' digits (row c of
+// `rows`), adds up the rows of its segment and moves its keys tile by tile, with a grid
+// barrier after both halves (a cooperative launch; none is reached without a chunk). The
+// input and output ranges serve as the two buffers (the first pass reads the input), and an
+// even number of passes ends with a copy to the output. Bound by the barriers' and the
+// ranks' latency. All keys under one prefix, the whole sort on a B200 (one CTA a segment /
+// now): 100,003 keys 1.25 / 0.12 ms, 1,048,573 12.4 / 0.22, 4.2 M 51 / 0.57; segments of 6,000,
+// the same sizes: 0.15 / 0.10, 0.26 / 0.16, 0.76 / 0.36.
+__global__ void __launch_bounds__(ONE_BLOCK, 1) k_seg_big(uint64_t* kin, int32_t* vin_buf, const int32_t* vin,
+                                                          uint64_t* kout, int32_t* vout, int L, const int2* big,
+                                                          const uint32_t* big_count, int64_t big_cap,
+                                                          const int4* chunks, uint32_t* rows, unsigned* bar, int64_t n,
+                                                          int* err) {
+    constexpr int PARTS = ONE_BLOCK / 256;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);
+    uint64_t* skeys = reinterpret_cast<uint64_t*>(smem);
+    int32_t* svals = reinterpret_cast<int32_t*>(smem + (size_t)ONE_CAP * sizeof(uint64_t));
+    __shared__ uint32_t s_w[ONE_BLOCK / 32], s_sum[PARTS][256], s_before[PARTS][256], s_next[256];
+    const int tid = threadIdx.x, dg = tid & 255, part = tid >> 8;
+    uint64_t key[ONE_ITEMS];
+    int32_t val[ONE_ITEMS];
+    auto load = [&](const one_shape& sh, const uint64_t* ks, const int32_t* vs, int64_t from) {
+#pragma unroll
+        for (int i = 0; i < ONE_ITEMS; ++i) {
+            const int64_t j = from + sh.at(i);
+            key[i] = sh.has(i) ? __ldcg(ks + j) : 0ull;
+            val[i] = sh.has(i) ? (vs ? __ldcg(vs + j) : (int32_t)j) : 0;
+        }
+    };
+    const int64_t count = min((int64_t)big_count[0], big_cap);
     for (int64_t g = blockIdx.x; g < count; g += gridDim.x) {
         const int64_t s0 = big[g].x, s1 = big[g].y;
-        if (s0 < 0 || s1 > n || s0 >= s1) {
-            if (threadIdx.x == 0) hp_report(err, HP_DEV_BAD_INDEX, (int)g);
+        if (s0 < 0 || s1 > n || s0 >= s1 || s1 - s0 > ONE_CAP) {
+            if (tid == 0) hp_report(err, HP_DEV_BAD_INDEX, (int)g);
             continue;
         }
-        // the first pass reads the input buffers, then output and input
-        // ranges alternate; an even pass count ends with a copy to the output
-        for (int p = 0; p < passes; ++p) {
-            const bool to_out = (p & 1) == 0;
-            const uint64_t* ks = to_out ? kin : kout;
-            uint64_t* kd = to_out ? kout : kin;
-            const int32_t* vs = p == 0 ? vin : (to_out ? vin_buf : vout);
-            int32_t* vd = to_out ? vout : vin_buf;
-            const int shift = 8 * p;
-            // digit histogram of the segment, exclusive offsets
-            if (tid < 256) S.tot[tid] = 0;
+        const one_shape sh((int)(s1 - s0));
+        load(sh, kin, vin, s0);
+        one_sort(key, val, sh, L, cnt, s_w, skeys, svals);
+        for (int j = tid; j < sh.n; j += ONE_BLOCK) {
+            kout[s0 + j] = skeys[j];
+            vout[s0 + j] = svals[j];
+        }
+        __syncthreads();
+    }
+    const int total = (int)min((int64_t)big_count[1], seg_chunks(n));
+    if (total == 0) return;
+    // chunk c's segment [x, y), its number z in it and the segment's first chunk w, its own
+    // keys [b, e); false: skip
+    int4 q;
+    int64_t b, e;
+    auto chunk = [&](int c) {
+        q = chunks[c];
+        if (q.x < 0 || q.y > n || q.x >= q.y || q.z < 0 || q.w < 0 || q.w != c - q.z) {
+            if (tid == 0) hp_report(err, HP_DEV_BAD_INDEX, c);
+            return false;
+        }
+        b = q.x + q.z * seg_chunk(n);
+        e = min(b + seg_chunk(n), (int64_t)q.y);
+        return b < e;
+    };
+    const int passes = (L + 7) / 8;
+    for (int p = 0; p < passes; ++p) {
+        const bool to_out = (p & 1) == 0;
+        const uint64_t* ks = to_out ? kin : kout;
+        uint64_t* kd = to_out ? kout : kin;
+        const int32_t* vs = p == 0 ? vin : (to_out ? vin_buf : vout);
+        int32_t* vd = to_out ? vout : vin_buf;
+        const int shift = 8 * p;
+        for (int c = blockIdx.x; c < total; c += gridDim.x) {
+            if (!chunk(c)) continue;
             __syncthreads();
-            for (int64_t j = s0 + tid; j < s1; j += SEG_BLOCK) atomicAdd(&S.tot[(uint32_t)(ks[j] >> shift) & 255u], 1u);
+            if (tid < 256) s_next[tid] = 0;
             __syncthreads();
-            if (tid == 0) {
-                uint32_t run = 0;
-                for (int d = 0; d < 256; ++d) { const uint32_t c = S.tot[d]; S.part[d] = run; run += c; }
+#pragma unroll 8
+            for (int64_t j = b + tid; j < e; j += ONE_BLOCK)
+                atomicAdd(&s_next[(uint32_t)(__ldcg(ks + j) >> shift) & 255u], 1u);
+            __syncthreads();
+            if (tid < 256) __stcg(rows + (size_t)c * 256 + tid, s_next[tid]);
+        }
+        if (!hp_grid_barrier(bar, err, LOOKBACK_SPIN_LIMIT)) return;
+        for (int c = blockIdx.x; c < total; c += gridDim.x) {
+            if (!chunk(c)) continue;
+            // the segment's rows, a quarter to each 256 threads
+            const int nc = min((int)((q.y - q.x + seg_chunk(n) - 1) / seg_chunk(n)), total - q.w);
+            const uint32_t* row = rows + (size_t)q.w * 256 + dg;
+            uint32_t sum = 0, before = 0;
+#pragma unroll 8
+            for (int i = part; i < nc; i += PARTS) {
+                const uint32_t x = __ldcg(row + (size_t)i * 256);
+                sum += x;
+                before += i < q.z ? x : 0u;
             }
             __syncthreads();
-            for (int64_t t0 = s0; t0 < s1; t0 += SEG_CAP) {
-                const int m = (int)min((int64_t)SEG_CAP, s1 - t0);
-                uint64_t key[SEG_ITEMS];
-                int32_t val[SEG_ITEMS];
+            s_sum[part][dg] = sum;
+            s_before[part][dg] = before;
+            __syncthreads();
+            uint32_t incl = 0;
+            if (tid < 256) {
+                sum = before = 0;
 #pragma unroll
-                for (int i = 0; i < SEG_ITEMS; ++i) {
-                    const int e = warp * 32 * SEG_ITEMS + i * 32 + lane;
-                    key[i] = e < m ? ks[t0 + e] : 0ull;
-                    val[i] = e < m ? (vs ? vs[t0 + e] : (int32_t)(t0 + e)) : 0;
+                for (int i = 0; i < PARTS; ++i) {
+                    sum += s_sum[i][tid];
+                    before += s_before[i][tid];
                 }
-                uint32_t pos[SEG_ITEMS];
-                seg_block_rank(key, m, shift, S.cnt, S.dstart, S.tot, pos);
+                incl = sum;
 #pragma unroll
-                for (int i = 0; i < SEG_ITEMS; ++i) {
-                    const int e = warp * 32 * SEG_ITEMS + i * 32 + lane;
-                    if (e < m) {
-                        const uint32_t d = (uint32_t)(key[i] >> shift) & 255u;
-                        const int64_t o = s0 + S.part[d] + (pos[i] - S.dstart[d]);
-                        if (o >= s0 && o < s1) {  // always, unless ranges listed twice overlap
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(HP_FULL_MASK, incl, o);
+                    if ((tid & 31) >= o) incl += y;
+                }
+                if ((tid & 31) == 31) s_w[tid >> 5] = incl;
+            }
+            __syncthreads();
+            if (tid < 256) {
+                for (int w = 0; w < (tid >> 5); ++w) before += s_w[w];
+                s_next[tid] = incl - sum + before;  // where the chunk's next key of the digit goes
+            }
+            for (int64_t t0 = b; t0 < e; t0 += ONE_CAP) {
+                const one_shape sh((int)min((int64_t)ONE_CAP, e - t0));
+                load(sh, ks, vs, t0);
+                __syncthreads();
+                uint32_t pos[ONE_ITEMS];
+                one_rank(key, sh, shift, 255u, cnt, s_w, pos);
+#pragma unroll
+                for (int i = 0; i < ONE_ITEMS; ++i) {
+                    if (sh.has(i)) {
+                        const uint32_t d = digit_of(key[i], shift, 255u);
+                        const int64_t o = q.x + (int64_t)(s_next[d] + (pos[i] - cnt[d]));
+                        if (o >= q.x && o < q.y) {  // always, unless ranges listed twice overlap
                             kd[o] = key[i];
                             vd[o] = val[i];
                         } else {
-                            hp_report(err, HP_DEV_BAD_INDEX, (int)g);
+                            hp_report(err, HP_DEV_BAD_INDEX, c);
                         }
                     }
                 }
                 __syncthreads();
-                if (tid < 256) S.part[tid] += S.tot[tid];
-                __syncthreads();
+                if (tid < 256) s_next[tid] += (tid < 255 ? cnt[tid + 1] : (uint32_t)sh.n) - cnt[tid];
             }
         }
-        if ((passes & 1) == 0) {  // the last pass wrote the input range
-            for (int64_t j = s0 + tid; j < s1; j += SEG_BLOCK) {
-                kout[j] = kin[j];
-                vout[j] = vin_buf[j];
+        if (!hp_grid_barrier(bar, err, LOOKBACK_SPIN_LIMIT)) return;
+    }
+    if ((passes & 1) == 0) {  // the last pass wrote the input range
+        for (int c = blockIdx.x; c < total; c += gridDim.x) {
+            if (!chunk(c)) continue;
+            for (int64_t j = b + tid; j < e; j += ONE_BLOCK) {
+                kout[j] = __ldcg(kin + j);
+                vout[j] = __ldcg(vin_buf + j);
             }
         }
-        __syncthreads();
     }
 }
 
@@ -938,18 +1066,32 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
             int32_t* sv = const_cast<int32_t*>(src_v);
             uint32_t* big_count = counters + 32;  // zeroed with the status words
             const int64_t big_cap = n / (SEG_CAP + 1) + 1;
-            int2* big = reinterpret_cast<int2*>(cv.take<int2>((size_t)big_cap));
+            int2* big = cv.take<int2>((size_t)big_cap);
+            int4* chunks = cv.take<int4>((size_t)seg_chunks(n));
+            // the look-back words of the passes that are not made hold the chunks' digit counts
+            uint32_t* rows = status + (size_t)SEG_TOP * plan.tiles * 256;
+            if (seg_chunks(n) > (plan.passes - SEG_TOP) * plan.tiles)
+                return hp_fail(HP_ERR_UNSUPPORTED, "radix sort: too few words for the chunks' digit counts");
             const size_t seg_bytes = sizeof(seg_smem);
             HP_CUDA(cudaFuncSetAttribute(k_seg_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_bytes));
-            HP_CUDA(cudaFuncSetAttribute(k_seg_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_bytes));
-            HP_CHAIN(k_seg_sort, hp_div_up(n, SEG_WINDOW), SEG_BLOCK, seg_bytes, stream, 
-                sk, sv, reinterpret_cast<uint64_t*>(a.keys_out), a.vals_out, n, s0, big, big_count, big_cap,
-                a.status);
-            HP_CUDA(cudaGetLastError());
-            HP_CHAIN(k_seg_big, std::min<int64_t>(big_cap, 296), SEG_BLOCK, seg_bytes, stream, 
-                sk, sv, sv, reinterpret_cast<uint64_t*>(a.keys_out), a.vals_out, s0, big, big_count, big_cap, n,
-                a.status);
-            HP_CUDA(cudaGetLastError());
+            constexpr size_t big_bytes = sort_one_smem<uint64_t>();
+            HP_CUDA(cudaFuncSetAttribute(k_seg_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)big_bytes));
+            HP_CHAIN(k_seg_sort, hp_div_up(n, SEG_WINDOW), SEG_BLOCK, seg_bytes, stream, sk, sv,
+                     reinterpret_cast<uint64_t*>(a.keys_out), a.vals_out, n, s0, big, big_count, big_cap, chunks,
+                     a.status);
+            int occ = 0, dev = 0, sms = 0;
+            HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_seg_big, ONE_BLOCK, big_bytes));
+            HP_CUDA(cudaGetDevice(&dev));
+            HP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            const int grid = (int)std::min<int64_t>(big_cap, std::min(SEG_CTAS, std::max(1, occ * sms)));
+            uint64_t* ok = reinterpret_cast<uint64_t*>(a.keys_out);
+            int32_t* ov = a.vals_out;
+            const int32_t* sv_in = sv;
+            unsigned* bar = counters + 40;  // zeroed likewise
+            int low = s0;
+            void* args[] = {&sk, &sv, &sv_in, &ok, &ov, &low, &big, &big_count, (void*)&big_cap, &chunks,
+                            &rows, &bar, (void*)&n, (void*)&a.status};
+            HP_CUDA(cudaLaunchCooperativeKernel((const void*)k_seg_big, grid, ONE_BLOCK, args, big_bytes, stream));
             hp_count_launch(2);
             hp_mark(a.ctx, stream, "sort_segments");
             return HP_OK;
@@ -1142,8 +1284,9 @@ hp_sort_plan hp_sort_make_plan(int64_t n, int key_bytes, int bits, int block) {
     p.tiles = std::max<int64_t>(1, (n + p.tile - 1) / p.tile);
     size_t kv = hp_carve::pad((size_t)n * key_bytes) + hp_carve::pad((size_t)n * 4);
     p.scratch_bytes = 2 * kv + hp_carve::pad(((size_t)p.passes * p.tiles * 256 + 64) * 4);
-    if (hybrid_sort(n, key_bytes, bits))  // the list of segments too large for one CTA's shared memory
-        p.scratch_bytes += hp_carve::pad((size_t)(n / (SEG_CAP + 1) + 1) * 8);
+    if (hybrid_sort(n, key_bytes, bits))  // the lists of segments too large for one CTA's shared memory
+        p.scratch_bytes += hp_carve::pad((size_t)(n / (SEG_CAP + 1) + 1) * 8) +
+                           hp_carve::pad((size_t)seg_chunks(n) * 16);
     return p;
 }
 
@@ -1220,7 +1363,8 @@ constexpr size_t NOALLOC_BYTES =
                                      sort_cfg<uint64_t>::BLOCK * sort_cfg<uint64_t>::ITEMS, 8),
                 noalloc_sort_scratch(HP_NOALLOC_SORT_MAX_KEYS, 4,
                                      sort_cfg<uint32_t>::BLOCK * sort_cfg<uint32_t>::ITEMS, 4)) +
-    noalloc_pad((HP_NOALLOC_SORT_MAX_KEYS / (SEG_CAP + 1) + 1) * 8) +  // long segments of wide keys
+    noalloc_pad((HP_NOALLOC_SORT_MAX_KEYS / (SEG_CAP + 1) + 1) * 8) +  // large segments of wide keys
+    noalloc_pad(seg_chunks(HP_NOALLOC_SORT_MAX_KEYS) * 16) +
     noalloc_pad(8 * 256 * 4) + 256;
 
 __device__ __align__(256) unsigned char g_noalloc_sort_scratch[NOALLOC_BYTES];

@@ -103,3 +103,66 @@ def test_sort_one_cta_edges(ctx, dtype, n, kind):
     ctx.check()
     np.testing.assert_array_equal(ko.cpu().numpy().view(dtype), keys[order])
     np.testing.assert_array_equal(vo.cpu().numpy(), vals[order])
+
+
+def _long_case(kind, n, bits, rng):
+    """Wide keys with runs of equal top 24 bits around the sizes where k_seg_big goes from
+    a CTA per run to chunks (8,192 keys; a chunk of these arrays is 2,048 or, of the largest, 6,144)."""
+    low = rng.integers(0, 1 << (bits - 24), size=n, dtype=np.uint64)
+    if kind == "one":
+        top = np.full(n, 9, np.uint64)
+    elif kind == "outlier":
+        top = np.zeros(n, np.uint64)
+        top[n // 3] = (1 << 24) - 1
+    else:  # whole runs, chunked ones and short ones together
+        sizes, left = [], n
+        for m in (8191, 8192, 8193, 2048, 2049, 10240, 10241, 5, 20000) * (n // 60000 + 1):
+            sizes.append(min(m, left))
+            left -= sizes[-1]
+        sizes.append(left)
+        top = np.repeat(np.arange(len(sizes), dtype=np.uint64) * np.uint64(3), sizes)
+        top = top[rng.permutation(n)]
+    low[: n // 50] = low[0]
+    return (top << np.uint64(bits - 24)) | low
+
+
+@pytest.mark.parametrize("kind", ["one", "outlier", "mixed"])
+@pytest.mark.parametrize("n,bits,with_vals", [(8193, 60, False), (16385, 64, True), (100003, 60, True),
+                                              (70001, 49, False), (131072, 56, True), (700001, 60, False)])
+def test_radix_sort_long_runs(ctx, kind, n, bits, with_vals):
+    rng = np.random.default_rng(n + len(kind))
+    keys = _long_case(kind, n, bits, rng)
+    vals = rng.permutation(n).astype(np.int32) if with_vals else None
+    K = torch.from_numpy(keys.view(np.int64)).cuda()
+    for block in (512, 256):
+        ctx.set_tune(sort_block=block)
+        try:
+            ko, vo = ctx.radix_sort(K, None if vals is None else torch.from_numpy(vals).cuda(), bits=bits)
+            ctx.check()
+        finally:
+            ctx.reset_tune()
+        order = np.argsort(keys, kind="stable")
+        np.testing.assert_array_equal(vo.cpu().numpy(), vals[order] if with_vals else order.astype(np.int32))
+        np.testing.assert_array_equal(ko.cpu().numpy().view(np.uint64), keys[order])
+
+
+@pytest.mark.parametrize("n", [100003, 1048573])
+def test_one_prefix_costs_little_more(ctx, n):
+    """Keys under one prefix take no more than four times as long as spread ones (twice, as
+    measured; 19 and 120 times when one CTA sorted them)."""
+    rng = np.random.default_rng(n)
+    low = rng.integers(0, 1 << 36, size=n, dtype=np.uint64)
+    ms = {}
+    for kind, top in (("spread", rng.integers(0, 1 << 24, size=n, dtype=np.uint64)), ("one", np.full(n, 9, np.uint64))):
+        K = torch.from_numpy(((top << np.uint64(36)) | low).view(np.int64)).cuda()
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        got = []
+        for _ in range(9):
+            a.record()
+            ctx.radix_sort(K, bits=60)
+            b.record()
+            b.synchronize()
+            got.append(a.elapsed_time(b))
+        ms[kind] = sorted(got)[4]
+    ctx.check()
+    assert ms["one"] < 4 * ms["spread"], ms

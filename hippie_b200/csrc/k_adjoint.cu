@@ -8,11 +8,11 @@
 //   dL/dv0 = -u q,  dL/dv1 = -v q,  dL/dv2 = -(1-u-v) q,
 // and A^-T g = (g_u (b x c) + g_v (c x a) + g_t (a x b)) / det(A) for A = [a b c].
 // Lanes of a warp whose rays hit the same triangle add their contributions with
-// shuffles first, so each distinct triangle costs one set of reductions per warp,
-// two requests a vertex. Bound by the reductions' and gathers' requests. The sums
-// run over all groups at once with full-warp shuffles: summing a group at a time
-// under its own mask ran a warp's groups one after another (4.2 M rays on a
-// 1 M-triangle heightfield 0.366 -> 0.089 ms).
+// shuffles first, and triangles around a vertex theirs for it, so each costs one set of
+// reductions per warp, two requests a vertex. Bound by the reductions' and gathers'
+// requests. The sums run over all groups at once with full-warp shuffles: summing a group at
+// a time under its own mask ran a warp's groups one after another (4.2 M rays on a
+// 1 M-triangle heightfield 0.366 -> 0.092 ms).
 //
 // Refit: HipBVH::update (rt/bvh/HipBVH.cpp:472-477) = woopifyTriangles +
 // refitLeavesBin + refitInteriorsBin (rt/bvh/HipBVHKernels.cu:240-326). The
@@ -49,14 +49,37 @@ __device__ __forceinline__ void add3(float* __restrict__ dverts, int idx, float 
     asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(hi ? p : p + 2), "f"(hi ? x : z) : "memory");
 }
 
+// Sums x over the lanes with the same id (no lane with a negative one); the lowest of them
+// gets the sum and true. As many rounds as the largest group has halvings: every round,
+// each remaining lane of a group takes its next one's sums, and every second lane drops
+// out. All 32 lanes take part in every shuffle, whatever their groups.
+template <int C>
+__device__ __forceinline__ bool join(int id, float (&x)[C]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned grp = __match_any_sync(HP_FULL_MASK, id), below = (1u << lane) - 1u;
+    unsigned rest = id >= 0 ? grp & ~below & ~(1u << lane) : 0u;  // the group's later lanes
+    const bool first = id >= 0 && (grp & below) == 0;
+    int pos = __popc(grp & below);
+    while (__any_sync(HP_FULL_MASK, rest != 0)) {
+        const int next = rest ? __ffs(rest) - 1 : lane;
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+            const float o = __shfl_sync(HP_FULL_MASK, x[k], next);
+            if (rest) x[k] += o;
+        }
+        rest &= __ballot_sync(HP_FULL_MASK, !(pos & 1));
+        pos >>= 1;
+    }
+    return first;
+}
+
 __global__ void __launch_bounds__(AB) k_adjoint(const float* __restrict__ verts, int64_t nv,
                                                 const int32_t* __restrict__ tris, int64_t ntri,
                                                 const float4* __restrict__ rays,
                                                 const int4* __restrict__ results,
                                                 const float* __restrict__ dl, int64_t num_rays,
-                                                float* __restrict__ dverts, int* err) {
+                                                float* __restrict__ dverts, bool dense, int* err) {
     const int64_t i = blockIdx.x * (int64_t)AB + threadIdx.x;
-    const int lane = threadIdx.x & 31;
     int hit = -1;  // triangle of the lane's contribution
     int idx[3] = {0, 0, 0};
     float g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -99,27 +122,25 @@ __global__ void __launch_bounds__(AB) k_adjoint(const float* __restrict__ verts,
             }
         }
     }
-    // Lanes of one triangle sum their nine components first, in as many rounds as
-    // the largest group has halvings: every round, each remaining lane of a group
-    // takes its next one's sums, and every second lane drops out. All 32 lanes
-    // take part in every shuffle, whatever their groups.
-    const unsigned grp = __match_any_sync(HP_FULL_MASK, hit);
-    unsigned rest = hit >= 0 ? grp & ~((2u << lane) - 1u) : 0u;  // the group's later lanes
-    const bool lead = hit >= 0 && (grp & ((1u << lane) - 1u)) == 0;
-    int pos = __popc(grp & ((1u << lane) - 1u));
-    while (__any_sync(HP_FULL_MASK, rest != 0)) {
-        const int next = rest ? __ffs(rest) - 1 : lane;
+    // Lanes of one triangle sum their nine components first; then, corner by corner, the
+    // triangles' first lanes with the same vertex sum its three, lest they add to one
+    // address one after another: where the warp's first triangle shares its vertex with two
+    // others (on a fan of 4,096 triangles around a vertex 4.2 M rays take 12.8 ms without,
+    // 0.44 with), and everywhere on a mesh so coarse that warps queue for its vertices
+    // (`dense`; 2 x 4 x 4 triangles 5.25 and 3.46 ms, 2 x 32 x 32 equal). Elsewhere the search
+    // costs more than it saves: a 1 M-triangle heightfield, where two share, 0.134 ms with it,
+    // 0.092 without.
+    const bool lead = join(hit, g);
+    const unsigned leads = __ballot_sync(HP_FULL_MASK, lead);
+    if (leads == 0) return;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const float o = __shfl_sync(HP_FULL_MASK, g[k], next);
-            if (rest) g[k] += o;
-        }
-        rest &= __ballot_sync(HP_FULL_MASK, !(pos & 1));
-        pos >>= 1;
-    }
-    if (lead) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) add3(dverts, idx[k], g[3 * k], g[3 * k + 1], g[3 * k + 2]);
+    for (int k = 0; k < 3; ++k) {
+        const int front = __shfl_sync(HP_FULL_MASK, idx[k], __ffs(leads) - 1);
+        bool add = lead;
+        float v[3] = {g[3 * k], g[3 * k + 1], g[3 * k + 2]};
+        const int same = __popc(__ballot_sync(HP_FULL_MASK, lead && idx[k] == front));
+        if (dense || same >= 3) add = join(lead ? idx[k] : -1, v);
+        if (add) add3(dverts, idx[k], v[0], v[1], v[2]);
     }
 }
 
@@ -204,7 +225,7 @@ hp_status hp_adjoint_launch(hp_ctx* ctx, const hp_mesh* m, const float* rays, co
     k_adjoint<<<hp_div_up(num_rays, AB), AB, 0, s>>>(
         m->vertices, m->num_vertices, m->triangles, m->num_triangles,
         reinterpret_cast<const float4*>(rays), reinterpret_cast<const int4*>(results), dl_dtuv,
-        num_rays, dl_dvertices, ctx->d_status);
+        num_rays, dl_dvertices, num_rays / 2048 >= m->num_vertices, ctx->d_status);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "adjoint");

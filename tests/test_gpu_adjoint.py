@@ -243,3 +243,71 @@ def test_adjoint_groups_and_alignment(ctx, group, shift):
     # numpy with 64-bit sums is 5e-7 to 8e-7 off): below 1e-5 of the norm
     err = np.linalg.norm(grad.cpu().numpy().astype(np.float64) - exp) / np.linalg.norm(exp)
     assert err < 1e-5
+
+
+def _fan(k, corner):
+    """k triangles around one vertex, which is their corner `corner`."""
+    a = 2 * np.pi * np.arange(k) / k
+    v = np.concatenate([[[0.5, 0.5, 0.0]], np.stack([0.5 + 0.7 * np.cos(a), 0.5 + 0.7 * np.sin(a),
+                                                      0.05 * np.sin(3 * a)], 1)]).astype(np.float32)
+    i = np.arange(k)
+    t = np.stack([np.zeros(k, int), 1 + i, 1 + (i + 1) % k], 1)
+    return v, np.roll(t, corner, axis=1).astype(np.int32).copy()
+
+
+@pytest.mark.parametrize("corner", [0, 1, 2])
+@pytest.mark.parametrize("k,n", [(3, 8191), (5, 20001), (64, 4099)])
+def test_adjoint_around_a_vertex(ctx, k, n, corner):
+    """Rays on the triangles of a fan in no order, so that a warp's triangles share a
+    vertex: many rays a vertex (both branches of the rule for coarse meshes) and few."""
+    v, t = _fan(k, corner)
+    rng = np.random.default_rng(k + corner)
+    tri = rng.integers(0, k, n)
+    uv = rng.uniform(0.1, 0.45, (n, 2))
+    p = v[t[tri]].astype(np.float64)
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, 4:7] = rng.normal(size=(n, 3)) * 0.1 + [0, 0, -1]
+    rays[:, :3] = uv[:, :1] * p[:, 0] + uv[:, 1:] * p[:, 1] + (1 - uv.sum(1, keepdims=True)) * p[:, 2] - rays[:, 4:7]
+    res = np.zeros((n, 4), np.int32)
+    res[:, 0] = np.where(rng.random(n) < 0.05, -1, tri)
+    res[:, 1] = np.ones(n, np.float32).view(np.int32)
+    res[:, 2:] = uv.astype(np.float32).view(np.int32)
+    w = rng.standard_normal((n, 3)).astype(np.float32)
+    grad = ctx.adjoint(dev(v), dev(t), dev(rays), dev(res), dev(w))
+    ctx.check()
+    exp = oracle.adjoint64(v, t, rays, res, w)
+    # as in test_adjoint_groups_and_alignment, with triangles of 0.07 and more
+    err = np.linalg.norm(grad.cpu().numpy().astype(np.float64) - exp) / np.linalg.norm(exp)
+    assert err < 1e-5
+
+
+def test_adjoint_fan_costs_little_more(ctx):
+    """Rays on 4,096 triangles around one vertex take no more than eight times as long as
+    on as many of a grid (twice, as measured; 50 times when every lane added to the
+    vertex by itself)."""
+    m = 1 << 20
+    rng = np.random.default_rng(1)
+    y, x = np.meshgrid(np.arange(46), np.arange(46), indexing="ij")
+    a = (y[:-1, :-1] * 46 + x[:-1, :-1]).reshape(-1)
+    grid = (np.stack([x, y, np.sin(x + y)], -1).reshape(-1, 3).astype(np.float32),
+            np.stack([a, a + 1, a + 47, a, a + 47, a + 46], -1).reshape(-1, 3).astype(np.int32))
+    ms = {}
+    for name, (v, t) in (("fan", _fan(4096, 0)), ("grid", grid)):
+        res = np.zeros((m, 4), np.int32)
+        res[:, 0] = rng.integers(0, len(t), m)
+        res[:, 2:] = np.float32(0.25).view(np.int32)
+        rays = np.zeros((m, 8), np.float32)
+        rays[:, 4:7] = [0.1, 0.2, -1]
+        V, T, R, H = dev(v), dev(t), dev(rays), dev(res)
+        W, G = torch.ones((m, 3), device="cuda"), torch.zeros_like(V)
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        got = []
+        for _ in range(7):
+            e[0].record()
+            ctx.adjoint(V, T, R, H, W, dl_dverts=G)
+            e[1].record()
+            e[1].synchronize()
+            got.append(e[0].elapsed_time(e[1]))
+        ms[name] = sorted(got)[3]
+    ctx.check()
+    assert ms["fan"] < 8 * ms["grid"], ms

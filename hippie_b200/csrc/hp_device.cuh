@@ -144,9 +144,9 @@ __device__ __forceinline__ void load3(const uint32_t* p, uint32_t& x, uint32_t& 
 }
 
 __device__ __forceinline__ void load_vertex(const float* __restrict__ v, int64_t nv, int idx,
-                                            float& x, float& y, float& z, int* err) {
+                                            float& x, float& y, float& z, int* err, int info) {
     if (idx < 0 || idx >= nv) {
-        hp_report(err, HP_DEV_BAD_INPUT, idx);
+        hp_report(err, HP_DEV_BAD_INPUT, info);
         idx = 0;
     }
     uint32_t a, b, c;
@@ -160,14 +160,16 @@ struct tri_verts {
     float x0, y0, z0, x1, y1, z1, x2, y2, z2;
 };
 
+// A vertex index out of range is reported with itself, or, for NAME_TRI, with the triangle.
+template <bool NAME_TRI = false>
 __device__ __forceinline__ tri_verts load_tri(const float* __restrict__ v, int64_t nv,
                                               const int32_t* __restrict__ t, int64_t tri, int* err) {
     tri_verts r;
     uint32_t a, b, c;
     load3(reinterpret_cast<const uint32_t*>(t + 3 * tri), a, b, c);
-    load_vertex(v, nv, (int)a, r.x0, r.y0, r.z0, err);
-    load_vertex(v, nv, (int)b, r.x1, r.y1, r.z1, err);
-    load_vertex(v, nv, (int)c, r.x2, r.y2, r.z2, err);
+    load_vertex(v, nv, (int)a, r.x0, r.y0, r.z0, err, NAME_TRI ? (int)tri : (int)a);
+    load_vertex(v, nv, (int)b, r.x1, r.y1, r.z1, err, NAME_TRI ? (int)tri : (int)b);
+    load_vertex(v, nv, (int)c, r.x2, r.y2, r.z2, err, NAME_TRI ? (int)tri : (int)c);
     return r;
 }
 

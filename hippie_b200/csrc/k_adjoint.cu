@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(AB) k_adjoint(const float* __restrict__ verts,
             for (int k = 0; k < 3; ++k) {
                 idx[k] = (int)l[k];
                 if (idx[k] < 0 || idx[k] >= nv) { ok = false; idx[k] = 0; }
-                load_vertex(verts, nv, idx[k], p[k].x, p[k].y, p[k].z, err);
+                load_vertex(verts, nv, idx[k], p[k].x, p[k].y, p[k].z, err, tri);
             }
             if (!ok) hp_report(err, HP_DEV_BAD_INPUT, tri);
             const float3 a = make_float3(p[0].x - p[2].x, p[0].y - p[2].y, p[0].z - p[2].z);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(AB) k_refit(const float* __restrict__ verts, i
     float mn[3] = {HP_MAX_FLOAT, HP_MAX_FLOAT, HP_MAX_FLOAT};
     float mx[3] = {-HP_MAX_FLOAT, -HP_MAX_FLOAT, -HP_MAX_FLOAT};
     for (int r = meta.x; r < meta.y; ++r) {
-        const tri_verts t = load_tri(verts, nv, tris, tri_idx[r], err);
+        const tri_verts t = load_tri<true>(verts, nv, tris, tri_idx[r], err);
         mn[0] = fminf(mn[0], fminf(fminf(t.x0, t.x1), t.x2));
         mn[1] = fminf(mn[1], fminf(fminf(t.y0, t.y1), t.y2));
         mn[2] = fminf(mn[2], fminf(fminf(t.z0, t.z1), t.z2));

@@ -1104,7 +1104,7 @@ __global__ void __launch_bounds__(256) k_topdown(td_args T) {
             T.woop[3 * (int64_t)toff + 2] = __ldg(T.woop_src + 3 * (int64_t)tri + 2);
             return;
         }
-        const tri_verts t = load_tri(T.verts, T.nv, T.tris, tri, T.err);
+        const tri_verts t = load_tri<true>(T.verts, T.nv, T.tris, tri, T.err);
         float4 w0, w1, w2;
         hp_woop(t.x0, t.y0, t.z0, t.x1, t.y1, t.z1, t.x2, t.y2, t.z2, w0, w1, w2);
         T.woop[3 * (int64_t)toff] = w0;

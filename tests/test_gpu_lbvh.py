@@ -177,3 +177,16 @@ def test_collapse_of_small_meshes(ctx, n, adaptive):
     ref = oracle.build_lbvh(v, t, bits=30, adaptive=adaptive, max_leaf=5, scale=np.array(bvh.c.morton_scale, np.float32))
     np.testing.assert_array_equal(nodes, ref["nodes"])
     np.testing.assert_array_equal(tri, ref["tri_idx"])
+
+
+def test_refit_names_the_triangle(ctx):
+    """A refit that meets a vertex index out of range reports the triangle that has it."""
+    v, t = hp.gen.uniform_mesh(1, 100)
+    bvh = ctx.build(dev(v), dev(t), hp.BuildParams(morton_bits=30))
+    bvh.sync()
+    t = t.copy()
+    t[10, 1] = 10 ** 6  # the kernel reads vertex 0 instead
+    ctx.refit(bvh, dev(v), dev(t))
+    with pytest.raises(hp.HPError) as ei:
+        ctx.check()
+    assert ei.value.status == 5 and "(info 10)" in str(ei.value)

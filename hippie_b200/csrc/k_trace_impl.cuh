@@ -65,7 +65,8 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 //     waits. The turn ends when fewer than NODE lanes have an interior node and no
 //     postponed leaf, so that a hit is found, and shortens the ray, soon;
 //   * triangles: every lane with a postponed leaf tests one triangle, until fewer
-//     than TRI lanes have one;
+//     than TRI lanes have one (or none, once the rays have run out and no lane has a
+//     node to go on with);
 //   * new rays: once FETCH lanes are without work.
 // A stack entry is the child alone. With its entry distance beside it, entries beyond
 // the hit found since could be dropped at the pop; that saved no time (bounce rays 19.6
@@ -81,18 +82,18 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 // 3: 126, 232; 4: 128, 235; 16: 151, 280. Up to 4 is as good as it was. A visibility
 // ray has no nearest hit to miss.
 //
-// Measured on a B200 (every lane in loops of its own / NODE 1 / 3 / 16): 16.8 M bounce
-// rays 28.4 / 22.9 / 20.0 / 18.4 ms, 43 M rays over 256 meshes 42.4 / 32.0 / 28.3 / 27.3,
-// 4 M sorted rays 3.86 / 3.23 / 3.01 / 3.00, 2.07 M primary rays 0.77 / 0.75 / 0.59 / 0.57,
-// 4.2 M downward rays 2.28 / 2.17 / 2.21 / 2.40, 4.2 M bounce rays on a terrain 3.12 / 2.66 /
-// 2.39 / 2.24, 4.2 M rays in 33.5 M triangles 22.2 / 22.3 / 22.7 / 24.3. FETCH: at 12 bounce
-// rays 19.4 and downward ones 2.35, at 20 20.8 and 2.18. TRI 1 to 6 differ by 2 % either way.
+// Measured on a B200, every lane in loops of its own -> now: 16.8 M bounce rays 28.4 ->
+// 19.1 ms, 43 M rays over 256 meshes 42.4 -> 28.0, 4 M sorted rays 3.86 -> 2.92, 2.07 M primary
+// rays 0.77 -> 0.56, 4.2 M downward rays 2.28 -> 2.22, 4.2 M bounce rays on a terrain 3.12 -> 2.29,
+// 4.2 M rays in 33.5 M triangles 22.2 -> 22.7. Bounce, sorted and primary rays at NODE 1: 22.9,
+// 3.23 and 0.75; 2: 20.9, 3.06, 0.66; 16: 18.4, 3.00, 0.57. FETCH 12 instead of 16: bounce rays
+// 3 % faster, downward ones 6 % slower; 20: the other way round. TRI 1 to 6 differ by 2 % either way.
 // Packed FP32 for the slabs and 32-byte loads of two Woop rows were slower or no faster.
 template <bool ANY_HIT>
 struct turns {
-    static constexpr int NODE = ANY_HIT ? 16 : 3, TRI = ANY_HIT ? 6 : 4, FETCH = 16;
+    static constexpr int NODE = ANY_HIT ? 16 : 4, TRI = ANY_HIT ? 6 : 2, FETCH = 16;
 };
-// CTAs per SM. Closest hits: 12 (40 registers, 8 bytes of spills read back) instead of 10
+// CTAs per SM. Closest hits: 12 (40 registers, 4 bytes of spills read back) instead of 10
 // shorten bounce rays by 8 % and downward ones by 3 %, and cost rays in 33.5 M triangles 3 %.
 // Any hit: 1.05 M shadow rays 0.91 ms at 8 and 9, 0.97 at 10, 1.02 at 12. Batch (the
 // mesh's bases in the lane, 55 registers): 27.3 ms at 8, 28.9 at 9, 30.0 at 10.
@@ -323,7 +324,9 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
             }
             pend = node < 0 || leaf < 0 || tri < tri_end;
             mask = __ballot_sync(HP_FULL_MASK, pend);
-            if (__popc(mask) < TURN::TRI) break;
+            if (__popc(mask) < TURN::TRI &&
+                !(exhausted && mask && !__any_sync(HP_FULL_MASK, (unsigned)node < (unsigned)SENTINEL)))
+                break;
         }
     }
 }

@@ -47,18 +47,21 @@ __device__ __forceinline__ float safe_rcp(float d) {
 // arithmetic and tie rule, so the hits equal the binary layout's.
 constexpr int TB1 = 128;
 constexpr int SST1 = 16;
-// Turns (k_trace_impl.cuh says what they are and what NODE decides: here too rays miss the
-// nearer of two near-tied hits as often at 3 or 4 as in the tracer before, 6 % more often
-// at 6 and 25 % at 12) and CTAs per SM. On a B200, the tracer before / NODE 1 / 3 / 12, 2 M bounce
-// rays in 1 M triangles, primary rays on a terrain and 4.2 M bounce rays on another: Quad 2.99 /
-// 2.55 / 2.24 / 2.15 ms, 0.65 / 0.58 / 0.54 / 0.53 and 3.11 / 2.65 / 2.39 / 2.31; Oct 3.71 / 3.37 /
-// 2.91 / 2.78, 0.74 / 0.75 / 0.67 / 0.62 and 3.95 / 3.51 / 3.14 / 3.05. FETCH 12: 1 to 2 % slower.
-// Visibility rays, where NODE is free: Quad 1.16 -> 0.96 ms, Oct 1.31 -> 1.15 for 1 M of them.
-// CTAs at 9 (56 registers): Quad equal, Oct 12 % slower.
+// Turns (k_trace_impl.cuh says what they are and what NODE decides: here rays miss the nearer of
+// two near-tied hits 304 times in the Quad and 260 in the Oct layout of the same frames and rays
+// with every lane in loops of its own, 329 and 290 times at 4, about 15 % more often at 6 and
+// 33 % at 12) and CTAs per SM. On a B200, every lane in loops of its own ->
+// now, 2 M bounce rays in 1 M triangles, primary rays on a terrain and 4.2 M bounce rays on
+// another: Quad 2.99 -> 2.17 ms, 0.65 -> 0.53 and 3.11 -> 2.29; Oct 3.71 -> 2.82, 0.74 -> 0.61 and
+// 3.95 -> 3.00. NODE 1: Quad 2.55, 0.58 and 2.65, Oct 3.37, 0.75 and 3.51. FETCH 12: 1 to 2 %
+// slower. Visibility rays, where NODE is free: Quad 1.16 -> 0.96 ms, Oct 1.31 -> 1.18 for 1 M of
+// them. Oct loses where there is little to do: 100,000 rays on a terrain of 1,000 triangles 91 -> 101
+// us, 8,192 triangles equal. CTAs at 9 (56 registers): Quad equal, Oct 12 % slower. Stack entries
+// without distances: Quad 1 to 2 % slower, Oct 1 to 8 %.
 constexpr int CTAS1 = 8;
 template <bool ANY_HIT>
 struct turns1 {
-    static constexpr int NODE = ANY_HIT ? 12 : 3, TRI = 4, FETCH = ANY_HIT ? 12 : 8;
+    static constexpr int NODE = ANY_HIT ? 12 : 4, TRI = 4, FETCH = ANY_HIT ? 12 : 8;
 };
 constexpr int SENT1 = 0x76543210;
 template <int N> struct wide1_cfg;
@@ -74,12 +77,12 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
                                                    const int32_t* __restrict__ order) {
     using TURN = turns1<ANY_HIT>;
     constexpr int STACK = wide1_cfg<N>::STACK, LST = STACK - SST1;
-    __shared__ int s_stack[SST1 * TB1];
-    int* sstack = s_stack + threadIdx.x;
-    // Entries past the shared part. Left uninitialised: sp
+    __shared__ int2 s_stack[SST1 * TB1];
+    int2* sstack = s_stack + threadIdx.x;
+    // Entries (child, entry distance) past the shared part. Left uninitialised: sp
     // counts the pushes that were stored (an overflowing push is dropped and
     // reported), so a pop reads only entries a push wrote.
-    int lstack[LST];
+    int2 lstack[LST];
     const int lane = threadIdx.x & 31;
 
     float ox = 0, oy = 0, oz = 0, tmin = 0, dx = 0, dy = 0, dz = 0;
@@ -91,17 +94,25 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
     int leaf = 0;              // postponed leaf (~index) whose range is not loaded yet, 0 when none
     int tri = 0, tri_end = 0;  // triangles of the postponed leaf still to test
     bool exhausted = false;    // warp-uniform: the counter has run past the rays
+    // An interior node beyond the hit found since is dropped: a child's slab values lie between
+    // its parent's, rounded or not, so all of its boxes would be missed. (Statistics count
+    // such visits, as the reference does.) A leaf is kept: its triangles are tested whatever
+    // its box, whose rounded slabs may lie beyond a nearer or equal hit in it.
     auto pop = [&]() {
-        if (sp == 0) {
-            node = SENT1;
-        } else {
+        node = SENT1;
+        while (sp > 0) {
             --sp;
-            node = sp < SST1 ? sstack[sp * TB1] : lstack[sp - SST1];
+            const int2 e = sp < SST1 ? sstack[sp * TB1] : lstack[sp - SST1];
+            if (STATS || e.x < 0 || !(__int_as_float(e.y) > hit_t)) {
+                node = e.x;
+                break;
+            }
         }
     };
-    auto push = [&](int v) {
-        if (sp < SST1) sstack[sp * TB1] = v;
-        else if (sp < STACK) lstack[sp - SST1] = v;
+    auto push = [&](int v, uint32_t key) {
+        const int2 e = make_int2(v, __float_as_int(hp_ord2f(key)));
+        if (sp < SST1) sstack[sp * TB1] = e;
+        else if (sp < STACK) lstack[sp - SST1] = e;
         else { hp_report(err, HP_DEV_STACK_OVERFLOW, (int)ray); --sp; }
         ++sp;
     };
@@ -205,7 +216,7 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
                     } else {
 #pragma unroll
                         for (int i = N - 1; i >= 1; --i)
-                            if (key[i] != 0xFFFFFFFFu) push(ref[i]);
+                            if (key[i] != 0xFFFFFFFFu) push(ref[i], key[i]);
                         node = ref[0];
                     }
                     if (node < 0 && leaf >= 0 && tri >= tri_end) {  // the first leaf is postponed
@@ -275,7 +286,9 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
             }
             pend = node < 0 || leaf < 0 || tri < tri_end;
             mask = __ballot_sync(HP_FULL_MASK, pend);
-            if (__popc(mask) < TURN::TRI) break;
+            if (__popc(mask) < TURN::TRI &&
+                !(exhausted && mask && !__any_sync(HP_FULL_MASK, (unsigned)node < (unsigned)SENT1)))
+                break;
         }
     }
 }

@@ -102,9 +102,10 @@ hp_status hp_sort_check_launch(hp_ctx* ctx, const void* keys_out, int64_t n, int
 // Launch of a kernel that begins with hp_after_previous() (hp_device.cuh): its CTAs
 // may be placed while the kernel before it on the stream drains, and wait there, so
 // that a chain of small kernels does not pay a launch's latency each (a build of 5,003
-// triangles on a B200 116 -> 105 us). Only grids that the GPU holds at once: larger ones
-// hide a launch anyway, and chained, the LBVH's of 16.8 M triangles (65,537 CTAs and
-// more) took 5.10 ms together instead of 4.21.
+// triangles on a B200 116 -> 105 us). Only small grids: large ones hide a launch anyway, and
+// chained, the LBVH's of 16.8 M triangles (65,537 CTAs and more) took 5.10 ms together instead of
+// 4.21. CHAIN_MAX_GRID is where it was tried, not what the GPU holds at once (a CTA of the
+// climb takes a quarter of an SM; its CTAs past the first 592 are placed as others end).
 constexpr unsigned CHAIN_MAX_GRID = 1024;
 template <typename... P, typename... A>
 cudaError_t hp_launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,

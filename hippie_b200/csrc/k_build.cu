@@ -801,7 +801,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         k_init_build<<<hp_div_up(plan.passes * 256, TB), TB, 0, s>>>(info, hist, plan.passes * 256, nullptr, nullptr, 0,
                                                                      nullptr);
         HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-                                            info->box_ord, err, woop_src);
+                 info->box_ord, err, woop_src);
         hp_count_launch(2);
         hp_mark(ctx, s, "boxes");
         HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
@@ -835,7 +835,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         k_init_build<<<hp_div_up(plan.passes * 256, TB), TB, 0, s>>>(info, hist, plan.passes * 256, nullptr, nullptr, 0,
                                                                      nullptr);
         HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-                                            info->box_ord, err, nullptr);
+                 info->box_ord, err, nullptr);
         hp_count_launch(2);
         hp_mark(ctx, s, "boxes");
         HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
@@ -896,7 +896,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
     k_init_build<<<std::max(hp_div_up(plan.passes * 256, TB), grid_red), TB, 0, s>>>(
         info, hist, plan.passes * 256, counters, max_hi, n, frontier_count);
     HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-                                        info->box_ord, err, nullptr);
+             info->box_ord, err, nullptr);
     hp_count_launch(2);
     hp_mark(ctx, s, "boxes");
     HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
@@ -906,7 +906,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
     hp_sort_args sa{keys, nullptr, skeys, out->tri_idx, sort_scratch, hist, true, err, ctx};
     HP_TRY(hp_sort_run(plan, sa, s));
     HP_CHAIN(k_leaves, grid_n, TB, 0, s, (int)n, out->tri_idx, m->vertices, m->num_vertices, m->triangles, nbmin,
-                                   nbmax, out->woop, p->ci, p->adaptive_leaf, err);
+             nbmax, out->woop, p->ci, p->adaptive_leaf, err);
     hp_count_launch();
     hp_mark(ctx, s, "leaves");
     {
@@ -922,7 +922,8 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         if (n <= FRONT_CAP)
             HP_CHAIN((k_climb_frontier<K, true>), 1, FRONT_BLOCK, 0, s, A, skeys);
         else
-            HP_CHAIN((k_climb_frontier<K, false>), std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s, A, skeys);
+            HP_CHAIN((k_climb_frontier<K, false>), std::min<int64_t>(hp_div_up(n, TB), ctx->sm_count * 8), TB, 0, s, A,
+                     skeys);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
     }
@@ -947,22 +948,22 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         W.tris = m->triangles;
         HP_TRY(hp_wide_collapse(ctx, W, out, wide_scratch, s));
     } else {
-    if (n <= SC_CAP) {
-        HP_CUDA(cudaFuncSetAttribute(k_collapse_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC_SMEM));
-        HP_CHAIN(k_collapse_small, 1, SC_BLOCK, SC_SMEM, s, (int)n, left, range, state, max_hi, reach, rank_int, rank_leaf,
-                                                     &info->num_interior);
-    } else {
-        hp_scan_max_excl(max_hi, n, reach, scan_a, err, s);
-        k_collapse_flags<<<hp_div_up(nn, TB), TB, 0, s>>>((int)n, left, range, state, max_hi, reach,
-                                                         flag_int, flag_leaf);
-        hp_scan2_sum(flag_int, n - 1, flag_leaf, n, rank_int, rank_leaf, &info->num_interior, scan_b, err, s);
-    }
-    emit_ctx e{(int)n, left, right, parent, range, state, rank_int, rank_leaf, nbmin, nbmax};
-    HP_CHAIN(k_emit, hp_div_up(nn, TB), TB, 0, s, e, max_hi, reach, info, out->nodes,
-                                            (int)std::max<int64_t>(2 * out->capacity - 1, 3), err);
-    HP_CUDA(cudaGetLastError());
-    hp_count_launch(2);
-    hp_mark(ctx, s, "collapse");
+        if (n <= SC_CAP) {
+            HP_CUDA(cudaFuncSetAttribute(k_collapse_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SC_SMEM));
+            HP_CHAIN(k_collapse_small, 1, SC_BLOCK, SC_SMEM, s, (int)n, left, range, state, max_hi, reach, rank_int,
+                     rank_leaf, &info->num_interior);
+        } else {
+            hp_scan_max_excl(max_hi, n, reach, scan_a, err, s);
+            k_collapse_flags<<<hp_div_up(nn, TB), TB, 0, s>>>((int)n, left, range, state, max_hi, reach, flag_int,
+                                                              flag_leaf);
+            hp_scan2_sum(flag_int, n - 1, flag_leaf, n, rank_int, rank_leaf, &info->num_interior, scan_b, err, s);
+        }
+        emit_ctx e{(int)n, left, right, parent, range, state, rank_int, rank_leaf, nbmin, nbmax};
+        HP_CHAIN(k_emit, hp_div_up(nn, TB), TB, 0, s, e, max_hi, reach, info, out->nodes,
+                 (int)std::max<int64_t>(2 * out->capacity - 1, 3), err);
+        HP_CUDA(cudaGetLastError());
+        hp_count_launch(2);
+        hp_mark(ctx, s, "collapse");
     }
 
     if (taps) {

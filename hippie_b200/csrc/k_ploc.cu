@@ -293,10 +293,10 @@ __device__ void nn_tile(const ploc_args& A, const int* __restrict__ cl, int N, i
             bi[q] = base - r + k;
         }
     };
-#define HP_PLOC_CAND(k)                                                             \
-    const int w_ = win<R>::at4(k);                                                          \
+#define HP_PLOC_CAND(k)            \
+    const int w_ = win<R>::at4(k); \
     const float cx = smnx[w_], cy = smny[w_], cz = smnz[w_], dx = smxx[w_], dy = smxy[w_], dz = smxz[w_]
-    if (B == 1 || r < 4) {
+    if (r < 4) {
         for (int k = l0; k <= l0 + (B - 1) + 2 * r; ++k) {
             HP_PLOC_CAND(k);
 #pragma unroll
@@ -423,8 +423,8 @@ __device__ void nn_halo(const ploc_args& A, const int* __restrict__ cl, int N, i
 }
 
 // One merge tile of at most ITEMS*LPB clusters: flags, prefix sums (tile + look-back),
-// new nodes, compaction. FUSED tiles (ITEMS 1) find their neighbours first;
-// the others read the neighbour phase's results.
+// new nodes, compaction. The tile finds its neighbours first: ITEMS 1 with nn_halo, the
+// others with nn_tile.
 template <int R, int ITEMS>
 __device__ void merge_tile(const ploc_args& A, const int* __restrict__ cl_in, int* __restrict__ cl_out,
                            int N, int r, int it, unsigned tile, int TSZ, unsigned long long* status, float* s_win,
@@ -432,7 +432,7 @@ __device__ void merge_tile(const ploc_args& A, const int* __restrict__ cl_in, in
     const unsigned tag = (unsigned)(it % 15) + 1u;
     const int tbase = (int)tile * TSZ;
     __syncthreads();  // the previous tile's shared memory is free
-    if (ITEMS == 1) nn_halo<R>(A, cl_in, N, r, tbase, TSZ, s_win, s_nn);
+    if constexpr (ITEMS == 1) nn_halo<R>(A, cl_in, N, r, tbase, TSZ, s_win, s_nn);
     else nn_tile<R, ITEMS>(A, cl_in, N, r, tbase - r, s_win, s_nn);  // TSZ + 2r <= ITEMS * LPB clusters
     const int nlo = tbase - r;  // cluster of s_nn[0]
     auto nn_of = [&](int c) { return s_nn[c - nlo]; };
@@ -748,7 +748,7 @@ __device__ __forceinline__ bool barrier_of(unsigned* bar, unsigned count, unsign
 
 template <int R>
 __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
-    extern __shared__ float s_win[];
+    extern __shared__ __align__(16) float s_win[];  // merge_tile keeps pairs in it
     int* s_nn = reinterpret_cast<int*>(s_win + 6 * win<R>::S);
     __shared__ int s_wa[LPB / 32 + 1], s_wb[LPB / 32 + 1];
     __shared__ unsigned s_pref[2];
@@ -806,7 +806,8 @@ __global__ void __launch_bounds__(LPB, 2) k_ploc_loop(ploc_args A) {
         if ((int)blockIdx.x >= count) return;
         const int* cl_in = (it & 1) ? A.cl1 : A.cl0;
         int* cl_out = (it & 1) ? A.cl0 : A.cl1;
-        small_iteration<R>(A, cl_in, cl_out, N, radius_at(A, it), it, tsz, S, s_win, s_nn, s_wa, s_wb, s_pref, &s_small);
+        small_iteration<R>(A, cl_in, cl_out, N, radius_at(A, it), it, tsz, S, s_win, s_nn, s_wa, s_wb, s_pref,
+                           &s_small);
         N = s_small.n;
         if (!s_small.ok) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -1005,8 +1005,7 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
         constexpr size_t one_smem = sort_one_smem<K>();
         HP_CUDA(cudaFuncSetAttribute(k_sort_one<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one_smem));
         HP_CHAIN(k_sort_one<K>, 1, ONE_BLOCK, one_smem, stream, reinterpret_cast<const K*>(a.keys_in), a.vals_in,
-                                                          reinterpret_cast<K*>(a.keys_out), a.vals_out, (int)plan.n,
-                                                          plan.bits);
+                 reinterpret_cast<K*>(a.keys_out), a.vals_out, (int)plan.n, plan.bits);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(a.ctx, stream, "sort_pass");
@@ -1053,9 +1052,9 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
             for (int d = 0; d < SEG_TOP; ++d) {  // in -> A -> B -> A
                 K* dk = (d & 1) ? kB : kA;
                 int32_t* dv = (d & 1) ? vB : vA;
-                HP_CHAIN((k_onesweep<K, BLOCK, ITEMS>), plan.tiles, BLOCK, smem, stream, 
-                    src_k, src_v, dk, dv, n, s0 + 8 * d, 0xffu, a.hist + 256 * d,
-                    status + (size_t)d * plan.tiles * 256, counters + d, a.status, sl);
+                HP_CHAIN((k_onesweep<K, BLOCK, ITEMS>), plan.tiles, BLOCK, smem, stream, src_k, src_v, dk, dv, n,
+                         s0 + 8 * d, 0xffu, a.hist + 256 * d, status + (size_t)d * plan.tiles * 256, counters + d,
+                         a.status, sl);
                 HP_CUDA(cudaGetLastError());
                 hp_count_launch();
                 hp_mark(a.ctx, stream, "sort_pass");
@@ -1112,10 +1111,9 @@ hp_status sort_run_t(const hp_sort_plan& plan, const hp_sort_args& a, cudaStream
         }
         int shift = 8 * p;
         int w = std::min(8, plan.bits - shift);
-        HP_CHAIN((k_onesweep<K, BLOCK, ITEMS>), plan.tiles, BLOCK, smem, stream, 
-            kin, vin, kout, vout, n, shift, (1u << w) - 1u, a.hist + 256 * p,
-            status + (size_t)p * plan.tiles * 256, counters + p, a.status,
-            a.ctx ? a.ctx->sort_spin_limit : LOOKBACK_SPIN_LIMIT);
+        HP_CHAIN((k_onesweep<K, BLOCK, ITEMS>), plan.tiles, BLOCK, smem, stream, kin, vin, kout, vout, n, shift,
+                 (1u << w) - 1u, a.hist + 256 * p, status + (size_t)p * plan.tiles * 256, counters + p, a.status,
+                 a.ctx ? a.ctx->sort_spin_limit : LOOKBACK_SPIN_LIMIT);
         HP_CUDA(cudaGetLastError());
         hp_count_launch();
         hp_mark(a.ctx, stream, "sort_pass");

@@ -151,9 +151,11 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
                 } else {
                     // u and v of the closest hit once more, by the steps of its test
                     const float4 v1 = __ldg(woop + 3 * (int64_t)r.hit + 1), v2 = __ldg(woop + 3 * (int64_t)r.hit + 2);
-                    const float hu = __fmaf_rn(r.hit_t, __fmaf_rn(r.dz, v1.z, __fmaf_rn(r.dy, v1.y, __fmul_rn(r.dx, v1.x))),
+                    const float hu = __fmaf_rn(
+                        r.hit_t, __fmaf_rn(r.dz, v1.z, __fmaf_rn(r.dy, v1.y, __fmul_rn(r.dx, v1.x))),
                         __fmaf_rn(r.oz, v1.z, __fmaf_rn(r.oy, v1.y, __fmaf_rn(r.ox, v1.x, v1.w))));
-                    const float hv = __fmaf_rn(r.hit_t, __fmaf_rn(r.dz, v2.z, __fmaf_rn(r.dx, v2.x, __fmul_rn(r.dy, v2.y))),
+                    const float hv = __fmaf_rn(
+                        r.hit_t, __fmaf_rn(r.dz, v2.z, __fmaf_rn(r.dx, v2.x, __fmul_rn(r.dy, v2.y))),
                         __fmaf_rn(r.oz, v2.z, __fmaf_rn(r.oy, v2.y, __fmaf_rn(r.ox, v2.x, v2.w))));
                     results[ray] = make_int4(__ldg(tri_idx + r.hit), __float_as_int(r.hit_t),
                                              __float_as_int(hu), __float_as_int(hv));

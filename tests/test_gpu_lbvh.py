@@ -190,3 +190,18 @@ def test_refit_names_the_triangle(ctx):
     with pytest.raises(hp.HPError) as ei:
         ctx.check()
     assert ei.value.status == 5 and "(info 10)" in str(ei.value)
+
+
+@pytest.mark.parametrize("bits", [30, 60])
+@pytest.mark.parametrize("n", [511, 512, 513, 1024, 8191, 8192, 8193])
+def test_climb_and_collapse_edges(ctx, bits, n):
+    """Around the triangles that a CTA of the climb owns (512) and the largest mesh whose
+    frontier is climbed and whose collapse is scanned by one CTA (8,192), with both key widths."""
+    v, t = hp.gen.clustered_mesh(90 + n, n, clusters=7, sigma=0.05, half_extent=0.02)
+    bvh, taps, V, T = build_with_taps(ctx, v, t, hp.BuildParams(morton_bits=bits))
+    ctx.check()
+    ref = oracle.build_lbvh(v, t, bits=bits, scale=np.array(bvh.c.morton_scale, np.float32))
+    nodes, woop, tri = bvh.download()
+    np.testing.assert_array_equal(nodes, ref["nodes"])
+    np.testing.assert_array_equal(tri, ref["tri_idx"])
+    assert bvh.validate(V, T)

@@ -160,6 +160,18 @@ struct tri_verts {
     float x0, y0, z0, x1, y1, z1, x2, y2, z2;
 };
 
+// Whether two triangles have a vertex position in common, whatever their indices.
+__device__ __forceinline__ bool share_vertex(const tri_verts& a, const tri_verts& b) {
+    const float ax[3] = {a.x0, a.x1, a.x2}, ay[3] = {a.y0, a.y1, a.y2}, az[3] = {a.z0, a.z1, a.z2};
+    const float bx[3] = {b.x0, b.x1, b.x2}, by[3] = {b.y0, b.y1, b.y2}, bz[3] = {b.z0, b.z1, b.z2};
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) any = any || (ax[i] == bx[j] && ay[i] == by[j] && az[i] == bz[j]);
+    return any;
+}
+
 // A vertex index out of range is reported with itself, or, for NAME_TRI, with the triangle.
 template <bool NAME_TRI = false>
 __device__ __forceinline__ tri_verts load_tri(const float* __restrict__ v, int64_t nv,

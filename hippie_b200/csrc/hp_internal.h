@@ -30,7 +30,8 @@ struct hp_bvh_info {
     int32_t num_leaf;
     uint32_t box_ord[6];    // scene box as order-preserving uints (min xyz, max xyz)
     float scale[3];         // Morton scale actually used
-    int32_t pad;
+    int32_t lone;           // 1: no triangle looked at has a vertex in common with the next one; 0: one has,
+                            // or nobody looked (the tracers' turns, k_trace_impl.cuh)
 };
 
 struct hp_bvh_impl {
@@ -299,6 +300,7 @@ struct hp_batch_seg {
     int32_t tri_off;
     int64_t node_off;
     int64_t ray_off;
+    int32_t lone;             // hp_bvh_info::lone, beside what a ray of the mesh reads
 };
 struct hp_batch_trace_args {
     const float* rays;
@@ -325,5 +327,13 @@ hp_status hp_trace_launch(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, con
 hp_status hp_adjoint_launch(hp_ctx* ctx, const hp_mesh* m, const float* rays,
                             const int32_t* results, const float* dl_dtuv, int64_t num_rays,
                             float* dl_dvertices, cudaStream_t stream);
+
+// Of every mask + 1 triangles a build compares one with the next (hp_bvh_info::lone): all of a
+// small mesh, 4,096 to 8,191 of a larger one, which costs its box kernel nothing that shows.
+__host__ __device__ inline int hp_look_mask(int64_t n) {
+    int every = 1;
+    while (n / every >= 8192) every *= 2;
+    return every - 1;
+}
 
 inline int hp_div_up(int64_t a, int64_t b) { return int((a + b - 1) / b); }

@@ -43,7 +43,7 @@ __device__ __forceinline__ int seg_of(const int32_t* __restrict__ off, int num_s
 }
 
 struct bargs {
-    const hp_batch_seg* seg;
+    hp_batch_seg* seg;
     const int32_t* tri_off;  // [M + 1]
     int M;
     int64_t N;
@@ -87,6 +87,7 @@ __global__ void k_b_init(bargs B, int hist_words) {
         for (int k = 0; k < 6; ++k) B.info[i].box_ord[k] = (k < 3) ? 0xffffffffu : 0u;
         B.info[i].num_interior = 0;
         B.info[i].num_leaf = 0;
+        B.info[i].lone = B.seg[i].lone = 1;
     }
 }
 
@@ -120,7 +121,11 @@ __global__ void __launch_bounds__(TB) k_b_boxes(bargs B) {
     uint32_t o[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     if (m >= 0) {
         const hp_batch_seg sg = B.seg[m];
-        const tri_verts t = load_tri(sg.verts, sg.nv, sg.tris, g - sg.tri_off, B.err);
+        const int64_t i = g - sg.tri_off;
+        const tri_verts t = load_tri(sg.verts, sg.nv, sg.tris, i, B.err);
+        if (((int)i & hp_look_mask(sg.n)) == 0 && i + 1 < sg.n &&
+            share_vertex(t, load_tri(sg.verts, sg.nv, sg.tris, i + 1, B.err)))
+            B.info[m].lone = B.seg[m].lone = 0;
         const float ax = fminf(fminf(t.x0, t.x1), t.x2), ay = fminf(fminf(t.y0, t.y1), t.y2),
                     az = fminf(fminf(t.z0, t.z1), t.z2);
         const float bx = fmaxf(fmaxf(t.x0, t.x1), t.x2), by = fmaxf(fmaxf(t.y0, t.y1), t.y2),

@@ -41,18 +41,23 @@ constexpr int TB = 256;
 
 // Per-triangle boxes (setupBoxes) and the scene box as their union
 // (SceneLoader.cpp:144-153 computes it over triangle boxes at load time).
+// Of every look + 1 triangles one is compared with the next in the mesh's order: triangles
+// that share vertices, whether through an index or as equal positions, are as a rule
+// neighbours there, and one pair found is enough (hp_bvh_info::lone).
 // woop (or null): the Woop rows of every triangle, in scene order, computed
 // here from the vertices the boxes read anyway (the collapse then gathers one
 // 48-byte record per reference instead of the triangle and its vertices).
 __global__ void __launch_bounds__(TB) k_tri_boxes(const float* __restrict__ verts, int64_t nv,
                                                   const int32_t* __restrict__ tris, int64_t n,
                                                   float4* __restrict__ bmin, float4* __restrict__ bmax,
-                                                  uint32_t* box_ord, int* err, float4* __restrict__ woop) {
+                                                  hp_bvh_info* info, int look, int* err, float4* __restrict__ woop) {
     hp_after_previous();
+    uint32_t* box_ord = info->box_ord;
     float mn[3] = {HP_MAX_FLOAT, HP_MAX_FLOAT, HP_MAX_FLOAT};
     float mx[3] = {-HP_MAX_FLOAT, -HP_MAX_FLOAT, -HP_MAX_FLOAT};
     for (int64_t i = blockIdx.x * (int64_t)TB + threadIdx.x; i < n; i += (int64_t)gridDim.x * TB) {
         tri_verts t = load_tri(verts, nv, tris, i, err);
+        if (((int)i & look) == 0 && i + 1 < n && share_vertex(t, load_tri(verts, nv, tris, i + 1, err))) info->lone = 0;
         float ax = fminf(fminf(t.x0, t.x1), t.x2), ay = fminf(fminf(t.y0, t.y1), t.y2),
               az = fminf(fminf(t.z0, t.z1), t.z2);
         float bx = fmaxf(fmaxf(t.x0, t.x1), t.x2), by = fmaxf(fmaxf(t.y0, t.y1), t.y2),
@@ -102,6 +107,7 @@ __global__ void k_init_build(hp_bvh_info* info, uint32_t* hist, int hist_words, 
     if (i0 == 0) {
         info->num_interior = 0;
         info->num_leaf = 0;
+        info->lone = 1;
         if (frontier_count) *frontier_count = 0;
     }
     for (int64_t i = i0; i < words; i += (int64_t)gridDim.x * blockDim.x) {
@@ -801,7 +807,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         k_init_build<<<hp_div_up(plan.passes * 256, TB), TB, 0, s>>>(info, hist, plan.passes * 256, nullptr, nullptr, 0,
                                                                      nullptr);
         HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-                 info->box_ord, err, woop_src);
+                 info, hp_look_mask(n), err, woop_src);
         hp_count_launch(2);
         hp_mark(ctx, s, "boxes");
         HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
@@ -835,7 +841,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
         k_init_build<<<hp_div_up(plan.passes * 256, TB), TB, 0, s>>>(info, hist, plan.passes * 256, nullptr, nullptr, 0,
                                                                      nullptr);
         HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-                 info->box_ord, err, nullptr);
+                 info, hp_look_mask(n), err, nullptr);
         hp_count_launch(2);
         hp_mark(ctx, s, "boxes");
         HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);
@@ -896,7 +902,7 @@ hp_status lbvh_t(hp_ctx* ctx, const hp_mesh* m, const hp_build_params* p, hp_bvh
     k_init_build<<<std::max(hp_div_up(plan.passes * 256, TB), grid_red), TB, 0, s>>>(
         info, hist, plan.passes * 256, counters, max_hi, n, frontier_count);
     HP_CHAIN(k_tri_boxes, grid_red, TB, 0, s, m->vertices, m->num_vertices, m->triangles, n, tbmin, tbmax,
-             info->box_ord, err, nullptr);
+             info, hp_look_mask(n), err, nullptr);
     hp_count_launch(2);
     hp_mark(ctx, s, "boxes");
     HP_CHAIN(k_morton<K>, grid_mor, TB, 0, s, tbmin, tbmax, n, info, bits, h_shift, h_count, keys, hist);

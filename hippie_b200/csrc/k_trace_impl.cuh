@@ -62,10 +62,10 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 // decided by ballots:
 //   * nodes: every lane at an interior node does one. The first leaf that a lane
 //     meets is postponed and the lane goes on from its stack; at a second one it
-//     waits. The turn ends when fewer than NODE lanes have an interior node and no
+//     waits. The turn ends when fewer than LEAST lanes have an interior node and no
 //     postponed leaf, so that a hit is found, and shortens the ray, soon;
 //   * triangles: every lane with a postponed leaf tests one triangle, until fewer
-//     than TRI lanes have one (or none, once the rays have run out and no lane has a
+//     than LEAST lanes have one (or none, once the rays have run out and no lane has a
 //     node to go on with);
 //   * new rays: once FETCH lanes are without work.
 // A stack entry is the child alone. With its entry distance beside it, entries beyond
@@ -73,25 +73,30 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 // ms with it, 19.5 without), and for a leaf it is wrong: a leaf's triangles are tested
 // whatever its box, whose rounded slabs may lie beyond a nearer or equal hit in it.
 //
-// NODE decides more than time. Of two hits nearer to each other than a slab's rounding
+// LEAST decides more than time. Of two hits nearer to each other than a slab's rounding
 // (on the edge that two triangles share) a ray misses the nearer one if the other was
 // tested before the nearer one's boxes were, and short node turns test sooner. Against
 // a tracer that gives boxes a slack, rays that missed the nearer hit in 360 frames of
 // 2.07 M primary rays and in 360 times 4.2 M sphere rays on terrains: every lane in
-// loops of its own, as in the reference, 122 and 217; NODE 1: 122 and 223; 2: 132, 228;
-// 3: 126, 232; 4: 128, 235; 16: 151, 280. Up to 4 is as good as it was. A visibility
-// ray has no nearest hit to miss.
+// loops of its own, as in the reference, 122 and 217; LEAST 1: 122 and 223; 2: 132, 228;
+// 3: 126, 232; 4: 128, 235; 16: 151, 280. Up to 4 that is as good, but it is other rays: of
+// runs over the 4.2 M, 5 % differ in a ray between two runs of either order (which rays share
+// a warp is decided as they come), 7 % between loops and 1, 20 % between loops and 4. So where
+// triangles share vertices leaves are tested late (LEAST 1), which returns what has always
+// been returned, and sooner elsewhere, where such pairs of hits do not come up. A build looks
+// whether they do (hp_bvh_info::lone); a batch's warp goes by the meshes whose rays it has.
+// A visibility ray has no nearest hit to miss.
 //
-// Measured on a B200, every lane in loops of its own -> now: 16.8 M bounce rays 28.4 ->
-// 19.1 ms, 43 M rays over 256 meshes 42.4 -> 28.0, 4 M sorted rays 3.86 -> 2.92, 2.07 M primary
-// rays 0.77 -> 0.56, 4.2 M downward rays 2.28 -> 2.22, 4.2 M bounce rays on a terrain 3.12 -> 2.29,
-// 4.2 M rays in 33.5 M triangles 22.2 -> 22.7. Bounce, sorted and primary rays at NODE 1: 22.9,
-// 3.23 and 0.75; 2: 20.9, 3.06, 0.66; 16: 18.4, 3.00, 0.57. FETCH 12 instead of 16: bounce rays
-// 3 % faster, downward ones 6 % slower; 20: the other way round. TRI 1 to 6 differ by 2 % either way.
+// Measured on a B200, every lane in loops of its own -> now: 16.8 M bounce rays 28.4 -> 19.1 ms,
+// 43 M rays over 256 meshes 42.4 -> 28.0, 4 M sorted rays 3.86 -> 2.91, 4.2 M rays in 33.5 M
+// triangles 22.2 -> 22.7; late, 2.07 M primary rays 0.77 -> 0.69, 4.2 M downward rays 2.28 -> 2.13,
+// 4.2 M bounce rays on a terrain 3.12 -> 2.63 (at LEAST 4: 0.55, 2.22 and 2.28). Bounce, sorted
+// and batch rays at 1: 22.9, 3.23 and 32; at 16: 18.4, 3.00 and 27.3. FETCH 12 instead of 16:
+// bounce rays 3 % faster, downward ones 6 % slower; 20: the other way round.
 // Packed FP32 for the slabs and 32-byte loads of two Woop rows were slower or no faster.
 template <bool ANY_HIT>
 struct turns {
-    static constexpr int NODE = ANY_HIT ? 16 : 4, TRI = ANY_HIT ? 6 : 2, FETCH = 16;
+    static constexpr int LEAST = ANY_HIT ? 12 : 4, FETCH = 16;
 };
 // CTAs per SM. Closest hits: 12 (40 registers, 4 bytes of spills read back) instead of 10
 // shorten bounce rays by 8 % and downward ones by 3 %, and cost rays in 33.5 M triangles 3 %.
@@ -101,17 +106,16 @@ constexpr int trace_ctas(bool any_hit, bool batch) { return batch ? 8 : any_hit 
 
 // BATCH: rays of many meshes in one launch; ray g belongs to the segment whose
 // ray range holds it, and the lane traverses that mesh's BVH.
-template <bool ANY_HIT, bool STATS, bool BATCH, int SST>
-__global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_trace(
+// LATE: leaves are tested late (a batch's warp decides for itself).
+template <bool ANY_HIT, bool STATS, bool BATCH, int SST, bool LATE>
+__device__ __forceinline__ void trace_rays(
     const float4* __restrict__ rays, int64_t num_rays, int4* __restrict__ results,
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
-    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order) {
+    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, int* sstack) {
     constexpr int LST = STACK - SST;
     using TURN = turns<ANY_HIT>;
-    __shared__ int s_stack[SST * TRACE_BLOCK];
-    int* sstack = s_stack + threadIdx.x;
     int lstack[LST];
     const int lane = threadIdx.x & 31;
 
@@ -125,6 +129,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
     int sp = 0;
     int steps = 0;           // node + leaf visits of the current ray (bounded)
     bool exhausted = false;  // warp-uniform: the counter has run past the rays
+    bool lone = true;        // of the lane's mesh (BATCH)
+    int least = LATE ? 1 : TURN::LEAST;  // warp-uniform
     const float4* nodes = nodes_all;
     const float4* woop = woop_all;
     const int32_t* tri_idx = tri_all;
@@ -191,6 +197,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
                     node = 0;
                     if (BATCH) {
                         const hp_batch_seg& g = segs[seg_search(ray_off, num_segs, id)];
+                        lone = g.lone != 0;
                         nodes = nodes_all + 4 * g.node_off;
                         woop = woop_all + 3 * (int64_t)g.tri_off;
                         tri_idx = tri_all + g.tri_off;
@@ -200,6 +207,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
                     }
                 }
             }
+            if (BATCH && !ANY_HIT) least = __any_sync(HP_FULL_MASK, ray >= 0 && !lone) ? 1 : TURN::LEAST;
         }
 
         // Interior nodes: one per lane and round.
@@ -258,7 +266,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
             }
             go = (unsigned)node < (unsigned)SENTINEL;
             mask = __ballot_sync(HP_FULL_MASK, go && leaf >= 0 && tri >= tri_end);
-            if (__popc(mask) < TURN::NODE) break;
+            if (__popc(mask) < least) break;
         }
 
         // Leaves: one triangle per lane and round.
@@ -326,11 +334,33 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
             }
             pend = node < 0 || leaf < 0 || tri < tri_end;
             mask = __ballot_sync(HP_FULL_MASK, pend);
-            if (__popc(mask) < TURN::TRI &&
+            if (__popc(mask) < least &&
                 !(exhausted && mask && !__any_sync(HP_FULL_MASK, (unsigned)node < (unsigned)SENTINEL)))
                 break;
         }
     }
+}
+
+template <bool ANY_HIT, bool STATS, bool BATCH, int SST>
+__global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_trace(
+    const float4* __restrict__ rays, int64_t num_rays, int4* __restrict__ results,
+    int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
+    const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
+    unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
+    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order,
+    const hp_bvh_info* __restrict__ info) {
+    __shared__ int s_stack[SST * TRACE_BLOCK];
+    int* sstack = s_stack + threadIdx.x;
+    // One body a kind of mesh: with one body and its limit in a register bounce rays take
+    // 20.0 ms, not 19.1.
+    if (!BATCH && !ANY_HIT && __ldg(&info->lone) == 0)
+        trace_rays<ANY_HIT, STATS, BATCH, SST, true>(rays, num_rays, results, stats, nodes_all, woop_all, tri_all,
+                                                     max_nodes_all, num_refs_all, ray_counter, err, segs, ray_off,
+                                                     num_segs, order, sstack);
+    else
+        trace_rays<ANY_HIT, STATS, BATCH, SST, false>(rays, num_rays, results, stats, nodes_all, woop_all, tri_all,
+                                                      max_nodes_all, num_refs_all, ray_counter, err, segs, ray_off,
+                                                      num_segs, order, sstack);
 }
 
 // Persistent grid: the tuned CTAs per SM, or as many as fit.
@@ -351,7 +381,7 @@ hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const floa
     k_trace<A, S, false, SST><<<trace_grid(ctx, per_sm, num_rays), TRACE_BLOCK, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const float4*>(b->nodes), b->woop, b->tri_idx,
-        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order);
+        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order, b->info);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

@@ -47,17 +47,15 @@ __device__ __forceinline__ float safe_rcp(float d) {
 // arithmetic and tie rule, so the hits equal the binary layout's.
 constexpr int TB1 = 128;
 constexpr int SST1 = 16;
-// Turns (k_trace_impl.cuh says what they are and what NODE decides: here rays miss the nearer of
-// two near-tied hits 304 times in the Quad and 260 in the Oct layout of the same frames and rays
-// with every lane in loops of its own, 329 and 290 times at 4, about 15 % more often at 6 and
-// 33 % at 12) and CTAs per SM. On a B200, every lane in loops of its own ->
-// now, 2 M bounce rays in 1 M triangles, primary rays on a terrain and 4.2 M bounce rays on
-// another: Quad 2.99 -> 2.17 ms, 0.65 -> 0.53 and 3.11 -> 2.29; Oct 3.71 -> 2.82, 0.74 -> 0.61 and
-// 3.95 -> 3.00. NODE 1: Quad 2.55, 0.58 and 2.65, Oct 3.37, 0.75 and 3.51. FETCH 12: 1 to 2 %
-// slower. Visibility rays, where NODE is free: Quad 1.16 -> 0.96 ms, Oct 1.31 -> 1.18 for 1 M of
-// them. Oct loses where there is little to do: 100,000 rays on a terrain of 1,000 triangles 91 -> 101
-// us, 8,192 triangles equal. CTAs at 9 (56 registers): Quad equal, Oct 12 % slower. Stack entries
-// without distances: Quad 1 to 2 % slower, Oct 1 to 8 %.
+// Turns (k_trace_impl.cuh says what they are, what LEAST decides and where it is 1; here NODE is
+// its part for nodes, and the triangles' limit hardly matters) and CTAs per SM. On a B200, every lane
+// in loops of its own -> now, 2 M bounce rays in 1 M triangles: Quad 2.99 -> 2.18 ms, Oct 3.71 -> 2.81
+// (at NODE 1 2.55 and 3.37, at 12 2.15 and 2.78); late, primary rays on a terrain and 4.2 M bounce
+// rays on another: Quad 0.65 -> 0.58 and 3.11 -> 2.65, Oct 0.74 -> 0.70 and 3.95 -> 3.49 (at NODE 4 0.53,
+// 2.29, 0.61 and 3.00). FETCH 12: 1 to 2 % slower. Visibility rays: Quad 1.16 -> 0.96 ms, Oct 1.31 ->
+// 1.18 for 1 M of them. Oct loses where there is little to do: 100,000 rays on a terrain of 1,000
+// triangles 91 -> 101 us, 8,192 triangles equal. CTAs at 9 (56 registers): Quad equal, Oct 12 %
+// slower. Stack entries without distances: Quad 1 to 2 % slower, Oct 1 to 8 %.
 constexpr int CTAS1 = 8;
 template <bool ANY_HIT>
 struct turns1 {
@@ -74,8 +72,10 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
                                                    const int4* __restrict__ nodes, const float4* __restrict__ woop,
                                                    const int32_t* __restrict__ tri_idx, int max_nodes, int num_refs,
                                                    unsigned long long* ray_counter, int* err,
-                                                   const int32_t* __restrict__ order) {
+                                                   const int32_t* __restrict__ order,
+                                                   const hp_bvh_info* __restrict__ info) {
     using TURN = turns1<ANY_HIT>;
+    const bool late = !ANY_HIT && __ldg(&info->lone) == 0;  // as in k_trace_impl.cuh
     constexpr int STACK = wide1_cfg<N>::STACK, LST = STACK - SST1;
     __shared__ int2 s_stack[SST1 * TB1];
     int2* sstack = s_stack + threadIdx.x;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
             }
             go = (unsigned)node < (unsigned)SENT1;
             mask = __ballot_sync(HP_FULL_MASK, go && leaf >= 0 && tri >= tri_end);
-            if (__popc(mask) < TURN::NODE) break;
+            if (__popc(mask) < (late ? 1 : TURN::NODE)) break;
         }
 
         // Leaves: one triangle per lane and round.
@@ -308,7 +308,7 @@ hp_status launch_wide_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const
     k_trace_wide1<N, A, S><<<(unsigned)grid, TB1, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const int4*>(b->nodes), b->woop, b->tri_idx, max_nodes,
-        (int)n_refs, counter, ctx->d_status, order);
+        (int)n_refs, counter, ctx->d_status, order, b->info);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

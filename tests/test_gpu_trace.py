@@ -212,3 +212,59 @@ def test_one_order_for_every_copy_of_a_mesh(ctx, layout):
         assert abs(visits[k] / visits["shared"] - 1) < 2e-3, visits
         # two hits on a shared edge, within a slab's rounding: a few in 1e8 rays
         assert int((hits[k][:, 0] != hits["shared"][:, 0]).sum()) <= 3, k
+
+
+@pytest.mark.parametrize("n,pair", [(3000, 2998), (8191, 17), (8192, 4096), (30000, 4)])
+def test_a_shared_vertex_is_found(ctx, n, pair):
+    """Triangles with vertices of their own are traced with short turns, those of a mesh in
+    which a triangle looked at (every one up to 8,191, of 30,000 every fourth) has a vertex
+    in common with the next late, as trees are that no build has looked over. The nodes
+    that rays visit tell which; the hits are the same."""
+    m = 1 << 19
+    v, t = hp.gen.uniform_mesh(n, n, 0.02)
+    w = v.copy()
+    w[3 * (pair + 1)] = w[3 * pair + 2]
+    R = dev(hp.gen.rays_sphere(4, m, np.concatenate([v.min(0), v.max(0)])))
+    p = hp.BuildParams(method="lbvh", morton_bits=60)
+
+    def visits(bvh):
+        res = torch.zeros((m, 4), dtype=torch.int32, device="cuda")
+        st = torch.zeros((m, 2), dtype=torch.int32, device="cuda")
+        ctx.trace(bvh, R, results=res, stats=st)
+        ctx.check()
+        return float(st[:, 0].double().sum()), res
+
+    for verts, late in ((v, False), (w, True)):
+        built = ctx.build(dev(verts), dev(t), p)
+        built.sync()
+        known = hp.BVH.reserve(ctx, n)
+        for to, frm in zip(known.arrays(), built.arrays()):
+            to.copy_(frm)
+        known.set_info(built.c.num_interior, built.c.num_leaf, built.c.scene_box, built.c.morton_scale)
+        (a, hits_a), (b, hits_b) = visits(built), visits(known)
+        assert torch.equal(hits_a, hits_b)
+        print(n, late, a / b)
+        assert (abs(a / b - 1) < 1e-3) if late else (a / b < 1 - 3e-3), (a, b)
+
+
+def test_batch_of_both_kinds(ctx):
+    """A batch whose warps trace meshes with and without shared vertices gives every mesh's
+    own hits."""
+    meshes = [hp.gen.uniform_mesh(5, 2000), hp.gen.heightfield(6, 40, 30), hp.gen.uniform_mesh(7, 300),
+              hp.gen.heightfield(8, 9, 7)]
+    counts = [5000, 77, 4001, 3000]
+    p = hp.BuildParams(method="lbvh", morton_bits=30)
+    batch = hp.Batch(ctx, [(dev(v), dev(t)) for v, t in meshes], counts, p)
+    rays = [hp.gen.rays_sphere(11 + i, k, np.concatenate([v.min(0), v.max(0)]))
+            for i, ((v, t), k) in enumerate(zip(meshes, counts))]
+    res = torch.zeros((sum(counts), 4), dtype=torch.int32, device="cuda")
+    batch.build(graph=False)
+    batch.trace(dev(np.concatenate(rays)), results=res, graph=False)
+    ctx.check()
+    at = 0
+    for (v, t), r in zip(meshes, rays):
+        one = torch.zeros((len(r), 4), dtype=torch.int32, device="cuda")
+        ctx.trace(ctx.build(dev(v), dev(t), p), dev(r), results=one)
+        assert torch.equal(res[at:at + len(r)], one)
+        at += len(r)
+    batch.close()

@@ -41,7 +41,8 @@ hp_status launch_batch_t(hp_ctx* ctx, const hp_batch_trace_args& t, unsigned lon
     k_trace<A, S, true, SST><<<trace_grid(ctx, per_sm, t.num_rays), TRACE_BLOCK, 0, s>>>(
         reinterpret_cast<const float4*>(t.rays), t.num_rays, reinterpret_cast<int4*>(t.results),
         reinterpret_cast<int2*>(t.stats), reinterpret_cast<const float4*>(t.nodes), t.woop, t.tri_idx, 0, 0,
-        counter, ctx->d_status, t.segs, t.ray_off, t.num_segs, nullptr, nullptr);
+        counter, ctx->d_status, t.segs, t.ray_off, t.num_segs, nullptr, nullptr,
+        few_rays(ctx, per_sm, t.num_rays));
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     return HP_OK;

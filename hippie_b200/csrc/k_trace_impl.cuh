@@ -79,24 +79,25 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 // a tracer that gives boxes a slack, rays that missed the nearer hit in 360 frames of
 // 2.07 M primary rays and in 360 times 4.2 M sphere rays on terrains: every lane in
 // loops of its own, as in the reference, 122 and 217; LEAST 1: 122 and 223; 2: 132, 228;
-// 3: 126, 232; 4: 128, 235; 16: 151, 280. Up to 4 that is as good, but it is other rays: of
-// runs over the 4.2 M, 5 % differ in a ray between two runs of either order (which rays share
-// a warp is decided as they come), 7 % between loops and 1, 20 % between loops and 4. So where
-// triangles share vertices leaves are tested late (LEAST 1), which returns what has always
-// been returned, and sooner elsewhere, where such pairs of hits do not come up. A build looks
+// 3: 126, 232; 4: 128, 235; 16: 151, 280. And it is other rays: of runs over the 4.2 M, 5 %
+// differ in a ray between two runs of either order (which rays share a warp is decided as
+// they come), 7 % between loops and LEAST 1, 20 % between loops and 4. So where triangles
+// share vertices leaves are tested late (LEAST 1), which returns what has always been
+// returned, and sooner elsewhere, where such pairs of hits do not come up. A build looks
 // whether they do (hp_bvh_info::lone); a batch's warp goes by the meshes whose rays it has.
 // A visibility ray has no nearest hit to miss.
 //
-// Measured on a B200, every lane in loops of its own -> now: 16.8 M bounce rays 28.4 -> 19.1 ms,
-// 43 M rays over 256 meshes 42.4 -> 28.0, 4 M sorted rays 3.86 -> 2.91, 4.2 M rays in 33.5 M
-// triangles 22.2 -> 22.7; late, 2.07 M primary rays 0.77 -> 0.69, 4.2 M downward rays 2.28 -> 2.13,
-// 4.2 M bounce rays on a terrain 3.12 -> 2.63 (at LEAST 4: 0.55, 2.22 and 2.28). Bounce, sorted
-// and batch rays at 1: 22.9, 3.23 and 32; at 16: 18.4, 3.00 and 27.3. FETCH 12 instead of 16:
-// bounce rays 3 % faster, downward ones 6 % slower; 20: the other way round.
+// Measured on a B200, every lane in loops of its own -> now: 16.8 M bounce rays 28.4 -> 18.2 ms,
+// 43 M rays over 256 meshes 42.4 -> 27.3, 4 M sorted rays 3.84 -> 2.87, 1.3 M rays in 10,763 triangles
+// 0.73 -> 0.62, 4.2 M rays in 33.5 M triangles 22.9 -> 24.4 (the one case that loses); late, 2.07 M
+// primary rays 0.76 -> 0.69, 4.2 M downward rays 2.28 -> 2.13, 4.2 M bounce rays on a terrain 3.12 ->
+// 2.63. Bounce, sorted, batch and large-tree rays at LEAST 1: 22.9, 3.23, 32 and 22.1; 4: 18.9, 2.90,
+// 28.0 and 24.4; 16: 19.5, 3.00, 27.9 and 24.2. FETCH 12 instead of 16: bounce rays 3 % faster,
+// downward ones 6 % slower and the large tree's 4 %; 20: the other way round.
 // Packed FP32 for the slabs and 32-byte loads of two Woop rows were slower or no faster.
 template <bool ANY_HIT>
 struct turns {
-    static constexpr int LEAST = ANY_HIT ? 12 : 4, FETCH = 16;
+    static constexpr int LEAST = ANY_HIT ? 12 : 8, FETCH = 16;
 };
 // CTAs per SM. Closest hits: 12 (40 registers, 4 bytes of spills read back) instead of 10
 // shorten bounce rays by 8 % and downward ones by 3 %, and cost rays in 33.5 M triangles 3 %.
@@ -113,7 +114,7 @@ __device__ __forceinline__ void trace_rays(
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
-    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, int* sstack) {
+    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, bool few, int* sstack) {
     constexpr int LST = STACK - SST;
     using TURN = turns<ANY_HIT>;
     int lstack[LST];
@@ -207,7 +208,8 @@ __device__ __forceinline__ void trace_rays(
                     }
                 }
             }
-            if (BATCH && !ANY_HIT) least = __any_sync(HP_FULL_MASK, ray >= 0 && !lone) ? 1 : TURN::LEAST;
+            if (BATCH)
+                least = few || (!ANY_HIT && __any_sync(HP_FULL_MASK, ray >= 0 && !lone)) ? 1 : TURN::LEAST;
         }
 
         // Interior nodes: one per lane and round.
@@ -348,27 +350,38 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
     const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order,
-    const hp_bvh_info* __restrict__ info) {
+    const hp_bvh_info* __restrict__ info, bool few) {
     __shared__ int s_stack[SST * TRACE_BLOCK];
     int* sstack = s_stack + threadIdx.x;
     // One body a kind of mesh: with one body and its limit in a register bounce rays take
     // 20.0 ms, not 19.1.
-    if (!BATCH && !ANY_HIT && __ldg(&info->lone) == 0)
+    if (!BATCH && (few || (!ANY_HIT && __ldg(&info->lone) == 0)))
         trace_rays<ANY_HIT, STATS, BATCH, SST, true>(rays, num_rays, results, stats, nodes_all, woop_all, tri_all,
                                                      max_nodes_all, num_refs_all, ray_counter, err, segs, ray_off,
-                                                     num_segs, order, sstack);
+                                                     num_segs, order, few, sstack);
     else
         trace_rays<ANY_HIT, STATS, BATCH, SST, false>(rays, num_rays, results, stats, nodes_all, woop_all, tri_all,
                                                       max_nodes_all, num_refs_all, ray_counter, err, segs, ray_off,
-                                                      num_segs, order, sstack);
+                                                      num_segs, order, few, sstack);
 }
 
-// Persistent grid: the tuned CTAs per SM, or as many as fit.
-int trace_grid(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
+// Persistent CTAs: the tuned number per SM, or as many as fit.
+int64_t trace_resident(const hp_ctx* ctx, int per_sm) {
     int k = std::max(per_sm, 1);
     if (ctx->tune.trace_ctas_per_sm > 0) k = std::min(k, (int)ctx->tune.trace_ctas_per_sm);
-    const int64_t grid = std::min<int64_t>((int64_t)ctx->sm_count * k, (num_rays + TRACE_BLOCK - 1) / TRACE_BLOCK);
+    return (int64_t)ctx->sm_count * k;
+}
+int trace_grid(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
+    const int64_t grid = std::min<int64_t>(trace_resident(ctx, per_sm), (num_rays + TRACE_BLOCK - 1) / TRACE_BLOCK);
     return (int)std::max<int64_t>(grid, 1);
+}
+
+// A launch that has no two rays for a lane lasts as long as its slowest warps: their lanes
+// take every turn they can (LEAST 1) instead of waiting for a fuller one, on any mesh (131,072
+// rays in 1.7 M triangles on a B200 587 -> 568 us, 1,000 visibility rays on a terrain 89 -> 72;
+// as a rule for 4 or 8 rays a lane 1 M visibility rays lose 6 %).
+bool few_rays(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
+    return num_rays < 2 * trace_resident(ctx, per_sm) * TRACE_BLOCK;
 }
 
 template <bool A, bool S, int SST>
@@ -381,7 +394,8 @@ hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const floa
     k_trace<A, S, false, SST><<<trace_grid(ctx, per_sm, num_rays), TRACE_BLOCK, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const float4*>(b->nodes), b->woop, b->tri_idx,
-        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order, b->info);
+        max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order, b->info,
+        few_rays(ctx, per_sm, num_rays));
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

@@ -49,17 +49,17 @@ constexpr int TB1 = 128;
 constexpr int SST1 = 16;
 // Turns (k_trace_impl.cuh says what they are, what LEAST decides and where it is 1; here NODE is
 // its part for nodes, and the triangles' limit hardly matters) and CTAs per SM. On a B200, every lane
-// in loops of its own -> now, 2 M bounce rays in 1 M triangles: Quad 2.99 -> 2.18 ms, Oct 3.71 -> 2.81
-// (at NODE 1 2.55 and 3.37, at 12 2.15 and 2.78); late, primary rays on a terrain and 4.2 M bounce
-// rays on another: Quad 0.65 -> 0.58 and 3.11 -> 2.65, Oct 0.74 -> 0.70 and 3.95 -> 3.49 (at NODE 4 0.53,
-// 2.29, 0.61 and 3.00). FETCH 12: 1 to 2 % slower. Visibility rays: Quad 1.16 -> 0.96 ms, Oct 1.31 ->
-// 1.18 for 1 M of them. Oct loses where there is little to do: 100,000 rays on a terrain of 1,000
-// triangles 91 -> 101 us, 8,192 triangles equal. CTAs at 9 (56 registers): Quad equal, Oct 12 %
+// in loops of its own -> now, 2 M bounce rays in 1 M triangles: Quad 2.99 -> 2.09 ms, Oct 3.71 -> 2.73
+// (at NODE 1 2.55 and 3.37, at 4 2.18 and 2.81); late, primary rays on a terrain and 4.2 M bounce
+// rays on another: Quad 0.65 -> 0.60 and 3.11 -> 2.65, Oct 0.74 -> 0.67 and 3.95 -> 3.47. FETCH 12: 1 to
+// 2 % slower. Visibility rays: Quad 1.16 -> 0.96 ms, Oct 1.31 -> 1.18 for 1 M of them. Oct loses where
+// there is little to do: 100,000 rays on a terrain of 1,000 triangles 91 -> 101 us, 8,192 triangles
+// equal. CTAs at 9 (56 registers): Quad equal, Oct 12 %
 // slower. Stack entries without distances: Quad 1 to 2 % slower, Oct 1 to 8 %.
 constexpr int CTAS1 = 8;
 template <bool ANY_HIT>
 struct turns1 {
-    static constexpr int NODE = ANY_HIT ? 12 : 4, TRI = 4, FETCH = ANY_HIT ? 12 : 8;
+    static constexpr int NODE = ANY_HIT ? 12 : 8, TRI = 4, FETCH = ANY_HIT ? 12 : 8;
 };
 constexpr int SENT1 = 0x76543210;
 template <int N> struct wide1_cfg;
@@ -73,9 +73,9 @@ __global__ void __launch_bounds__(TB1, CTAS1) k_trace_wide1(const float4* __rest
                                                    const int32_t* __restrict__ tri_idx, int max_nodes, int num_refs,
                                                    unsigned long long* ray_counter, int* err,
                                                    const int32_t* __restrict__ order,
-                                                   const hp_bvh_info* __restrict__ info) {
+                                                   const hp_bvh_info* __restrict__ info, bool few) {
     using TURN = turns1<ANY_HIT>;
-    const bool late = !ANY_HIT && __ldg(&info->lone) == 0;  // as in k_trace_impl.cuh
+    const bool late = few || (!ANY_HIT && __ldg(&info->lone) == 0);  // as in k_trace_impl.cuh
     constexpr int STACK = wide1_cfg<N>::STACK, LST = STACK - SST1;
     __shared__ int2 s_stack[SST1 * TB1];
     int2* sstack = s_stack + threadIdx.x;
@@ -308,7 +308,8 @@ hp_status launch_wide_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const
     k_trace_wide1<N, A, S><<<(unsigned)grid, TB1, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const int4*>(b->nodes), b->woop, b->tri_idx, max_nodes,
-        (int)n_refs, counter, ctx->d_status, order, b->info);
+        (int)n_refs, counter, ctx->d_status, order, b->info,
+        num_rays < 2 * (int64_t)ctx->sm_count * k * TB1);
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

@@ -89,11 +89,11 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 //
 // Measured on a B200, every lane in loops of its own -> now: 16.8 M bounce rays 28.4 -> 18.2 ms,
 // 43 M rays over 256 meshes 42.4 -> 27.3, 4 M sorted rays 3.84 -> 2.87, 1.3 M rays in 10,763 triangles
-// 0.73 -> 0.62, 4.2 M rays in 33.5 M triangles 22.9 -> 24.4 (the one case that loses); late, 2.07 M
+// 0.73 -> 0.62, 8.4 M rays in 33 M triangles 44.5 -> 45.6 (late, as LARGE_REFS says); late, 2.07 M
 // primary rays 0.76 -> 0.69, 4.2 M downward rays 2.28 -> 2.13, 4.2 M bounce rays on a terrain 3.12 ->
-// 2.63. Bounce, sorted, batch and large-tree rays at LEAST 1: 22.9, 3.23, 32 and 22.1; 4: 18.9, 2.90,
-// 28.0 and 24.4; 16: 19.5, 3.00, 27.9 and 24.2. FETCH 12 instead of 16: bounce rays 3 % faster,
-// downward ones 6 % slower and the large tree's 4 %; 20: the other way round.
+// 2.63. Bounce, sorted and batch rays at LEAST 1: 22.9, 3.23 and 32; 4: 18.9, 2.90 and 28.0; 16: 19.5,
+// 3.00 and 27.9. FETCH 12 instead of 16: bounce rays 3 % faster, downward ones 6 % slower and a large
+// tree's 4 %; 20: the other way round.
 // Packed FP32 for the slabs and 32-byte loads of two Woop rows were slower or no faster.
 template <bool ANY_HIT>
 struct turns {
@@ -114,7 +114,7 @@ __device__ __forceinline__ void trace_rays(
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
-    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, bool few, int* sstack) {
+    const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order, bool late, int* sstack) {
     constexpr int LST = STACK - SST;
     using TURN = turns<ANY_HIT>;
     int lstack[LST];
@@ -209,7 +209,7 @@ __device__ __forceinline__ void trace_rays(
                 }
             }
             if (BATCH)
-                least = few || (!ANY_HIT && __any_sync(HP_FULL_MASK, ray >= 0 && !lone)) ? 1 : TURN::LEAST;
+                least = late || (!ANY_HIT && __any_sync(HP_FULL_MASK, ray >= 0 && !lone)) ? 1 : TURN::LEAST;
         }
 
         // Interior nodes: one per lane and round.
@@ -350,19 +350,19 @@ __global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_tra
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
     unsigned long long* ray_counter, int* err, const hp_batch_seg* __restrict__ segs,
     const int64_t* __restrict__ ray_off, int num_segs, const int32_t* __restrict__ order,
-    const hp_bvh_info* __restrict__ info, bool few) {
+    const hp_bvh_info* __restrict__ info, bool late) {
     __shared__ int s_stack[SST * TRACE_BLOCK];
     int* sstack = s_stack + threadIdx.x;
     // One body a kind of mesh: with one body and its limit in a register bounce rays take
     // 20.0 ms, not 19.1.
-    if (!BATCH && (few || (!ANY_HIT && __ldg(&info->lone) == 0)))
+    if (!BATCH && (late || (!ANY_HIT && __ldg(&info->lone) == 0)))
         trace_rays<ANY_HIT, STATS, BATCH, SST, true>(rays, num_rays, results, stats, nodes_all, woop_all, tri_all,
                                                      max_nodes_all, num_refs_all, ray_counter, err, segs, ray_off,
-                                                     num_segs, order, few, sstack);
+                                                     num_segs, order, late, sstack);
     else
         trace_rays<ANY_HIT, STATS, BATCH, SST, false>(rays, num_rays, results, stats, nodes_all, woop_all, tri_all,
                                                       max_nodes_all, num_refs_all, ray_counter, err, segs, ray_off,
-                                                      num_segs, order, few, sstack);
+                                                      num_segs, order, late, sstack);
 }
 
 // Persistent CTAs: the tuned number per SM, or as many as fit.
@@ -384,6 +384,13 @@ bool few_rays(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
     return num_rays < 2 * trace_resident(ctx, per_sm) * TRACE_BLOCK;
 }
 
+// Closest hits of rays in an order of their own in trees far beyond the L2 wait for DRAM, and
+// wait less with leaves tested late, while more lanes have a node to ask for: 8.4 M sphere
+// rays, late and not, in 8 M triangles 14.5 and 14.0 ms, 16 M 25.2 and 25.9, 33 M 45.6 and 47.6
+// (25.3 and 44.5 with every lane in loops of its own); in ray Morton order 14.5 and 12.5 for
+// 16 M, 23.9 and 21.5 for 33 M.
+constexpr int64_t LARGE_REFS = 12 << 20;
+
 template <bool A, bool S, int SST>
 hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const float* rays,
                    int64_t num_rays, int32_t* results, int32_t* stats, unsigned long long* counter,
@@ -395,7 +402,7 @@ hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const floa
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const float4*>(b->nodes), b->woop, b->tri_idx,
         max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order, b->info,
-        few_rays(ctx, per_sm, num_rays));
+        few_rays(ctx, per_sm, num_rays) || (!A && !order && n_refs >= LARGE_REFS));
     HP_CUDA(cudaGetLastError());
     hp_count_launch();
     hp_mark(ctx, s, "trace");

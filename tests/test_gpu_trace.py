@@ -268,3 +268,30 @@ def test_batch_of_both_kinds(ctx):
         assert torch.equal(res[at:at + len(r)], one)
         at += len(r)
     batch.close()
+
+
+@pytest.mark.parametrize("ctas", [0, 5])
+@pytest.mark.parametrize("layout", [2, 4, 8])
+def test_launches_of_few_and_many_rays_agree(ctx, layout, ctas):
+    """Just below and at two rays a lane of the CTAs that are launched (12 or 8 per SM, or what
+    trace_ctas_per_sm says), and in chunks far below it: the same hits, of a mesh whose
+    triangles share vertices and of one whose do not."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    m = 2 * sms * 128 * (ctas or (12 if layout == 2 else 8))
+    ctx.set_tune(trace_ctas_per_sm=ctas)
+    try:
+        for v, t in (hp.gen.heightfield(3, 120, 150), hp.gen.uniform_mesh(4, 30000)):
+            rays = hp.gen.rays_sphere(5, m, np.concatenate([v.min(0), v.max(0)]))
+            bvh = ctx.build(dev(v), dev(t), hp.BuildParams(method="lbvh", morton_bits=60, layout=layout))
+            R, got = dev(rays), []
+            for cuts in ([0, m], [0, m - 1, m], list(range(0, m, 50021)) + [m]):
+                res = torch.zeros((m, 4), dtype=torch.int32, device="cuda")
+                for a, b in zip(cuts, cuts[1:]):
+                    ctx.trace(bvh, R[a:b], results=res[a:b])
+                got.append(res)
+            ctx.check()
+            for other in got[1:]:
+                # on a shared edge, within a slab's rounding: a few in 1e8 rays
+                assert int((other[:, 0] != got[0][:, 0]).sum()) <= 2
+    finally:
+        ctx.reset_tune()

@@ -273,7 +273,10 @@ hp_status hp_refit(hp_ctx* ctx, hp_bvh* bvh, const hp_mesh* m, void* stream);
  * results: 4 int32 per ray {triangle id, t bits, u bits, v bits} (RayResult);
  * on a miss only {-1, tmax bits} are written. stats (or NULL): 2 int32 per ray
  * {traversed nodes, tested triangles}. Closest hits break ties in t by the
- * lower triangle id. */
+ * lower triangle id. Of two hits whose t differ by less than the rounding of a
+ * node's slab distances (on an edge that two triangles share) either can be
+ * returned, by the order in which a ray comes to them; with or without stats,
+ * and from run to run, that can be the other one. */
 hp_status hp_trace(hp_ctx* ctx, const hp_bvh* bvh, const float* rays, int64_t num_rays,
                    int32_t* results, int32_t* stats, uint32_t flags, void* stream);
 

@@ -41,10 +41,10 @@ def test_radix_sort_with_values(ctx):
 
 
 def _wide_case(kind, n, bits, rng):
-    """Keys for the wide-key path (bits > 48, n >= 2^20): the array is first
-    ordered by its top 16 sorted bits, then every run of equal top bits is
-    sorted by the rest, in shared memory, or by the large-segment kernel when
-    a run exceeds 4096 keys."""
+    """Keys for the wide-key path (bits > 48): the array is first ordered by its top
+    24 sorted bits, then every run of equal top bits is sorted by the rest, in
+    shared memory, or by the large-segment kernel when a run exceeds 2,048 keys.
+    The top 16 bits are chosen here, so a run has about 1/256 of a prefix's keys."""
     low = rng.integers(0, 1 << (bits - 16), size=n, dtype=np.uint64)
     if kind == "uniform":
         top = rng.integers(0, 1 << 16, size=n, dtype=np.uint64)

@@ -37,8 +37,8 @@ __global__ void k_trace_empty(const float4* rays, int64_t num_rays, int4* result
 template <bool A, bool S, int SST>
 hp_status launch_batch_t(hp_ctx* ctx, const hp_batch_trace_args& t, unsigned long long* counter, cudaStream_t s) {
     int per_sm = 0;
-    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<A, S, true, SST>, TRACE_BLOCK, 0));
-    k_trace<A, S, true, SST><<<trace_grid(ctx, per_sm, t.num_rays), TRACE_BLOCK, 0, s>>>(
+    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<A, S, true, SST, CTAS_BATCH>, TRACE_BLOCK, 0));
+    k_trace<A, S, true, SST, CTAS_BATCH><<<trace_grid(ctx, per_sm, t.num_rays), TRACE_BLOCK, 0, s>>>(
         reinterpret_cast<const float4*>(t.rays), t.num_rays, reinterpret_cast<int4*>(t.results),
         reinterpret_cast<int2*>(t.stats), reinterpret_cast<const float4*>(t.nodes), t.woop, t.tri_idx, 0, 0,
         counter, ctx->d_status, t.segs, t.ray_off, t.num_segs, nullptr, nullptr,

@@ -89,8 +89,8 @@ __device__ __forceinline__ int seg_search(const int64_t* __restrict__ off, int n
 //
 // Measured on a B200, every lane in loops of its own -> now: 16.8 M bounce rays 28.4 -> 18.2 ms,
 // 43 M rays over 256 meshes 42.4 -> 27.3, 4 M sorted rays 3.84 -> 2.87, 1.3 M rays in 10,763 triangles
-// 0.73 -> 0.62, 8.4 M rays in 33 M triangles 44.5 -> 45.6 (late, as LARGE_REFS says); late, 2.07 M
-// primary rays 0.76 -> 0.69, 4.2 M downward rays 2.28 -> 2.13, 4.2 M bounce rays on a terrain 3.12 ->
+// 0.73 -> 0.60, 8.4 M rays in 33 M triangles 44.5 -> 45.6 (late, as LARGE_REFS says); late, 2.07 M
+// primary rays 0.76 -> 0.65, 4.2 M downward rays 2.28 -> 2.13, 4.2 M bounce rays on a terrain 3.12 ->
 // 2.63. Bounce, sorted and batch rays at LEAST 1: 22.9, 3.23 and 32; 4: 18.9, 2.90 and 28.0; 16: 19.5,
 // 3.00 and 27.9. FETCH 12 instead of 16: bounce rays 3 % faster, downward ones 6 % slower and a large
 // tree's 4 %; 20: the other way round.
@@ -99,11 +99,14 @@ template <bool ANY_HIT>
 struct turns {
     static constexpr int LEAST = ANY_HIT ? 12 : 8, FETCH = 16;
 };
-// CTAs per SM. Closest hits: 12 (40 registers, 4 bytes of spills read back) instead of 10
-// shorten bounce rays by 8 % and downward ones by 3 %, and cost rays in 33.5 M triangles 3 %.
+// CTAs per SM that the kernel is compiled for. Closest hits: 12 (40 registers, some spilled) in
+// trees that the L1 does not help much, where bounce rays take 18.2 ms instead of 19.8 at 10 (46
+// registers); 10 below SMALL_REFS, where instructions count: 1.3 M rays in 10,763 triangles 0.598
+// instead of 0.625 ms, 1 M in 100,003 1.07 instead of 1.12; at 0.5 to 1 M triangles equal.
 // Any hit: 1.05 M shadow rays 0.91 ms at 8 and 9, 0.97 at 10, 1.02 at 12. Batch (the
 // mesh's bases in the lane, 55 registers): 27.3 ms at 8, 28.9 at 9, 30.0 at 10.
-constexpr int trace_ctas(bool any_hit, bool batch) { return batch ? 8 : any_hit ? 9 : 12; }
+constexpr int CTAS_LARGE = 12, CTAS_SMALL = 10, CTAS_ANY = 9, CTAS_BATCH = 8;
+constexpr int64_t SMALL_REFS = 1 << 19;
 
 // BATCH: rays of many meshes in one launch; ray g belongs to the segment whose
 // ray range holds it, and the lane traverses that mesh's BVH.
@@ -343,8 +346,8 @@ __device__ __forceinline__ void trace_rays(
     }
 }
 
-template <bool ANY_HIT, bool STATS, bool BATCH, int SST>
-__global__ void __launch_bounds__(TRACE_BLOCK, trace_ctas(ANY_HIT, BATCH)) k_trace(
+template <bool ANY_HIT, bool STATS, bool BATCH, int SST, int CTAS>
+__global__ void __launch_bounds__(TRACE_BLOCK, CTAS) k_trace(
     const float4* __restrict__ rays, int64_t num_rays, int4* __restrict__ results,
     int2* __restrict__ stats, const float4* __restrict__ nodes_all, const float4* __restrict__ woop_all,
     const int32_t* __restrict__ tri_all, int max_nodes_all, int num_refs_all,
@@ -391,14 +394,14 @@ bool few_rays(const hp_ctx* ctx, int per_sm, int64_t num_rays) {
 // 16 M, 23.9 and 21.5 for 33 M.
 constexpr int64_t LARGE_REFS = 12 << 20;
 
-template <bool A, bool S, int SST>
+template <bool A, bool S, int SST, int CTAS>
 hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const float* rays,
                    int64_t num_rays, int32_t* results, int32_t* stats, unsigned long long* counter,
                    const int32_t* order, cudaStream_t s) {
     int per_sm = 0;
-    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<A, S, false, SST>, TRACE_BLOCK, 0));
+    HP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<A, S, false, SST, CTAS>, TRACE_BLOCK, 0));
     const int max_nodes = (int)std::max<int64_t>(2 * b->capacity - 1, 3);
-    k_trace<A, S, false, SST><<<trace_grid(ctx, per_sm, num_rays), TRACE_BLOCK, 0, s>>>(
+    k_trace<A, S, false, SST, CTAS><<<trace_grid(ctx, per_sm, num_rays), TRACE_BLOCK, 0, s>>>(
         reinterpret_cast<const float4*>(rays), num_rays, reinterpret_cast<int4*>(results),
         reinterpret_cast<int2*>(stats), reinterpret_cast<const float4*>(b->nodes), b->woop, b->tri_idx,
         max_nodes, (int)n_refs, counter, ctx->d_status, nullptr, nullptr, 0, order, b->info,
@@ -409,13 +412,25 @@ hp_status launch_t(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const floa
     return HP_OK;
 }
 
+template <bool A, bool S, int SST>
+hp_status launch_size(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const float* rays,
+                      int64_t num_rays, int32_t* results, int32_t* stats, unsigned long long* counter,
+                      const int32_t* order, cudaStream_t s) {
+    if constexpr (A)
+        return launch_t<A, S, SST, CTAS_ANY>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+    else if (n_refs < SMALL_REFS)
+        return launch_t<A, S, SST, CTAS_SMALL>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+    else
+        return launch_t<A, S, SST, CTAS_LARGE>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+}
+
 template <bool A, bool S>
 hp_status launch_st(hp_ctx* ctx, const hp_bvh_impl* b, int64_t n_refs, const float* rays,
                     int64_t num_rays, int32_t* results, int32_t* stats, unsigned long long* counter,
                     const int32_t* order, cudaStream_t s) {
     switch (ctx->tune.trace_stack) {
-        case 8: return launch_t<A, S, 8>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
-        case 32: return launch_t<A, S, 32>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
-        default: return launch_t<A, S, 16>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+        case 8: return launch_size<A, S, 8>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+        case 32: return launch_size<A, S, 32>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
+        default: return launch_size<A, S, 16>(ctx, b, n_refs, rays, num_rays, results, stats, counter, order, s);
     }
 }

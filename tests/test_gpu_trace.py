@@ -273,11 +273,11 @@ def test_batch_of_both_kinds(ctx):
 @pytest.mark.parametrize("ctas", [0, 5])
 @pytest.mark.parametrize("layout", [2, 4, 8])
 def test_launches_of_few_and_many_rays_agree(ctx, layout, ctas):
-    """Just below and at two rays a lane of the CTAs that are launched (12 or 8 per SM, or what
+    """Just below and at two rays a lane of the CTAs that are launched (10 or 8 per SM, or what
     trace_ctas_per_sm says), and in chunks far below it: the same hits, of a mesh whose
     triangles share vertices and of one whose do not."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    m = 2 * sms * 128 * (ctas or (12 if layout == 2 else 8))
+    m = 2 * sms * 128 * (ctas or (10 if layout == 2 else 8))
     ctx.set_tune(trace_ctas_per_sm=ctas)
     try:
         for v, t in (hp.gen.heightfield(3, 120, 150), hp.gen.uniform_mesh(4, 30000)):
@@ -295,3 +295,12 @@ def test_launches_of_few_and_many_rays_agree(ctx, layout, ctas):
                 assert int((other[:, 0] != got[0][:, 0]).sum()) <= 2
     finally:
         ctx.reset_tune()
+
+
+@pytest.mark.parametrize("n", [(1 << 19) - 1, 1 << 19])
+def test_both_sizes_of_tracer(ctx, n):
+    """Around the tree size where closest hits go to the tracer of more CTAs per SM."""
+    v, t, rays, bvh = _setup(ctx, "uniform", n, 50000, 60, seed=3)
+    got = ctx.trace(bvh, dev(rays), results=torch.zeros((len(rays), 4), dtype=torch.int32, device="cuda"))
+    ctx.check()
+    np.testing.assert_array_equal(got.cpu().numpy(), oracle.trace(*bvh.download(), rays))
